@@ -15,7 +15,7 @@
 // components/interactions/{base,list}.py and coulomb/{secondorder,
 // thirdorder,multipole}.py (potentials and energies), scf/base.py:510-619
 // (energy and electronic free energy).
-#include "linalg.cuh"
+#include "eigemm.cuh"
 
 namespace dxtb {
 
@@ -45,10 +45,14 @@ __host__ __device__ inline int64_t lu_size(int64_t n) {
 }
 
 // Per-molecule workspace layout (doubles).
-__host__ __device__ inline int64_t ws_size_mol(int64_t n, int64_t nat) {
+__host__ __device__ inline int64_t ws_size_base(int64_t n, int64_t nat) {
   const int64_t N = n + 9 * nat;
   return 3 * n * n + 10 * n + (2 * kRank + 7) * N + 64 + 16 * nat + lu_size(n) + n + 8 +
          4 * kRank + 64 + 64;
+}
+// with the digit planes of the tensor-core path (eigemm.cuh)
+__host__ __device__ inline int64_t ws_size_mol(int64_t n, int64_t nat) {
+  return ws_size_base(n, nat) + fast_size(n);
 }
 
 struct Ws {
@@ -164,6 +168,7 @@ struct ScfArgs {
   double *ws, *P, *W, *C, *evals, *occ, *q, *dp, *qp, *vorb, *vdp, *vqp, *energies;
   int32_t *status;
   int thr[kClasses];  // smallest n of each size class (thr[0] = 0)
+  int fast;           // the workspace has room for the digit planes
 };
 
 // Potential x = (vorb [n], vdp [nat][3], vqp [nat][6]) from the orbital
@@ -566,6 +571,7 @@ template <bool CL>
 __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bool rows) {
   __shared__ double red[32];
   __shared__ double spart[kPart];
+  __shared__ float4 sfour[32];
   const dxtb_batch &b = a.b;
   MolView mv;
   mv.m = m_;
@@ -610,6 +616,15 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
   if (status == DXTB_OK) team_trinv(tm, n, w.A, w.Linv);
   for (int t = tm.tid; t < N; t += tm.nthr) w.x[t] = 0.0;
   tm.sync();
+  // The products and the eigenproblem run on digit planes; where a norm is not
+  // finite or the vectors do not settle, or without the workspace for the
+  // planes, the float64 path takes over for the rest of this SCF.
+  Fast f = {};
+  bool fast = a.fast != 0 && status == DXTB_OK;
+  if (fast) {
+    f = fast_carve(a.ws + a.ws_off[m] + ws_size_base(n, nat), n);
+    fast = fast_setup(tm, n, w.Linv, f, sfour);
+  }
 
   int it = 0, mo = 1;
   Broyden br;
@@ -649,35 +664,48 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
       }
       tm.sync();
     }
-    // ---- F' = X F X^T (exlibs/xitorch/_impls/linalg/symeig.py:57-61) ----
-    // X = L^-1 is lower triangular: A = X F needs k <= i; only the lower
-    // triangle of (X F) X^T is formed (k <= j), then mirrored.
-    team_gemm<false, false>(tm, n, n, n, 1.0, w.Linv, n, w.Zt, n, 0.0, w.A, n, kALower);
-    team_gemm<false, true>(tm, n, n, n, 1.0, w.A, n, w.Linv, n, 0.0, w.Zt, n, kBLowerT, true);
-    for (int64_t t = tm.tid; t < (int64_t)n * n; t += tm.nthr) {
-      const int i = (int)(t / n), j = (int)(t % n);
-      w.A[t] = j <= i ? ld<CL>(w.Zt + t) : ld<CL>(w.Zt + (size_t)j * n + i);
-    }
-    tm.sync();
-    // ---- eigenvalues: Householder tridiagonalisation + bisection/Newton ----
-    {
-      uint32_t dyn;
-      asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
-      const int64_t cap = (int64_t)(dyn / sizeof(double)) - 4 * (int64_t)n;
-      team_tridiag(tm, n, w.A, w.d, w.e, w.tau, sd, se, sw, reinterpret_cast<double *>(df), spart,
-                   rows && cap > 0 ? dsm + 4 * n : nullptr, cap);
-    }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      sd[i] = ld<CL>(w.d + i);
-      se[i] = ld<CL>(w.e + i);
-    }
-    __syncthreads();
-    team_tri_eigenvalues(tm, n, sd, se, sw, w.rc, df, e2f);  // sw: e^2 scratch here
-    team_rank_sort(tm, n, w.rc, w.eps, sw);  // ascending, like eigh
-    for (int i = threadIdx.x; i < n; i += blockDim.x) sw[i] = ld<CL>(w.eps + i);
+    // ---- F' = X F X^T and its eigenvalues (ascending, sw) and vectors ----
     double tnorm = 0.0;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) tnorm = fmax(tnorm, fabs(sd[j]) + 2.0 * fabs(se[j]));
-    tnorm = block_max(tnorm, red);  // also orders the sw writes
+    if (fast) {
+      int s2;
+      fast = fast_transform(tm, n, f, w.Zt, w.A, s2, sfour) && fast_eigen(tm, n, f, sd, se, df, e2f, sfour);
+      if (fast) {
+        const double scale = ldexp(1.0, s2);
+        for (int i = threadIdx.x; i < n; i += blockDim.x) sw[i] = sd[i] * scale;
+      }
+      __syncthreads();
+    }
+    if (!fast) {
+      // ---- F' = X F X^T (exlibs/xitorch/_impls/linalg/symeig.py:57-61) ----
+      // X = L^-1 is lower triangular: A = X F needs k <= i; only the lower
+      // triangle of (X F) X^T is formed (k <= j), then mirrored.
+      team_gemm<false, false>(tm, n, n, n, 1.0, w.Linv, n, w.Zt, n, 0.0, w.A, n, kALower);
+      team_gemm<false, true>(tm, n, n, n, 1.0, w.A, n, w.Linv, n, 0.0, w.Zt, n, kBLowerT, true);
+      for (int64_t t = tm.tid; t < (int64_t)n * n; t += tm.nthr) {
+        const int i = (int)(t / n), j = (int)(t % n);
+        w.A[t] = j <= i ? ld<CL>(w.Zt + t) : ld<CL>(w.Zt + (size_t)j * n + i);
+      }
+      tm.sync();
+      // ---- eigenvalues: Householder tridiagonalisation + bisection/Newton ----
+      {
+        uint32_t dyn;
+        asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
+        const int64_t cap = (int64_t)(dyn / sizeof(double)) - 4 * (int64_t)n;
+        team_tridiag(tm, n, w.A, w.d, w.e, w.tau, sd, se, sw, reinterpret_cast<double *>(df), spart,
+                     rows && cap > 0 ? dsm + 4 * n : nullptr, cap);
+      }
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        sd[i] = ld<CL>(w.d + i);
+        se[i] = ld<CL>(w.e + i);
+      }
+      __syncthreads();
+      team_tri_eigenvalues(tm, n, sd, se, sw, w.rc, df, e2f);  // sw: e^2 scratch here
+      team_rank_sort(tm, n, w.rc, w.eps, sw);  // ascending, like eigh
+      for (int i = threadIdx.x; i < n; i += blockDim.x) sw[i] = ld<CL>(w.eps + i);
+      tnorm = 0.0;
+      for (int j = threadIdx.x; j < n; j += blockDim.x) tnorm = fmax(tnorm, fabs(sd[j]) + 2.0 * fabs(se[j]));
+      tnorm = block_max(tnorm, red);  // also orders the sw writes
+    }
     // ---- Fermi occupations (filling.py:428-742), both spin channels ----
     if (tm.lead() && threadIdx.x < 32) {
       bool ok = fermi_warp(n, sw, nel_a, a.kt, w.fa);
@@ -694,7 +722,7 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
         while (mm < n && w.fa[mm] + w.fb[mm] > kOccCut) ++mm;
         mm = mm > 0 ? mm : 1;
         const double ctol = 1e-6 * fmax(tnorm, 1.0);
-        while (mm < n && sw[mm] - sw[mm - 1] <= ctol) ++mm;
+        while (!fast && mm < n && sw[mm] - sw[mm - 1] <= ctol) ++mm;
         tm.gctl[0] = ok ? 1 : 0;
         tm.gctl[1] = mm;
       }
@@ -705,20 +733,26 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
       break;
     }
     mo = ldi<CL>(tm.gctl + 1);
-    // ---- eigenvectors of the mo lowest orbitals only ----
-    team_tri_vectors(tm, n, sd, se, sw, mo, tnorm, w.Zt, w.lu, (int)min((int64_t)tm.nthr, lu_slots(n)), w.cl,
-                     reinterpret_cast<double *>(df));
-    team_back_transform(tm, n, w.A, w.tau, w.Zt, mo, w.lu, spart);  // lu: free after the vectors
-    // ---- C^T = Y^T X (orbital j is row j; X lower -> k >= i) ----
-    team_gemm<true, false>(tm, mo, n, n, 1.0, w.Zt, mo, w.Linv, n, 0.0, C, n, kBUpper);
-    // ---- density P = C diag(occ) C^T (scf/utils.py:29-52) ----
-    for (int64_t t = tm.tid; t < (int64_t)mo * n; t += tm.nthr) {
-      const int j = (int)(t / n);
-      w.A[t] = ld<CL>(C + t) * (ld<CL>(w.fa + j) + ld<CL>(w.fb + j));
+    if (fast) {
+      // ---- C^T, then P = C diag(occ) C^T (scf/utils.py:29-52) ----
+      fast_coefficients(tm, f, mo);
+      fast_density(tm, n, f, mo, 1, [&](int j) { return ld<CL>(w.fa + j) + ld<CL>(w.fb + j); }, P);
+    } else {
+      // ---- eigenvectors of the mo lowest orbitals only ----
+      team_tri_vectors(tm, n, sd, se, sw, mo, tnorm, w.Zt, w.lu, (int)min((int64_t)tm.nthr, lu_slots(n)), w.cl,
+                       reinterpret_cast<double *>(df));
+      team_back_transform(tm, n, w.A, w.tau, w.Zt, mo, w.lu, spart);  // lu: free after the vectors
+      // ---- C^T = Y^T X (orbital j is row j; X lower -> k >= i) ----
+      team_gemm<true, false>(tm, mo, n, n, 1.0, w.Zt, mo, w.Linv, n, 0.0, C, n, kBUpper);
+      // ---- density P = C diag(occ) C^T (scf/utils.py:29-52) ----
+      for (int64_t t = tm.tid; t < (int64_t)mo * n; t += tm.nthr) {
+        const int j = (int)(t / n);
+        w.A[t] = ld<CL>(C + t) * (ld<CL>(w.fa + j) + ld<CL>(w.fb + j));
+      }
+      tm.sync();
+      team_gemm<true, false>(tm, n, n, mo, 1.0, C, n, w.A, n, 0.0, P, n, kFull, true);
+      team_mirror_lower(tm, n, P);
     }
-    tm.sync();
-    team_gemm<true, false>(tm, n, n, mo, 1.0, C, n, w.A, n, 0.0, P, n, kFull, true);
-    team_mirror_lower(tm, n, P);
     // ---- Mulliken charges and atomic multipoles (conversions.py:203-251) ----
     for (int i = tm.tid; i < n; i += tm.nthr) {
       double pop = 0.0;
@@ -803,7 +837,12 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
       }
     }
     // energy-weighted density W = C diag(occ eps) C^T over the mo orbitals
-    if (a.W != nullptr) {
+    if (a.W != nullptr && fast) {
+      const double top = fmax(fabs(sw[0]), fabs(sw[n - 1]));
+      const int e2 = top > 1e-30 ? exp_above((float)top) + 1 : 0;
+      fast_density(tm, n, f, mo, e2, [&](int j) { return (ld<CL>(w.fa + j) + ld<CL>(w.fb + j)) * sw[j]; },
+                   a.W + mv.moff);
+    } else if (a.W != nullptr) {
       for (int64_t t = tm.tid; t < (int64_t)mo * n; t += tm.nthr) {
         const int j = (int)(t / n);
         w.A[t] = ld<CL>(C + t) * (ld<CL>(w.fa + j) + ld<CL>(w.fb + j)) * sw[j];
@@ -812,6 +851,7 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
       team_gemm<true, false>(tm, n, n, mo, 1.0, C, n, w.A, n, 0.0, a.W + mv.moff, n, kFull, true);
       team_mirror_lower(tm, n, a.W + mv.moff);
     }
+    if (fast) fast_orbitals(tm, n, f, mo, C);
     // coefficients of orbitals without occupation are not computed
     for (int64_t t = (int64_t)mo * n + tm.tid; t < (int64_t)n * n; t += tm.nthr) C[t] = 0.0;
   }
@@ -833,7 +873,7 @@ __global__ void __launch_bounds__(NT, MINB) k_scf(ScfArgs a, int cls) {
   tm.tid = threadIdx.x;
   tm.stid = threadIdx.x;
   tm.nthr = blockDim.x;
-  scf_body<false>(a, m, tm, dsm, MINB == 1);
+  scf_body<false>(a, m, tm, dsm, false);
 }
 
 // One thread-block cluster per molecule of size class `cls` (2..5); the
@@ -853,7 +893,7 @@ __global__ void __launch_bounds__(kScfBigThreads, 1) k_scf_cluster(ScfArgs a, in
   for (int i = 0; i < a.b.nmol; ++i) {
     const int m = a.order ? a.order[i] : i;
     if (scf_class(a.thr, (int)(a.b.ao_off[m + 1] - a.b.ao_off[m])) != cls) continue;
-    if (cnt++ % nq == q) scf_body<true>(a, m, tm, dsm, true);
+    if (cnt++ % nq == q) scf_body<true>(a, m, tm, dsm, false);
   }
 }
 
@@ -1027,22 +1067,8 @@ static int32_t launch_scf(ScfArgs a, int nmol, cudaStream_t st, const GradArgs *
                                     kMaxDynSmem) == cudaSuccess;
       }) != DXTB_OK)
     return DXTB_ERR_LAUNCH;
-  // shared memory of class c: the base plus the rows of the Householder
-  // reduction of its largest possible molecule (and, for clusters, one
-  // broadcast row). When they do not all fit, the CTA takes the most shared
-  // memory if that still holds 60 % of the rows; below that the rows stay in
-  // L1/L2 (shared memory is carved out of L1; a carve-out holding a fifth to
-  // a third of the rows gained nothing at n ~ 900-1000)
-  auto class_smem = [&](int c) -> size_t {
-    const int csize = c >= 2 ? 1 << (c - 1) : 1;
-    const int nub = (c + 1 < kClasses && a.thr[c + 1] != INT32_MAX) ? min(nmax, a.thr[c + 1] - 1) : nmax;
-    const int nown = (nub + csize - 1) / csize;
-    const int rows = nown + (c >= 2 ? 1 : 0);
-    const size_t full = smem + (size_t)rows * nub * sizeof(double);
-    if (full <= (size_t)kMaxDynSmem) return full;
-    const int64_t fit = ((int64_t)kMaxDynSmem / 8 - 4 * (int64_t)nub) / nub - (c >= 2 ? 1 : 0);
-    return 10 * fit >= 6 * (int64_t)nown ? (size_t)kMaxDynSmem : smem;
-  };
+  // shared memory of every class: the base. The L1 serves the digit planes.
+  auto class_smem = [&](int) -> size_t { return smem; };
   // largest classes first: clusters, then one-SM CTAs, then the shared SMs
   for (int c = cmax; c >= 2; --c) {
     const int csize = 1 << (c - 1);
@@ -1143,16 +1169,17 @@ static int32_t apply_config(const dxtb_scf_config *c, ScfArgs &a) {
 
 }  // namespace dxtb
 
-extern "C" int32_t dxtb_scf(const dxtb_batch *b, const double *par_f, const int32_t *par_i,
-                            const double *overlap, const double *h0, const double *dipole,
-                            const double *quadrupole, const double *gamma, const double *hd,
-                            const double *amat_sd, const double *amat_dd, const double *amat_sq,
-                            const double *gb_mat, const double *n0, const double *nel, double kt,
-                            const dxtb_scf_config *cfg, const int64_t *ws_off,
-                            const int32_t *order, double *workspace, double *density,
-                            double *wdensity, double *coeff, double *evals, double *occ, double *q,
-                            double *dp, double *qp, double *vorb, double *vdp, double *vqp,
-                            double *energies, int32_t *status, void *stream) {
+// dxtb_scf; fast: the workspace holds ws_size_mol (else ws_size_base) doubles a molecule.
+static int32_t scf_call(const dxtb_batch *b, const double *par_f, const int32_t *par_i,
+                        const double *overlap, const double *h0, const double *dipole,
+                        const double *quadrupole, const double *gamma, const double *hd,
+                        const double *amat_sd, const double *amat_dd, const double *amat_sq,
+                        const double *gb_mat, const double *n0, const double *nel, double kt,
+                        const dxtb_scf_config *cfg, const int64_t *ws_off, const int32_t *order,
+                        double *workspace, double *density, double *wdensity, double *coeff,
+                        double *evals, double *occ, double *q, double *dp, double *qp, double *vorb,
+                        double *vdp, double *vqp, double *energies, int32_t *status, void *stream,
+                        int fast) {
   if (!b || b->nmol <= 0 || !overlap || !h0 || !gamma || !hd || !n0 || !nel || !ws_off ||
       !workspace || !density || !coeff || !evals || !occ || !q || !vorb || !energies || !status)
     return DXTB_ERR_ARGS;
@@ -1191,7 +1218,23 @@ extern "C" int32_t dxtb_scf(const dxtb_batch *b, const double *par_f, const int3
   a.vqp = vqp;
   a.energies = energies;
   a.status = status;
+  a.fast = fast;
   return launch_scf(a, b->nmol, (cudaStream_t)stream);
+}
+
+extern "C" int32_t dxtb_scf(const dxtb_batch *b, const double *par_f, const int32_t *par_i,
+                            const double *overlap, const double *h0, const double *dipole,
+                            const double *quadrupole, const double *gamma, const double *hd,
+                            const double *amat_sd, const double *amat_dd, const double *amat_sq,
+                            const double *gb_mat, const double *n0, const double *nel, double kt,
+                            const dxtb_scf_config *cfg, const int64_t *ws_off,
+                            const int32_t *order, double *workspace, double *density,
+                            double *wdensity, double *coeff, double *evals, double *occ, double *q,
+                            double *dp, double *qp, double *vorb, double *vdp, double *vqp,
+                            double *energies, int32_t *status, void *stream) {
+  return scf_call(b, par_f, par_i, overlap, h0, dipole, quadrupole, gamma, hd, amat_sd, amat_dd,
+                  amat_sq, gb_mat, n0, nel, kt, cfg, ws_off, order, workspace, density, wdensity,
+                  coeff, evals, occ, q, dp, qp, vorb, vdp, vqp, energies, status, stream, 1);
 }
 
 extern "C" int32_t dxtb_scf_gradient(
@@ -1243,6 +1286,7 @@ extern "C" int32_t dxtb_scf_gradient(
   a.vqp = vqp;
   a.energies = energies;
   a.status = status;
+  a.fast = 1;
   GradArgs g{cn, mrad, dedcn, grad};
   return launch_scf(a, b->nmol, (cudaStream_t)stream, &g);
 }
@@ -1273,17 +1317,25 @@ static __device__ __align__(256) double g_scf_scratch[DXTB_NOALLOC_SCRATCH_DOUBL
 // per-molecule workspace offsets (int64, relative to the workspace start).
 constexpr int64_t kNoallocHeader = 1;
 
+// A batch whose digit planes do not fit keeps the float64 path, whose
+// workspace is smaller: what the array holds without the planes is accepted.
+constexpr int64_t kNoallocFast = int64_t(1) << 62;  // flag in [0]: room for the planes
+
 __global__ void k_noalloc_layout(dxtb_batch b, int64_t *hdr, int64_t ws_start) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int64_t off = 0;
-  for (int m = 0; m < b.nmol; ++m) {
-    hdr[kNoallocHeader + m] = off;
-    const int64_t n = b.ao_off[m + 1] - b.ao_off[m];
-    const int64_t nat = b.atom_off[m + 1] - b.atom_off[m];
-    off += ws_size_mol(n, nat);
-  }
-  hdr[kNoallocHeader + b.nmol] = off;
-  hdr[0] = ws_start + off;  // doubles needed from the start of the array
+  auto lay = [&](bool fast) {
+    int64_t off = 0;
+    for (int m = 0; m < b.nmol; ++m) {
+      hdr[kNoallocHeader + m] = off;
+      const int64_t n = b.ao_off[m + 1] - b.ao_off[m];
+      const int64_t nat = b.atom_off[m + 1] - b.atom_off[m];
+      off += fast ? ws_size_mol(n, nat) : ws_size_base(n, nat);
+    }
+    hdr[kNoallocHeader + b.nmol] = off;
+    return ws_start + off;  // doubles needed from the start of the array
+  };
+  const int64_t need = lay(true);
+  hdr[0] = need <= DXTB_NOALLOC_SCRATCH_DOUBLES ? (need | kNoallocFast) : lay(false);
 }
 
 static std::mutex g_noalloc_mutex;
@@ -1330,7 +1382,8 @@ extern "C" int32_t dxtb_scf_noalloc(
   if (cudaMemcpyAsync(&need, hdr, sizeof(int64_t), cudaMemcpyDeviceToHost, st) != cudaSuccess)
     return DXTB_ERR_LAUNCH;
   if (cudaStreamSynchronize(st) != cudaSuccess) return DXTB_ERR_LAUNCH;
-  if (need > DXTB_NOALLOC_SCRATCH_DOUBLES) return DXTB_ERR_TOO_LARGE;
+  const int fast = (need & kNoallocFast) != 0;
+  if ((need & ~kNoallocFast) > DXTB_NOALLOC_SCRATCH_DOUBLES) return DXTB_ERR_TOO_LARGE;
   // the implicit-mode root solver with one tolerance for x_atol and f_atol
   dxtb_scf_config cfg = {};
   cfg.maxiter = maxiter;
@@ -1338,8 +1391,8 @@ extern "C" int32_t dxtb_scf_noalloc(
   cfg.x_atol = tol;
   cfg.f_atol = tol;
   cfg.damp = 0.5;
-  return dxtb_scf(b, par_f, par_i, overlap, h0, dipole, quadrupole, gamma, hd, amat_sd, amat_dd,
+  return scf_call(b, par_f, par_i, overlap, h0, dipole, quadrupole, gamma, hd, amat_sd, amat_dd,
                   amat_sq, gb_mat, n0, nel, kt, &cfg, hdr + kNoallocHeader, order,
                   scratch + ws_start, density, wdensity, coeff, evals, occ, q, dp, qp, vorb, vdp,
-                  vqp, energies, status, stream);
+                  vqp, energies, status, stream, fast);
 }
