@@ -15,10 +15,12 @@
 // exact in fp16, so |value| < 4). Results are 64-bit integers of weight 2^-56.
 //
 // Digit planes are stored in the register layout of the instruction: a block
-// of 16 x 16 values is one 16-byte word per lane and plane. The layout of the
-// A operand (rows i, inner index k) with its four registers permuted is that
-// of two B operands, so one set of planes serves on both sides of
-// C = A B^T, and a result tile has the layout of an A operand.
+// of 16 x 16 values is one 16-byte word per lane and plane. The four registers
+// of an A operand (rows i, inner index k) in the order 0, 2, 1, 3 are those of
+// two B operands (C = A B^T), so a matrix is stored in the order of the side
+// it stands on ("left" or "right"; X and V stand on both), and no register is
+// moved between a load and the instruction. A result tile has the layout of
+// an A operand, transposed blocks come from movmatrix.
 //
 // Eigenvectors are iterated (Ogita and Aishima, Japan J. Indust. Appl. Math.
 // 35 (2018) 1007, here with the first-order rotation clamped): for approximate
@@ -47,64 +49,125 @@ constexpr int kDigLow = 3;       // digits of the coarse steps and of the rotati
 constexpr int kDrain = 8;        // k blocks of 16 per float32 accumulation
 constexpr int kMaxSteps = 160;   // steps of one eigenproblem before it is given up
 constexpr float kZMax = 0.4f;    // largest rotation of one pair in one step
-constexpr float kZFinal = 0x1p-28f;  // a full step below this is the last (its error is quadratic)
+constexpr float kZNorm = 1.2f;   // largest Frobenius norm (over sqrt 2) of the rotations of a small problem
+constexpr float kZFinal = 0x1p-30f;  // a full step below this is the last (its error is quadratic)
 constexpr float kZLow = 0x1p-10f;    // above this the next step is coarse
 
 __host__ __device__ inline int64_t blocks16(int64_t n) { return (n + 15) / 16; }
 
 __device__ __forceinline__ void mma16816(float *c, const uint4 &a, uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
 }
 
+// A word of planes. Other warps write them in earlier phases: not the
+// read-only path, and volatile so that no load moves across a barrier.
+__device__ __forceinline__ uint4 ld_plane(const uint4 *p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
+__device__ __forceinline__ void st_plane(uint4 *p, const uint4 &v) {
+  asm volatile("st.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(__cvta_generic_to_global(p)), "r"(v.x), "r"(v.y),
+               "r"(v.z), "r"(v.w)
+               : "memory");
+}
+
 // The 16 x 16 tile sum_k A[i][k] B[j][k] over the k blocks [k0, k1) with NP
-// digits: A, B are the first blocks of the two block rows, PA, PB the planes
-// stored per block. t[e], weight 2^-56: row g + 8 ((e >> 1) & 1), column
-// 8 (e >> 2) + 2 q + (e & 1) for lane 4 g + q.
-template <int NP, int PA, int PB>
-__device__ __forceinline__ void tile_nt(const uint4 *A, const uint4 *B, int k0, int k1, long long (&t)[8]) {
+// digits, as the sums of each order (acc[d], weight 2^(-9 (d + 2)), exact
+// integers): A, B are the first blocks of the two block rows, sa, sb the words
+// per block (planes stored x 32). Value e: row g + 8 ((e >> 1) & 1), column
+// 8 (e >> 2) + 2 q + (e & 1) for lane 4 g + q. Every 128 terms the orders are
+// carried into the one above (multiples of 512), which keeps them exact.
+template <int NP>
+__device__ __forceinline__ void tile_nt(const uint4 *A, int sa, const uint4 *B, int sb, int k0, int k1,
+                                        float (&acc)[NP][8]) {
   const int lane = threadIdx.x & 31;
+  const uint4 *pa = A + (size_t)k0 * sa + lane, *pb = B + (size_t)k0 * sb + lane;
 #pragma unroll
-  for (int e = 0; e < 8; ++e) t[e] = 0;
-  for (int kc = k0; kc < k1; kc += kDrain) {
-    float acc[NP][8];
+  for (int p = 0; p < NP; ++p)
 #pragma unroll
-    for (int p = 0; p < NP; ++p)
+    for (int e = 0; e < 8; ++e) acc[p][e] = 0.0f;
+  int left = kDrain;
+  constexpr int kUnroll = NP == kDigLow ? 2 : 1;  // loads of two k blocks in flight where registers allow
+#pragma unroll kUnroll
+  for (int kb = k0; kb < k1; ++kb) {
+    uint4 a[NP];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[p][e] = 0.0f;
-    const int ke = min(kc + kDrain, k1);
-    const uint4 *pa = A + (size_t)kc * PA * 32 + lane, *pb = B + (size_t)kc * PB * 32 + lane;
-#pragma unroll 1
-    for (int kb = kc; kb < ke; ++kb) {
-      uint4 a[NP];
+    for (int p = 0; p < NP; ++p) a[p] = ld_plane(pa + p * 32);
 #pragma unroll
-      for (int p = 0; p < NP; ++p) a[p] = pa[p * 32];
+    for (int q = 0; q < NP; ++q) {
+      const uint4 b = ld_plane(pb + q * 32);
 #pragma unroll
-      for (int q = 0; q < NP; ++q) {
-        const uint4 b = pb[q * 32];
-#pragma unroll
-        for (int p = 0; p < NP - q; ++p) {
-          mma16816(acc[p + q], a[p], b.x, b.z);
-          mma16816(acc[p + q] + 4, a[p], b.y, b.w);
-        }
-      }
-      pa += PA * 32;
-      pb += PB * 32;
-    }
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      // orders 0..2 have weights 2^-18, 2^-27, 2^-36, orders 3..5 2^-45 .. 2^-63
-      const long long hi = (long long)__float2int_rn(acc[0][e]) * (1 << 18) +
-                           (long long)__float2int_rn(acc[1][e]) * (1 << 9) + __float2int_rn(acc[2][e]);
-      t[e] += hi * (1 << 20);
-      if constexpr (NP > 3) {
-        const long long lo = (long long)__float2int_rn(acc[3][e]) * (1 << 18) +
-                             (long long)__float2int_rn(acc[4][e]) * (1 << 9) + __float2int_rn(acc[5][e]);
-        t[e] += (lo + 64) >> 7;
+      for (int p = 0; p < NP - q; ++p) {
+        mma16816(acc[p + q], a[p], b.x, b.y);
+        mma16816(acc[p + q] + 4, a[p], b.z, b.w);
       }
     }
+    pa += sa;
+    pb += sb;
+    if (--left == 0) {
+      left = kDrain;
+      if (kb + 1 < k1) {
+#pragma unroll
+        for (int p = NP - 1; p > 0; --p)
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const float c = fmaf(acc[p][e], 0x1p-9f, 0x1.8p23f) - 0x1.8p23f;  // rounded to an integer
+            acc[p - 1][e] += c;
+            acc[p][e] = fmaf(-512.0f, c, acc[p][e]);
+          }
+      }
+    }
+  }
+}
+
+// x rounded to an integer (|x| < 2^22)
+__device__ __forceinline__ float rint_f(float x) { return (x + 0x1.8p23f) - 0x1.8p23f; }
+// an integer in float32 (|x| < 2^22) as an int: no conversion (those run at
+// an eighth of the rate)
+__device__ __forceinline__ int int_f(float x) { return __float_as_int(x + 0x1.8p23f) - 0x4b400000; }
+
+// A tile's value e less one (where asked) in float32: where the leading orders
+// cancel the partial results are exact integers, so the error is relative.
+template <int NP>
+__device__ __forceinline__ float tile_float(const float (&acc)[NP][8], int e, bool less_one) {
+  float v = less_one ? acc[0][e] - 0x1p18f : acc[0][e];
+#pragma unroll
+  for (int p = 1; p < NP; ++p) v = fmaf(v, 512.0f, acc[p][e]);
+  return v * (NP == 6 ? 0x1p-63f : 0x1p-36f);
+}
+
+// A tile's value e as the NP digits of an operand, and the rest below the last
+// (weight 2^(-9 (NP + 1)), |rest| <= 256). Carries in float32, all exact.
+template <int NP>
+__device__ __forceinline__ float tile_digits(const float (&acc)[NP][8], int e, float (&d)[NP]) {
+  float c = fmaf(acc[NP - 1][e], 0x1p-9f, 0x1.8p23f) - 0x1.8p23f;
+  const float rest = fmaf(-512.0f, c, acc[NP - 1][e]);
+#pragma unroll
+  for (int i = NP - 1; i > 0; --i) {
+    const float x = acc[i - 1][e] + c;
+    c = fmaf(x, 0x1p-9f, 0x1.8p23f) - 0x1.8p23f;
+    d[i] = fmaf(-512.0f, c, x);
+  }
+  d[0] = c;
+  return rest;
+}
+
+// A tile's value e as an integer of weight 2^-56.
+template <int NP>
+__device__ __forceinline__ long long tile_fix(const float (&acc)[NP][8], int e) {
+  float d[NP];
+  const float rest = tile_digits<NP>(acc, e, d);
+  const int hi = (int_f(d[0]) * 512 + int_f(d[1])) * 512 + int_f(d[2]);  // weight 2^-27
+  if constexpr (NP > 3) {
+    const int lo = ((int_f(d[3]) * 512 + int_f(d[4])) * 512 + int_f(d[5])) * 4 + int_f(fmaf(rest, 0x1p-7f, 0.0f));
+    return (long long)hi * (1 << 29) + lo;
+  } else {
+    return (long long)hi * (1 << 29) + int_f(rest) * (1 << 20);
   }
 }
 
@@ -152,11 +215,52 @@ __device__ __forceinline__ void cut_block(const long long (&r)[8], uint32_t (&w)
   }
 }
 
+// Digit words of values of weight 2^-27.
+__device__ __forceinline__ void cut_words(const int (&r)[8], uint32_t (&w)[kDigLow][4]) {
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    int d[2][3];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int x = r[2 * h + k], y1 = (x + 256) >> 9, y2 = (y1 + 256) >> 9;
+      d[k][2] = x - (y1 << 9);
+      d[k][1] = y1 - (y2 << 9);
+      d[k][0] = y2;
+    }
+    w[0][h] = pack_first(d[0][0], d[1][0]);
+    w[1][h] = pack_small(d[0][1], d[1][1]);
+    w[2][h] = pack_small(d[0][2], d[1][2]);
+  }
+}
+
+// Digit words from a result tile.
 template <int NP>
-__device__ __forceinline__ void put_block(uint4 *blk, const uint32_t (&w)[NP][4]) {
+__device__ __forceinline__ void tile_words(const float (&acc)[NP][8], uint32_t (&w)[NP][4]) {
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    float a[NP], b[NP];
+    tile_digits<NP>(acc, 2 * h, a);
+    tile_digits<NP>(acc, 2 * h + 1, b);
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const __half2 x = __floats2half2_rn(a[p], b[p]);
+      w[p][h] = *reinterpret_cast<const uint32_t *>(&x);
+    }
+  }
+}
+
+// A block of planes for the left (A) or the right (B) side of a product.
+template <int NP>
+__device__ __forceinline__ void put_left(uint4 *blk, const uint32_t (&w)[NP][4]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int p = 0; p < NP; ++p) blk[p * 32 + lane] = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+  for (int p = 0; p < NP; ++p) st_plane(blk + p * 32 + lane, make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]));
+}
+template <int NP>
+__device__ __forceinline__ void put_right(uint4 *blk, const uint32_t (&w)[NP][4]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int p = 0; p < NP; ++p) st_plane(blk + p * 32 + lane, make_uint4(w[p][0], w[p][2], w[p][1], w[p][3]));
 }
 
 __device__ __forceinline__ uint32_t transpose8(uint32_t v) {
@@ -167,11 +271,20 @@ __device__ __forceinline__ uint32_t transpose8(uint32_t v) {
 
 // The first NP planes of a block's digit words as the transposed block.
 template <int NP, int NW>
-__device__ __forceinline__ void put_block_t(uint4 *blk, const uint32_t (&w)[NW][4]) {
+__device__ __forceinline__ void put_left_t(uint4 *blk, const uint32_t (&w)[NW][4]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int p = 0; p < NP; ++p)
-    blk[p * 32 + lane] = make_uint4(transpose8(w[p][0]), transpose8(w[p][2]), transpose8(w[p][1]), transpose8(w[p][3]));
+    st_plane(blk + p * 32 + lane,
+             make_uint4(transpose8(w[p][0]), transpose8(w[p][2]), transpose8(w[p][1]), transpose8(w[p][3])));
+}
+template <int NP, int NW>
+__device__ __forceinline__ void put_right_t(uint4 *blk, const uint32_t (&w)[NW][4]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int p = 0; p < NP; ++p)
+    st_plane(blk + p * 32 + lane,
+             make_uint4(transpose8(w[p][0]), transpose8(w[p][1]), transpose8(w[p][2]), transpose8(w[p][3])));
 }
 
 // x 2^sh rounded to an integer (|result| < 2^62; 0 for a denormal x).
@@ -251,28 +364,46 @@ __device__ Four team_four(Team<CL> &tm, Four v, float4 *sm, float4 *g) {
 }
 // fmaxf drops a NaN: sums carry it, so a caller that must see one looks there.
 
+// 16-byte words of a lower tile's integrals: per lane 8 values (i, j) and
+// their mirrors (j, i), 10 numbers of 8 bytes each
+constexpr int kPairWords = 5 * 2 * 8 * 32;
+
 // Workspace of this path (doubles), np = n rounded up to 16.
-__host__ __device__ inline int64_t fast_size(int64_t n) {
+__host__ __device__ inline int64_t fast_size(int64_t n, int64_t nat) {
   const int64_t nb = blocks16(n), np2 = 256 * nb * nb;
-  // planes of six digits are 12 bytes a value (3/2 doubles), of three 3/4
-  return (5 * 3 * np2) / 2 + (3 * 3 * np2) / 4 + 2 * np2 + 6 * 16 * nb + 64 + 64;
+  // planes of six digits are 12 bytes a value (3/2 doubles), of three 3/4;
+  // the integrals S, D, Q in fixed point; potential and population tables
+  return (7 * 3 * np2) / 2 + (3 * 3 * np2) / 4 + 2 * np2 + 6 * 16 * nb + 64 + 64 +
+         nb * (nb + 1) / 2 * kPairWords * 2 + (n + 9 * nat) + 10 * n + 8;
 }
 
+// One copy per CTA in shared memory: as a local variable handed to functions
+// its 300 bytes a thread filled the L1. Written by thread 0 between barriers.
 struct Fast {
   int nb;
-  uint4 *Xp, *XTp, *Fp, *Gp, *Vp, *VT[2], *Ep;
+  uint4 *Xl, *Xr, *XTl;      // X = L^-1 for both sides, X^T for the left
+  uint4 *Fr, *Gl;            // F, F', weighted C^T (right); H, G, C^T (left)
+  uint4 *Vl, *Vr, *VT[2], *El;  // V for both sides, V^T (right), E^T (left)
   long long *Vm, *Vm2;       // vectors, weight 2^-60, tile layout
   float *T, *R;              // tile layout (Vm2's memory)
   long long *td, *rd;        // diagonals of T and R
   double *lam;               // eigenvalue of each row of V
   int *xe, *xte, *inv;       // row exponents of X and X^T; row order
   float4 *red;
+  long long *Ft;             // F and F' in fixed point, lower tiles (Vm2's memory)
+  int4 *M;                   // S, D (3), Q (6) in fixed point, lower tiles: [5][pair, mirror][8][lane]
+  long long *vo;             // orbital potential in fixed point
+  int2 *vm;                  // atomic dipole and quadrupole potential, [9][nat]
+  long long *pop;            // populations: charge and moments per orbital, [10][n]
+  int eS, eD, eQ, eH;        // |S| <= 2^eS, ...
+  int nat, nm;               // atoms; 10 matrices in M, or 1 without multipoles
+  int xtm;                   // largest xte
   int cur;                   // VT in use
   bool warm;                 // V holds vectors of an earlier problem
   float z0;                  // first rotation of the last problem
 };
 
-__device__ inline Fast fast_carve(double *base, int n) {
+__device__ inline Fast fast_carve(double *base, int n, int nat, bool multipole) {
   Fast f;
   const int64_t nb = blocks16(n), np2 = 256 * nb * nb;
   f.nb = (int)nb;
@@ -283,14 +414,16 @@ __device__ inline Fast fast_carve(double *base, int n) {
     q += bytes;
     return r;
   };
-  f.Xp = (uint4 *)take(12 * np2);
-  f.XTp = (uint4 *)take(12 * np2);
-  f.Fp = (uint4 *)take(12 * np2);
-  f.Gp = (uint4 *)take(12 * np2);
-  f.Vp = (uint4 *)take(12 * np2);
+  f.Xl = (uint4 *)take(12 * np2);
+  f.Xr = (uint4 *)take(12 * np2);
+  f.XTl = (uint4 *)take(12 * np2);
+  f.Fr = (uint4 *)take(12 * np2);
+  f.Gl = (uint4 *)take(12 * np2);
+  f.Vl = (uint4 *)take(12 * np2);
+  f.Vr = (uint4 *)take(12 * np2);
   f.VT[0] = (uint4 *)take(6 * np2);
   f.VT[1] = (uint4 *)take(6 * np2);
-  f.Ep = (uint4 *)take(6 * np2);
+  f.El = (uint4 *)take(6 * np2);
   f.Vm = (long long *)take(8 * np2);
   f.Vm2 = (long long *)take(8 * np2);
   f.T = (float *)f.Vm2;
@@ -302,6 +435,14 @@ __device__ inline Fast fast_carve(double *base, int n) {
   f.xe = (int *)take(4 * 16 * nb);
   f.xte = (int *)take(4 * 16 * nb);
   f.inv = (int *)take(4 * 16 * nb);
+  q += (16 - ((uintptr_t)q & 15)) & 15;
+  f.Ft = f.Vm2;
+  f.M = (int4 *)take(nb * (nb + 1) / 2 * kPairWords * 16);
+  f.vo = (long long *)take(8 * (int64_t)n);
+  f.vm = (int2 *)take(8 * 9 * (int64_t)nat);
+  f.pop = (long long *)take(8 * 10 * (int64_t)n);
+  f.nat = nat;
+  f.nm = multipole ? 10 : 1;
   f.cur = 0;
   f.warm = false;
   f.z0 = 1.0f;
@@ -333,9 +474,10 @@ __device__ __forceinline__ int tile_row(int e) { return ((threadIdx.x & 31) >> 2
 __device__ __forceinline__ int tile_col(int e) { return 8 * (e >> 2) + 2 * (threadIdx.x & 3) + (e & 1); }
 
 // Digit planes of the row-major n x n matrix M (TR: of its transpose) whose
-// row i is scaled by 2^-s(i).
-template <bool TR, bool CL, typename S>
-__device__ __noinline__ void planes_of(Team<CL> &tm, int n, int nb, const double *M, uint4 *out, S s) {
+// row i is scaled by 2^-e[i], for the left side and, if given, the right.
+template <bool TR, bool CL>
+__device__ __noinline__ void planes_of(Team<CL> &tm, int n, int nb, const double *M, uint4 *left, uint4 *right,
+                                       const int *ex) {
   for (int t = team_warp(tm); t < nb * nb; t += team_warps(tm)) {
     const int ti = t / nb, tj = t % nb;
     long long r[8];
@@ -343,30 +485,87 @@ __device__ __noinline__ void planes_of(Team<CL> &tm, int n, int nb, const double
     for (int e = 0; e < 8; ++e) {
       const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
       r[e] = 0;
-      if (i < n && j < n) r[e] = fix(ld<CL>(TR ? M + (size_t)j * n + i : M + (size_t)i * n + j), 54 - s(i));
+      if (i < n && j < n) r[e] = fix(ld<CL>(TR ? M + (size_t)j * n + i : M + (size_t)i * n + j), 54 - ldi<CL>(ex + i));
     }
     uint32_t w[kDig][4];
     cut_block<kDig>(r, w);
-    put_block<kDig>(out + (size_t)t * kDig * 32, w);
+    put_left<kDig>(left + (size_t)t * kDig * 32, w);
+    if (right != nullptr) put_right<kDig>(right + (size_t)t * kDig * 32, w);
   }
 }
 
-// Largest row sum of |M| (row-major, n x n) over the team; NaN or infinity
-// gives a value that is not finite. Ends with a team barrier.
+// |x| in float32, rounded up; infinity for |x| >= 2^127 and for a NaN. No
+// FP64 instruction.
+__device__ __forceinline__ float mag(double x) {
+  const int hi = __double2hiint(x) & 0x7fffffff;
+  if (hi >= 0x47e00000) return INFINITY;
+  return hi < 0x38100000 ? 0.0f : __int_as_float(((hi - 0x38000000) << 3) + 8);
+}
+
+// Fixed point with 53 bits in two signed halves: h 2^28 + l.
+__device__ __forceinline__ int2 halves(long long m) {
+  const int h = (int)((m + (1 << 27)) >> 28);
+  return make_int2(h, (int)(m - ((long long)h << 28)));
+}
+
+// A product of two such numbers without its low x low part (2^-50 of a unit
+// of h x h): three 32-bit multiply-adds in place of a float64 one, which
+// costs nineteen times an IMAD's issue on this part.
+__device__ __forceinline__ void mul_add(long long &a0, long long &a1, int2 x, int2 y) {
+  a0 += (long long)x.x * y.x;
+  a1 += (long long)x.x * y.y;
+  a1 += (long long)x.y * y.x;
+}
+
+// S, D, Q in fixed point with their exponents (the factors of the Fock build
+// and of the populations). False if an entry is not finite. Once per geometry.
 template <bool CL>
-__device__ float team_inf_norm(Team<CL> &tm, int n, const double *M, float4 *sm, float4 *g) {
-  const int lane = threadIdx.x & 31;
-  float mx = 0.0f, all = 0.0f;
-  for (int i = team_warp(tm); i < n; i += team_warps(tm)) {
-    float s = 0.0f;
-    for (int j = lane; j < n; j += 32) s += fabsf((float)ld<CL>(M + (size_t)i * n + j));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    mx = fmaxf(mx, s);
-    all += s;
+__device__ __noinline__ bool fast_integrals(Team<CL> &tm, int n, Fast &f, const double *S, const double *H0,
+                                            const double *D, const double *Q, int64_t mtot, float4 *sm) {
+  const int64_t n2 = (int64_t)n * n;
+  Four v = {0.0f, 0.0f, 0.0f, 0.0f};
+  float h = 0.0f, s = 0.0f;
+  for (int64_t t = tm.tid; t < n2; t += tm.nthr) {
+    s = fmaxf(s, mag(S[t]));
+    h = fmaxf(h, mag(H0[t]));
+    if (f.nm > 1) {
+      for (int c = 0; c < 3; ++c) v.m0 = fmaxf(v.m0, mag(D[c * mtot + t]));
+      for (int c = 0; c < 6; ++c) v.m1 = fmaxf(v.m1, mag(Q[c * mtot + t]));
+    }
   }
-  const Four f = team_four(tm, Four{mx, 0.0f, lane == 0 ? all : 0.0f, 0.0f}, sm, g);
-  return isfinite(f.s0) ? f.m0 : f.s0;
+  const Four a = team_four(tm, v, sm, f.red), b = team_four(tm, Four{s, h, 0.0f, 0.0f}, sm, f.red);
+  if (!(fmaxf(fmaxf(a.m0, a.m1), fmaxf(b.m0, b.m1)) < 0x1p60f)) return false;
+  auto ex = [](float m) { return m > 0x1p-40f ? exp_above(m) : -40; };
+  if (threadIdx.x == 0) {
+    f.eS = ex(b.m0);
+    f.eH = ex(b.m1);
+    f.eD = ex(a.m0);
+    f.eQ = ex(a.m1);
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, nlow = f.nb * (f.nb + 1) / 2;
+  for (int t = team_warp(tm); t < nlow; t += team_warps(tm)) {
+    int ti, tj;
+    lower_tile(t, ti, tj);
+    for (int e = 0; e < 8; ++e) {
+      const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
+      const bool in = i < n && j < n;
+      for (int y = 0; y < (f.nm > 1 ? 2 : 1); ++y) {
+        const int64_t o = y ? (int64_t)j * n + i : (int64_t)i * n + j;
+        int2 m[10];
+        m[0] = halves(in ? fix(S[o], 53 - f.eS) : 0);
+        int4 *out = f.M + (size_t)t * kPairWords + (y * 8 + e) * 32 + lane;
+        if (f.nm > 1) {
+          for (int c = 0; c < 3; ++c) m[1 + c] = halves(in ? fix(D[c * mtot + o], 53 - f.eD) : 0);
+          for (int c = 0; c < 6; ++c) m[4 + c] = halves(in ? fix(Q[c * mtot + o], 53 - f.eQ) : 0);
+          for (int c = 0; c < 5; ++c) out[c * 512] = make_int4(m[2 * c].x, m[2 * c].y, m[2 * c + 1].x, m[2 * c + 1].y);
+        } else {
+          *out = make_int4(m[0].x, m[0].y, 0, 0);
+        }
+      }
+    }
+  }
+  return true;
 }
 
 // Planes of X = L^-1 and of its transpose, rows scaled to a 2-norm in
@@ -374,7 +573,7 @@ __device__ float team_inf_norm(Team<CL> &tm, int n, const double *M, float4 *sm,
 template <bool CL>
 __device__ __noinline__ bool fast_setup(Team<CL> &tm, int n, const double *X, Fast &f, float4 *sm) {
   const int lane = threadIdx.x & 31;
-  float bad = 0.0f;
+  float bad = 0.0f, top = 0.0f;
   for (int q = team_warp(tm); q < 2 * n; q += team_warps(tm)) {
     const int i = q >> 1;
     const bool tr = q & 1;
@@ -388,12 +587,15 @@ __device__ __noinline__ bool fast_setup(Team<CL> &tm, int n, const double *X, Fa
     const float nrm = sqrtf(s) * 1.000001f;
     const bool ok = nrm > 0x1p-60f && nrm < 0x1p60f;
     if (!ok) bad = 1.0f;
-    if (lane == 0) (tr ? f.xte : f.xe)[i] = ok ? exp_above(nrm) : 0;
+    const int ex = ok ? exp_above(nrm) : 0;
+    if (tr) top = fmaxf(top, (float)(ex + 128));
+    if (lane == 0) (tr ? f.xte : f.xe)[i] = ex;
   }
-  const Four r = team_four(tm, Four{bad, 0.0f, 0.0f, 0.0f}, sm, f.red);
+  const Four r = team_four(tm, Four{bad, top, 0.0f, 0.0f}, sm, f.red);
   if (r.m0 > 0.0f) return false;
-  planes_of<false>(tm, n, f.nb, X, f.Xp, [&](int i) { return ldi<CL>(f.xe + i); });
-  planes_of<true>(tm, n, f.nb, X, f.XTp, [&](int i) { return ldi<CL>(f.xte + i); });
+  if (threadIdx.x == 0) f.xtm = (int)r.m1 - 128;
+  planes_of<false>(tm, n, f.nb, X, f.Xl, f.Xr, f.xe);
+  planes_of<true>(tm, n, f.nb, X, f.XTl, (uint4 *)nullptr, f.xte);
   tm.sync();
   return true;
 }
@@ -414,67 +616,188 @@ __device__ __noinline__ void fast_identity(Team<CL> &tm, int n, Fast &f) {
     }
     uint32_t w[kDig][4];
     cut_block<kDig>(r, w);
-    put_block<kDig>(f.Vp + (size_t)t * kDig * 32, w);
-    put_block_t<kDigLow>(f.VT[0] + ((size_t)tj * nb + ti) * kDigLow * 32, w);
+    put_left<kDig>(f.Vl + (size_t)t * kDig * 32, w);
+    put_right<kDig>(f.Vr + (size_t)t * kDig * 32, w);
+    put_right_t<kDigLow>(f.VT[0] + ((size_t)tj * nb + ti) * kDigLow * 32, w);
   }
-  f.cur = 0;
+  if (threadIdx.x == 0) f.cur = 0;
   tm.sync();
 }
 
-// One step's G = V F and R = I - V V^T (lower tiles).
-template <int NP, bool CL>
-__device__ __noinline__ void step_products(Team<CL> &tm, int n, const Fast &f) {
-  const int nb = f.nb, nlow = nb * (nb + 1) / 2, lane = threadIdx.x & 31;
-  for (int t = team_warp(tm); t < nb * nb + nlow; t += team_warps(tm)) {
-    long long c[8];
-    if (t < nb * nb) {
-      const int ti = t / nb, tj = t % nb;
-      tile_nt<NP, kDig, kDig>(f.Vp + (size_t)ti * nb * kDig * 32, f.Fp + (size_t)tj * nb * kDig * 32, 0, nb, c);
+// Lower tiles of a symmetric matrix in fixed point: value e of lane l of tile t.
+__device__ __forceinline__ void put_tile(long long *F, int t, const long long (&v)[8]) {
+  longlong2 *out = reinterpret_cast<longlong2 *>(F) + (size_t)t * 128 + (threadIdx.x & 31);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) c[e] = (c[e] + 2) >> 2;
-      uint32_t w[NP][4];
-      cut_block<NP>(c, w);
-      put_block<NP>(f.Gp + (size_t)t * kDig * 32, w);
+  for (int h = 0; h < 4; ++h) out[32 * h] = make_longlong2(v[2 * h], v[2 * h + 1]);
+}
+__device__ __forceinline__ void get_tile(const long long *F, int t, long long (&v)[8]) {
+  const longlong2 *in = reinterpret_cast<const longlong2 *>(F) + (size_t)t * 128 + (threadIdx.x & 31);
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    const longlong2 x = in[32 * h];
+    v[2 * h] = x.x;
+    v[2 * h + 1] = x.y;
+  }
+}
+
+__device__ __forceinline__ long long shift(long long x, int left) {
+  if (left >= 0) return x << min(left, 62);
+  return left < -62 ? 0 : (x + (1ll << (-left - 1))) >> -left;
+}
+
+// The products of a step, a Fock build and a density: which tiles, what
+// becomes of a result. One function per digit count: the instruction cache
+// does not hold a copy of the tile loop for each product.
+enum Product : int {
+  kStep,    // G = V F (planes), R = I - V V^T (float32, lower tiles)
+  kProject, // T = G V^T (float32, lower tiles)
+  kApply,   // V <- V + E^T V, planes of V and of its transpose
+  kHalf,    // H = X F (planes), X lower triangular
+  kFockX,    // F' = H X^T (fixed point, lower tiles)
+  kCoeff,   // C^T = X^T V^T (planes), the mo lowest vectors
+  kDensity, // P = C w C^T (fixed point, lower tiles)
+  kWeighted // the same in float64, both triangles
+};
+
+template <int NP, bool CL>
+__device__ __noinline__ float tiles(Team<CL> &tm, int n, const Fast &f, Product what, int arg, int arg2, double *out) {
+  const int nb = f.nb, nlow = nb * (nb + 1) / 2, lane = threadIdx.x & 31;
+  const bool dens = what == kDensity || what == kWeighted;
+  const int mb = what == kCoeff || dens ? (int)blocks16(arg) : nb;
+  constexpr int S6 = kDig * 32, S3 = kDigLow * 32;
+  const int row6 = nb * S6, row3 = nb * S3;
+  const uint4 *VT = f.VT[f.cur];
+  uint4 *VN = f.VT[f.cur ^ 1];
+  const int ntile = what == kStep                      ? nb * nb + nlow
+                    : what == kApply || what == kHalf  ? nb * nb
+                    : what == kCoeff                   ? nb * mb
+                                                       : nlow;
+  float sum = 0.0f;
+  for (int t = team_warp(tm); t < ntile; t += team_warps(tm)) {
+    int ti, tj, k0 = 0, k1 = nb, sa = S6, sb = S6;
+    const uint4 *A, *B;
+    bool square = false;  // a tile of the full matrix (else of the lower triangle)
+    if (what == kApply || what == kHalf || (what == kStep && t < nb * nb)) {
+      ti = t / nb;
+      tj = t - ti * nb;
+      square = true;
+    } else if (what == kCoeff) {
+      ti = t / mb;
+      tj = t - ti * mb;
+      square = true;
     } else {
-      int ti, tj;
-      lower_tile(t - nb * nb, ti, tj);
-      tile_nt<NP, kDig, kDig>(f.Vp + (size_t)ti * nb * kDig * 32, f.Vp + (size_t)tj * nb * kDig * 32, 0, nb, c);
-      float4 *out = reinterpret_cast<float4 *>(f.R) + (size_t)(t - nb * nb) * 64 + lane;
+      lower_tile(what == kStep ? t - nb * nb : t, ti, tj);
+    }
+    if (what == kHalf) {
+      ti = nb - 1 - ti;  // the long rows first
+      k1 = ti + 1;
+    }
+    if (what == kCoeff) k0 = ti;
+    if (what == kFockX) k1 = tj + 1;
+    if (dens) k1 = mb;
+    if (what == kApply) {
+      sa = sb = S3;
+      A = f.El + (size_t)ti * row3;
+      B = VT + (size_t)tj * row3;
+    } else {
+      A = (what == kStep ? f.Vl : what == kHalf ? f.Xl : what == kCoeff ? f.XTl : f.Gl) + (size_t)ti * row6;
+      B = (what == kStep ? (square ? f.Fr : f.Vr)
+           : what == kHalf || dens ? f.Fr
+           : what == kFockX ? f.Xr : f.Vr) + (size_t)tj * row6;
+    }
+    longlong2 vm[4];  // kApply: the vectors to update, loaded ahead
+    if (NP == kDigLow && what == kApply) {
+      const longlong2 *pv = reinterpret_cast<const longlong2 *>(f.Vm) + (size_t)t * 128 + lane;
+#pragma unroll
+      for (int h = 0; h < 4; ++h) vm[h] = pv[32 * h];
+    }
+    float acc[NP][8];
+    tile_nt<NP>(A, sa, B, sb, k0, k1, acc);
+    const size_t blk = (size_t)ti * row6 + (size_t)tj * S6;
+    if (NP == kDigLow && what == kApply) {
+      longlong2 *pv = reinterpret_cast<longlong2 *>(f.Vm) + (size_t)t * 128 + lane;
+      long long c[8];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        longlong2 v = vm[h];
+        v.x += shift(tile_fix(acc, 2 * h), 4 - arg);  // weight 2^-56 2^-ke to 2^-60
+        v.y += shift(tile_fix(acc, 2 * h + 1), 4 - arg);
+        pv[32 * h] = v;
+        c[2 * h] = (v.x + 32) >> 6;
+        c[2 * h + 1] = (v.y + 32) >> 6;
+      }
+      uint4 *vt = VN + (size_t)tj * row3 + (size_t)ti * S3;
+      if (arg2) {
+        uint32_t w[kDig][4];
+        cut_block<kDig>(c, w);
+        put_left<kDig>(f.Vl + blk, w);
+        put_right<kDig>(f.Vr + blk, w);
+        put_right_t<kDigLow>(vt, w);
+      } else {
+        uint32_t w[kDigLow][4];
+        cut_block<kDigLow>(c, w);
+        put_left<kDigLow>(f.Vl + blk, w);
+        put_right<kDigLow>(f.Vr + blk, w);
+        put_right_t<kDigLow>(vt, w);
+      }
+    } else if (square) {
+      uint32_t w[NP][4];
+      tile_words<NP>(acc, w);
+      put_left<NP>(f.Gl + blk, w);
+    } else if (what == kStep || what == kProject) {
+      const bool isr = what == kStep;
+      const int tl = isr ? t - nb * nb : t;
+      float4 *o = reinterpret_cast<float4 *>(isr ? f.R : f.T) + (size_t)tl * 64 + lane;
       float r[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
-        const long long v = (i == j && i < n) ? (1ll << 56) - c[e] : -c[e];
-        r[e] = fix_to_float(v);
-        if (i == j) f.rd[i] = v;
+        const bool one = isr && ti == tj && tile_row(e) == tile_col(e) && 16 * ti + tile_row(e) < n;
+        r[e] = tile_float(acc, e, one);
+        if (isr) r[e] = -r[e];
       }
-      out[0] = make_float4(r[0], r[1], r[2], r[3]);
-      out[32] = make_float4(r[4], r[5], r[6], r[7]);
-    }
-  }
-  tm.sync();
-}
-
-// T = G V^T (lower tiles).
-template <int NP, bool CL>
-__device__ __noinline__ void step_project(Team<CL> &tm, const Fast &f) {
-  const int nb = f.nb, nlow = nb * (nb + 1) / 2, lane = threadIdx.x & 31;
-  for (int t = team_warp(tm); t < nlow; t += team_warps(tm)) {
-    int ti, tj;
-    lower_tile(t, ti, tj);
-    long long c[8];
-    tile_nt<NP, kDig, kDig>(f.Gp + (size_t)ti * nb * kDig * 32, f.Vp + (size_t)tj * nb * kDig * 32, 0, nb, c);
-    float4 *out = reinterpret_cast<float4 *>(f.T) + (size_t)t * 64 + lane;
-    float r[8];
+      o[0] = make_float4(r[0], r[1], r[2], r[3]);
+      o[32] = make_float4(r[4], r[5], r[6], r[7]);
+      if (ti == tj) {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      r[e] = fix_to_float(c[e]);
-      if (ti == tj && tile_row(e) == tile_col(e)) f.td[16 * ti + tile_row(e)] = c[e];
+        for (int e = 0; e < 8; ++e) {
+          const int i = 16 * ti + tile_row(e);
+          if (tile_row(e) == tile_col(e)) {
+            const long long v = tile_fix(acc, e);
+            if (isr) f.rd[i] = (i < n ? (1ll << 56) : 0) - v; else f.td[i] = v;
+          }
+        }
+      }
+    } else if (what == kFockX) {
+      long long c[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        c[e] = tile_fix(acc, e);
+        const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
+        if (i < n && j < n) {
+          const float y = ldexpf(tile_float(acc, e, false), f.xe[i] + f.xe[j]);
+          sum = fmaf(ti == tj ? y : 2.0f * y, y, sum);
+        }
+      }
+      put_tile(f.Ft, t, c);
+    } else if (what == kDensity) {
+      long long c[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) c[e] = tile_fix(acc, e);
+      put_tile(f.Ft, t, c);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
+        if (i < n && j <= i) {
+          const double v = unfix(tile_fix(acc, e), f.xte[i] + f.xte[j] + arg2 - 56);
+          out[(size_t)i * n + j] = v;
+          out[(size_t)j * n + i] = v;
+        }
+      }
     }
-    out[0] = make_float4(r[0], r[1], r[2], r[3]);
-    out[32] = make_float4(r[4], r[5], r[6], r[7]);
   }
-  tm.sync();
+  if (what != kFockX) tm.sync();
+  return sum;
 }
 
 // Rotations Z of the lower tiles over T, with the figures that scale them.
@@ -551,55 +874,20 @@ __device__ __noinline__ void step_update_planes(Team<CL> &tm, int n, const Fast 
     *reinterpret_cast<float4 *>(z + 4) = pt[32];
     *reinterpret_cast<float4 *>(r) = pr[0];
     *reinterpret_cast<float4 *>(r + 4) = pr[32];
-    long long a[8], b[8];
+    int a[8], b[8];  // weight 2^-27; zero outside the matrix
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
-      const bool in = i < n && j < n;
-      a[e] = in ? (long long)__float2int_rn(fmaf(-sc, z[e], 0.5f * r[e]) * up) << 27 : 0;  // E_ji
-      b[e] = in ? (long long)__float2int_rn(fmaf(sc, z[e], 0.5f * r[e]) * up) << 27 : 0;   // E_ij
+      a[e] = __float2int_rn(fmaf(-sc, z[e], 0.5f * r[e]) * up);  // E_ji
+      b[e] = __float2int_rn(fmaf(sc, z[e], 0.5f * r[e]) * up);   // E_ij
     }
     uint32_t w[kDigLow][4];
-    cut_block<kDigLow>(a, w);
-    put_block<kDigLow>(f.Ep + ((size_t)ti * nb + tj) * kDigLow * 32, w);
+    cut_words(a, w);
+    put_left<kDigLow>(f.El + ((size_t)ti * nb + tj) * kDigLow * 32, w);
     if (ti != tj) {
-      cut_block<kDigLow>(b, w);
-      put_block_t<kDigLow>(f.Ep + ((size_t)tj * nb + ti) * kDigLow * 32, w);
+      cut_words(b, w);
+      put_left_t<kDigLow>(f.El + ((size_t)tj * nb + ti) * kDigLow * 32, w);
     }
   }
-  tm.sync();
-}
-
-// V <- V + E^T V; NP planes of the new V (3 for a coarse next step) and the
-// three of its transpose in the other buffer.
-template <int NP, bool CL>
-__device__ __noinline__ void step_apply(Team<CL> &tm, Fast &f, int ke) {
-  const int nb = f.nb, lane = threadIdx.x & 31;
-  const uint4 *VT = f.VT[f.cur];
-  uint4 *VN = f.VT[f.cur ^ 1];
-  for (int t = team_warp(tm); t < nb * nb; t += team_warps(tm)) {
-    const int ti = t / nb, tj = t % nb;
-    long long c[8];
-    tile_nt<kDigLow, kDigLow, kDigLow>(f.Ep + (size_t)ti * nb * kDigLow * 32, VT + (size_t)tj * nb * kDigLow * 32, 0,
-                                       nb, c);
-    longlong2 *pv = reinterpret_cast<longlong2 *>(f.Vm) + (size_t)t * 128 + lane;
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      longlong2 v = pv[32 * h];
-      const int sh = ke - 4;  // weight 2^-56 2^-ke to 2^-60
-      auto move = [&](long long x) { return sh > 0 ? (x + (1ll << (sh - 1))) >> sh : x << -sh; };
-      v.x += move(c[2 * h]);
-      v.y += move(c[2 * h + 1]);
-      pv[32 * h] = v;
-      c[2 * h] = (v.x + 32) >> 6;
-      c[2 * h + 1] = (v.y + 32) >> 6;
-    }
-    uint32_t w[NP][4];
-    cut_block<NP>(c, w);
-    put_block<NP>(f.Vp + (size_t)t * kDig * 32, w);
-    put_block_t<kDigLow>(VN + ((size_t)tj * nb + ti) * kDigLow * 32, w);
-  }
-  f.cur ^= 1;
   tm.sync();
 }
 
@@ -648,121 +936,411 @@ __device__ __noinline__ void fast_sort(Team<CL> &tm, int n, Fast &f, double *lam
     }
     uint32_t w[kDig][4];
     cut_block<kDig>(v, w);
-    put_block<kDig>(f.Vp + (size_t)t * kDig * 32, w);
-    put_block_t<kDigLow>(f.VT[f.cur ^ 1] + ((size_t)tj * nb + ti) * kDigLow * 32, w);
+    put_left<kDig>(f.Vl + (size_t)t * kDig * 32, w);
+    put_right<kDig>(f.Vr + (size_t)t * kDig * 32, w);
+    put_right_t<kDigLow>(f.VT[f.cur ^ 1] + ((size_t)tj * nb + ti) * kDigLow * 32, w);
   }
-  f.cur ^= 1;
-  long long *sw = f.Vm;
-  f.Vm = f.Vm2;
-  f.Vm2 = sw;
-  f.T = reinterpret_cast<float *>(f.Vm2);
-  f.R = f.T + (size_t)256 * nb * nb;
   tm.sync();
+  if (threadIdx.x == 0) {
+    f.cur ^= 1;
+    long long *sw = f.Vm;
+    f.Vm = f.Vm2;
+    f.Vm2 = sw;
+    f.Ft = sw;
+    f.T = reinterpret_cast<float *>(f.Vm2);
+    f.R = f.T + (size_t)256 * nb * nb;
+  }
+  __syncthreads();
 }
 
 // Eigenvectors (rows of V, ascending) and eigenvalues (lam, shared, every
 // CTA; in units of 2^s) of the matrix whose planes, scaled by 2^-s to a
-// row-sum norm in (1, 2], are in f.Fp. False when the steps do not converge.
+// Frobenius norm in (1, 2], are in f.Fr. False when the steps do not converge.
 template <bool CL>
 __device__ bool fast_eigen(Team<CL> &tm, int n, Fast &f, double *lam, double *sk, float *lh, float *ll, float4 *sm) {
-  if (!f.warm) fast_identity(tm, n, f);
+  const bool warm = f.warm;
+  const float z0 = f.z0;
+  __syncthreads();
+  if (threadIdx.x == 0) f.warm = false;
+  if (!warm) fast_identity(tm, n, f);
   // the first rotation shrinks from one problem to the next as the SCF converges
-  bool low = !f.warm || 0.5f * f.z0 > kZLow;
-  f.warm = false;
+  bool low = !warm || 0.5f * z0 > kZLow;
+  float top = fmaxf(kZNorm, 0.2f * sqrtf((float)n)), zprev = 1.0f;
+  bool stalled = false;
   for (int it = 0; it < kMaxSteps; ++it) {
     if (low) {
-      step_products<kDigLow>(tm, n, f);
-      step_project<kDigLow>(tm, f);
+      tiles<kDigLow>(tm, n, f, kStep, 0, 0, nullptr);
+      tiles<kDigLow>(tm, n, f, kProject, 0, 0, nullptr);
     } else {
-      step_products<kDig>(tm, n, f);
-      step_project<kDig>(tm, f);
+      tiles<kDig>(tm, n, f, kStep, 0, 0, nullptr);
+      tiles<kDig>(tm, n, f, kProject, 0, 0, nullptr);
     }
     const Four s = step_rotations(tm, n, f, low, lam, lh, ll, sm);
-    if (!isfinite(s.s0) || !(s.s1 < 1e4f)) return false;
-    // the singular values of I + E stay below sqrt(3), where the R / 2 part
-    // contracts towards orthonormal rows
+    if (!isfinite(s.s0) || !(s.s1 < 1e4f)) {
+      // too large a rotation: once more from the start with the bound that holds for any Z
+      if (!(top > kZNorm)) return false;
+      top = kZNorm;
+      low = true;
+      fast_identity(tm, n, f);
+      continue;
+    }
+    // The singular values of I + E must stay below sqrt(3), where the R / 2
+    // part contracts towards orthonormal rows. kZNorm bounds them for any Z by
+    // its Frobenius norm; the many small rotations of a large problem have a
+    // spectral norm far below that one (0.85 of 3.8 at n = 233), so the bound
+    // grows with sqrt(n): 201 -> 143 coarse steps over an SCF at n = 233.
     const float zf = sqrtf(s.s0), rf = sqrtf(s.s1);
-    const float lim = fmaxf(0.15f, 1.2f - 0.7f * rf);
+    const float lim = fmaxf(0.15f, top - 0.7f * rf);
     const float sc = zf > lim ? lim / zf : 1.0f;
     const float zm = s.m0 * sc;
-    if (it == 0) f.z0 = zm;
+    if (it == 0 && threadIdx.x == 0) f.z0 = zm;
     const bool last = !low && zm < kZFinal && s.m1 < 0x1p-26f;
     const float em = zm + 0.5f * s.m1;
     const int ke = em > 0x1p-50f ? -exp_above(em) : 50;
     step_update_planes(tm, n, f, sc, ke);
-    low = !last && zm > kZLow;
-    if (low) step_apply<kDigLow>(tm, f, ke); else step_apply<kDig>(tm, f, ke);
+    // a coarse step that no longer shrinks the rotations has met its own rounding
+    // (pairs closer than ~2^-17 of the norm): full steps from here on
+    if (low && zm < 0.125f && zm > 0.7f * zprev) stalled = true;
+    zprev = zm;
+    low = !last && !stalled && zm > kZLow;
+    tiles<kDigLow>(tm, n, f, kApply, ke, low ? 0 : 1, nullptr);
+    if (threadIdx.x == 0) f.cur ^= 1;  // read next after further barriers
     if (last) {
       __shared__ int sflag;
       fast_sort(tm, n, f, lam, sk, &sflag);
-      f.warm = true;
+      if (threadIdx.x == 0) f.warm = true;
       return true;
     }
   }
   return false;
 }
 
-// F' = X F X^T into A (both triangles): F (row-major n x n) must be symmetric.
-// Then the planes of F' in f.Fp scaled by 2^-s. False if a norm is not finite.
-template <bool CL>
-__device__ __noinline__ bool fast_transform(Team<CL> &tm, int n, Fast &f, const double *F, double *A, int &s,
-                                            float4 *sm) {
-  const int nb = f.nb;
-  const float nf = team_inf_norm(tm, n, F, sm, f.red);
-  if (!(nf < 0x1p60f)) return false;
-  const int sf = nf > 0x1p-60f ? exp_above(nf * 1.0001f) - 1 : 0;
-  planes_of<false>(tm, n, nb, F, f.Fp, [&](int) { return sf; });
-  tm.sync();
-  // H = X F: the planes of X are zero above the diagonal
-  for (int t = team_warp(tm); t < nb * nb; t += team_warps(tm)) {
-    const int ti = nb - 1 - t / nb, tj = t % nb;  // the long rows first
-    long long c[8];
-    tile_nt<kDig, kDig, kDig>(f.Xp + (size_t)ti * nb * kDig * 32, f.Fp + (size_t)tj * nb * kDig * 32, 0, ti + 1, c);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) c[e] = (c[e] + 2) >> 2;
-    uint32_t w[kDig][4];
-    cut_block<kDig>(c, w);
-    put_block<kDig>(f.Gp + ((size_t)ti * nb + tj) * kDig * 32, w);
-  }
-  tm.sync();
-  for (int t = team_warp(tm); t < nb * (nb + 1) / 2; t += team_warps(tm)) {
+// Planes in f.Fr of the symmetric matrix in f.Ft, whose value (i, j) counts
+// 2^(u(i) + u(j) + c) (ROWS: u the row exponents xe; else 0), scaled by 2^-s.
+// The part below the diagonal is taken for both.
+template <bool ROWS, bool CL>
+__device__ __noinline__ void planes_of_tiles(Team<CL> &tm, int n, const Fast &f, int c) {
+  const int nb = f.nb, nlow = nb * (nb + 1) / 2;
+  for (int t = team_warp(tm); t < nlow; t += team_warps(tm)) {
     int ti, tj;
     lower_tile(t, ti, tj);
-    long long c[8];
-    tile_nt<kDig, kDig, kDig>(f.Gp + (size_t)ti * nb * kDig * 32, f.Xp + (size_t)tj * nb * kDig * 32, 0, tj + 1, c);
+    long long v[8];
+    get_tile(f.Ft, t, v);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
-      if (i < n && j <= i) {
-        const double v = unfix(c[e], ldi<CL>(f.xe + i) + ldi<CL>(f.xe + j) + sf - 56);
-        A[(size_t)i * n + j] = v;
-        A[(size_t)j * n + i] = v;
+      int k = c + 54;
+      if constexpr (ROWS) {
+        if (i < n && j < n) k += f.xe[i] + f.xe[j];
+      }
+      v[e] = (i < n && j <= i) ? shift(v[e], k) : 0;
+    }
+    uint32_t w[kDig][4];
+    cut_block<kDig>(v, w);
+    if (ti != tj) {
+      put_right<kDig>(f.Fr + ((size_t)ti * nb + tj) * kDig * 32, w);
+      put_right_t<kDig>(f.Fr + ((size_t)tj * nb + ti) * kDig * 32, w);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (tile_row(e) == tile_col(e)) v[e] = 0;
+      uint32_t z[kDig][4];
+      cut_block<kDig>(v, z);
+#pragma unroll
+      for (int p = 0; p < kDig; ++p) {
+        const uint32_t y[4] = {transpose8(z[p][0]), transpose8(z[p][2]), transpose8(z[p][1]), transpose8(z[p][3])};
+#pragma unroll
+        for (int h = 0; h < 4; ++h) w[p][h] |= y[h];  // one of the two is zero
+      }
+      put_right<kDig>(f.Fr + ((size_t)ti * nb + ti) * kDig * 32, w);
+    }
+  }
+  tm.sync();
+}
+
+// Exponent s of a scale 2^-s that puts a matrix of Frobenius norm sqrt(sum) to
+// a norm in (1, 2].
+__device__ __forceinline__ int norm_exp(float sum) {
+  return sum > 0x1p-100f ? exp_above(sqrtf(sum) * 1.0001f) - 1 : 0;
+}
+
+// The Fock matrix F = H0 - S (v_i + v_j) / 2 - (T + T^T) / 2, T_ij = sum_c
+// M_c,ij v_c(atom of j) (conversions.py:255-297), and F' = X F X^T, whose
+// planes, scaled by 2^-s to a Frobenius norm in (1, 2], go to f.Fr. x: the
+// potential (orbitals, atomic dipoles, quadrupoles); aoat: shared, atom of
+// each orbital. All in fixed point: the float64 form (14 FMA a value) was
+// bound by the FP64 pipe. False if a potential or norm is out of range.
+template <bool CL>
+__device__ __noinline__ bool fast_fock(Team<CL> &tm, int n, Fast &f, const double *H0, const double *x,
+                                       const int *aoat, int &s, float4 *sm) {
+  const int nb = f.nb, nlow = nb * (nb + 1) / 2, nat = f.nat;
+  // exponents of the potentials, then their tables
+  {
+    float vo = 0.0f, vd = 0.0f, vq = 0.0f;
+    const int N = f.nm > 1 ? n + 9 * nat : n;
+    for (int t = threadIdx.x; t < N; t += blockDim.x) {
+      const float m = mag(ld<CL>(x + t));
+      if (t < n) vo = fmaxf(vo, m);
+      else if (t < n + 3 * nat) vd = fmaxf(vd, m);
+      else vq = fmaxf(vq, m);
+    }
+    // every CTA holds all values: the maxima need no exchange between them
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      vo = fmaxf(vo, __shfl_xor_sync(0xffffffffu, vo, o));
+      vd = fmaxf(vd, __shfl_xor_sync(0xffffffffu, vd, o));
+      vq = fmaxf(vq, __shfl_xor_sync(0xffffffffu, vq, o));
+    }
+    __syncthreads();
+    if (lane == 0) sm[wid] = make_float4(vo, vd, vq, 0.0f);
+    __syncthreads();
+    for (int w = 0; w < nw; ++w) {
+      vo = fmaxf(vo, sm[w].x);
+      vd = fmaxf(vd, sm[w].y);
+      vq = fmaxf(vq, sm[w].z);
+    }
+    if (!(fmaxf(vo, fmaxf(vd, vq)) < 0x1p60f)) return false;
+    auto ex = [](float m) { return m > 0x1p-60f ? exp_above(m) : -60; };
+    // one exponent E for all products: |M| 2^-eM and |v| 2^-(E - eM) are at most 1
+    int E = max(f.eS + ex(vo) + 1, f.eH - 3);
+    if (f.nm > 1) E = max(E, max(f.eD + ex(vd), f.eQ + ex(vq)));
+    s = E;
+    for (int t = tm.tid; t < f.nm * n; t += tm.nthr) f.pop[t] = 0;  // for this iteration's populations
+    for (int t = tm.tid; t < N; t += tm.nthr) {
+      const double v = ld<CL>(x + t);
+      if (t < n) {
+        f.vo[t] = fix(v, 53 - E + f.eS);
+      } else if (t < n + 3 * nat) {
+        const int u = t - n;
+        f.vm[(u % 3) * nat + u / 3] = halves(fix(v, 53 - E + f.eD));
+      } else {
+        const int u = t - n - 3 * nat;
+        f.vm[(3 + u % 6) * nat + u / 6] = halves(fix(v, 53 - E + f.eQ));
+      }
+    }
+    tm.sync();
+  }
+  const int E = s;
+  Four sum = {0.0f, 0.0f, 0.0f, 0.0f};
+  for (int t = team_warp(tm); t < nlow; t += team_warps(tm)) {
+    int ti, tj;
+    lower_tile(t, ti, tj);
+    long long a0[8];
+    int r[2], c[4];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) r[k] = min(16 * ti + tile_row(2 * k), n - 1);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c[k] = min(16 * tj + tile_col((k >> 1) * 4 + (k & 1)), n - 1);
+    if (f.nm > 1) {
+      int ar[2], ac[4];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) ar[k] = aoat[r[k]];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) ac[k] = aoat[c[k]];
+      // two matrices at a time: a 16-byte word of the pair (i, j) and of (j, i);
+      // the words of the next two are loaded ahead (their latency bounds this)
+      const int4 *M = f.M + (size_t)t * kPairWords + (threadIdx.x & 31);
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        long long b0[4], b1[4];
+        int4 x[4], y[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          b0[k] = b1[k] = 0;
+          x[k] = M[(4 * h + k) * 32];
+          y[k] = M[(8 + 4 * h + k) * 32];
+        }
+        const int h2 = 2 * h;
+        const int c0 = h ? c[2] : c[0], c1 = h ? c[3] : c[1], q0 = h ? ac[2] : ac[0], q1 = h ? ac[3] : ac[1];
+#pragma unroll
+        for (int m = 0; m < 5; ++m) {
+          int4 xn[4], yn[4];
+          if (m < 4) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              xn[k] = M[(m + 1) * 512 + (4 * h + k) * 32];
+              yn[k] = M[(m + 1) * 512 + (8 + 4 * h + k) * 32];
+            }
+          }
+          const int2 *v = f.vm + (2 * m - 1) * nat, *u = v + nat;  // matrix 0 is S
+          int2 vr[2], vc[2], ur[2], uc[2];
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            vr[k] = m ? v[ar[k]] : make_int2(0, 0);
+            ur[k] = u[ar[k]];
+            vc[k] = m ? v[k ? q1 : q0] : make_int2(0, 0);
+            uc[k] = u[k ? q1 : q0];
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int kr = k >> 1, kc = k & 1;
+            if (m == 0) mul_add(b0[k], b1[k], make_int2(x[k].x, x[k].y), halves(f.vo[r[kr]] + f.vo[kc ? c1 : c0]));
+            else mul_add(b0[k], b1[k], make_int2(x[k].x, x[k].y), vc[kc]);
+            if (m) mul_add(b0[k], b1[k], make_int2(y[k].x, y[k].y), vr[kr]);
+            mul_add(b0[k], b1[k], make_int2(x[k].z, x[k].w), uc[kc]);
+            mul_add(b0[k], b1[k], make_int2(y[k].z, y[k].w), ur[kr]);
+          }
+          if (m < 4) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              x[k] = xn[k];
+              y[k] = yn[k];
+            }
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          // |b0| < 20 2^50: the sum in units of 2^(E - 58) fits
+          const long long acc = b0[k] * 256 + (b1[k] >> 20);
+          if (h2) a0[4 + k] = acc; else a0[k] = acc;
+        }
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int i = r[(e >> 1) & 1], j = c[(e >> 2) * 2 + (e & 1)];
+        const int4 x = f.M[(size_t)t * kPairWords + e * 32 + (threadIdx.x & 31)];
+        long long b0 = 0, b1 = 0;
+        mul_add(b0, b1, make_int2(x.x, x.y), halves(f.vo[i] + f.vo[j]));
+        a0[e] = b0 * 256 + (b1 >> 20);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
+      long long v = 0;
+      if (i < n && j < n) v = fix(H0[(size_t)i * n + j], 58 - E) - ((a0[e] + 1) >> 1);
+      a0[e] = v;
+      const float y = fix_to_float(v);
+      sum.s0 = fmaf(ti == tj ? y : 2.0f * y, y, sum.s0);
+    }
+    put_tile(f.Ft, t, a0);
+  }
+  const Four q = team_four(tm, sum, sm, f.red);
+  const int sf = norm_exp(q.s0) + E - 2;  // fix_to_float took 2^-56 for 2^(E - 58)
+  planes_of_tiles<false>(tm, n, f, E - 58 - sf);
+  tiles<kDig>(tm, n, f, kHalf, 0, 0, nullptr);
+  sum.s0 = tiles<kDig>(tm, n, f, kFockX, 0, 0, nullptr);
+  const Four p = team_four(tm, sum, sm, f.red);
+  if (!(p.s0 < 0x1p100f)) return false;
+  const int sn = norm_exp(p.s0);
+  planes_of_tiles<true>(tm, n, f, -56 - sn);
+  s = sn + sf;
+  return true;
+}
+
+// Populations sum_k P_ki M_c,ki of every orbital i for the 10 (1) matrices,
+// from the density in f.Ft (C w C^T with |w| <= 2): f.pop[c n + i] in units of
+// 2^(xte_i + xtm + 1 + eM - 106 + 56 - sh), sh returned. A lower tile serves the
+// sums of its columns with the pairs and of its rows with their mirrors. Exact
+// sums of 53-bit factors: the order of the atomics does not matter.
+// In float64 (10 FMA a pair) this was bound by the FP64 pipe; here by the
+// loads, 80 bytes a pair, which the tile order makes contiguous.
+template <bool CL>
+__device__ __noinline__ int fast_populations(Team<CL> &tm, int n, Fast &f) {
+  const int lane = threadIdx.x & 31, nlow = f.nb * (f.nb + 1) / 2;
+  int sh = 12;  // sums over n products of at most 2^50 in units of 2^(56 - sh)
+  while (sh > 0 && ((int64_t)n << sh) > (int64_t(1) << 12)) --sh;
+  const int nw = f.nm > 1 ? 5 : 1;
+  for (int t = team_warp(tm); t < nlow; t += team_warps(tm)) {
+    int ti, tj;
+    lower_tile(t, ti, tj);
+    long long p[8];
+    get_tile(f.Ft, t, p);
+    int2 pc[8], pr[8];  // for the column sums (scaled by the row's exponent) and the row sums
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int i = min(16 * ti + tile_row(e), n - 1), j = min(16 * tj + tile_col(e), n - 1);
+      pc[e] = halves(shift(p[e], f.xte[i] - f.xtm - 3));
+      pr[e] = ti == tj ? make_int2(0, 0) : halves(shift(p[e], f.xte[j] - f.xtm - 3));
+    }
+    const int4 *M = f.M + (size_t)t * kPairWords + lane;
+    const int mirror = f.nm > 1 ? 256 : 0;
+    int4 x[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = M[e * 32];
+#pragma unroll 1
+    for (int m = 0; m < nw; ++m) {
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {  // columns, then rows
+        if (half == 1 && ti == tj) break;     // a diagonal tile holds every pair
+        int4 xn[8];  // the next half's words, loaded ahead
+        {
+          const bool turn = half == 1 || ti == tj;
+          const int4 *next = M + (turn ? (m + 1 < nw ? (m + 1) * 512 : 0) : m * 512 + mirror);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) xn[e] = next[e * 32];
+        }
+        long long s[4][2];
+        {
+          long long a0[4][2], a1[4][2];
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) a0[k][c] = a1[k][c] = 0;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            // columns: (e >> 2, e & 1); rows: (e >> 1) & 1
+            const int k = half ? (e >> 1) & 1 : (e >> 2) * 2 + (e & 1);
+            const int2 q = half ? pr[e] : pc[e];
+            mul_add(a0[k][0], a1[k][0], q, make_int2(x[e].x, x[e].y));
+            mul_add(a0[k][1], a1[k][1], q, make_int2(x[e].z, x[e].w));
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) s[k][c] = (a0[k][c] << sh) + (a1[k][c] >> (28 - sh));
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = xn[e];
+        // columns: over the 8 lanes of equal lane & 3; rows: over the 4 of equal lane >> 2
+#pragma unroll
+        for (int k = 0; k < (half ? 2 : 4); ++k)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            long long v = s[k][c];
+#pragma unroll
+            for (int o = half ? 1 : 4; o < (half ? 4 : 32); o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            s[k][c] = v;
+          }
+        // lane l keeps one sum: column (k, c) from the lane >> 2 = 2 k + c of each
+        // lane & 3; row (k, c) from the lane & 3 = 2 k + c of each lane >> 2
+        const int w = half ? lane & 3 : lane >> 2;
+        long long v = 0;
+#pragma unroll
+        for (int k = 0; k < (half ? 2 : 4); ++k)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) v = w == 2 * k + c ? s[k][c] : v;
+        const int k = w >> 1, c = 2 * m + (w & 1);
+        const int o = half ? 16 * ti + (lane >> 2) + 8 * k : 16 * tj + 8 * (k >> 1) + 2 * (lane & 3) + (k & 1);
+        if (o < n && c < f.nm)
+          atomicAdd(reinterpret_cast<unsigned long long *>(f.pop + (size_t)c * n + o), (unsigned long long)v);
       }
     }
   }
   tm.sync();
-  const float na = team_inf_norm(tm, n, A, sm, f.red);
-  if (!(na < 0x1p60f)) return false;
-  s = na > 0x1p-60f ? exp_above(na * 1.0001f) - 1 : 0;
-  planes_of<false>(tm, n, nb, A, f.Fp, [&](int) { return s; });
-  tm.sync();
-  return true;
+  return sh;
 }
 
-// Planes of C^T (rows: orbitals of the basis, columns: the mo lowest vectors)
-// in f.Gp, rows scaled by 2^-xte.
+// The density of f.Ft in float64 (both triangles).
 template <bool CL>
-__device__ __noinline__ void fast_coefficients(Team<CL> &tm, Fast &f, int mo) {
-  const int nb = f.nb, mb = (int)blocks16(mo);
-  for (int t = team_warp(tm); t < nb * mb; t += team_warps(tm)) {
-    const int ti = t / mb, tj = t % mb;
-    long long c[8];
-    tile_nt<kDig, kDig, kDig>(f.XTp + (size_t)ti * nb * kDig * 32, f.Vp + (size_t)tj * nb * kDig * 32, ti, nb, c);
+__device__ __noinline__ void fast_store_density(Team<CL> &tm, int n, const Fast &f, double *out) {
+  const int nlow = f.nb * (f.nb + 1) / 2;
+  for (int t = team_warp(tm); t < nlow; t += team_warps(tm)) {
+    int ti, tj;
+    lower_tile(t, ti, tj);
+    long long p[8];
+    get_tile(f.Ft, t, p);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) c[e] = (c[e] + 2) >> 2;
-    uint32_t w[kDig][4];
-    cut_block<kDig>(c, w);
-    put_block<kDig>(f.Gp + ((size_t)ti * nb + tj) * kDig * 32, w);
+    for (int e = 0; e < 8; ++e) {
+      const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
+      if (i < n && j <= i) {
+        const double v = unfix(p[e], f.xte[i] + f.xte[j] + 1 - 56);
+        out[(size_t)i * n + j] = v;
+        out[(size_t)j * n + i] = v;
+      }
+    }
   }
   tm.sync();
 }
@@ -785,8 +1363,9 @@ __device__ __forceinline__ void join_block(const uint4 *blk, long long (&r)[8]) 
   }
 }
 
-// out = C diag(w) C^T over the mo lowest orbitals (both triangles), from the
-// planes of C^T in f.Gp; w(j): weight of orbital j, |w| <= 2^sw.
+// C diag(w) C^T over the mo lowest orbitals from the planes of C^T in f.Gl;
+// w(j): weight of orbital j, |w| <= 2^sw. To out (both triangles), or without
+// it to f.Ft in units of 2^(xte_i + xte_j + sw - 56).
 template <bool CL, typename W>
 __device__ __noinline__ void fast_density(Team<CL> &tm, int n, Fast &f, int mo, int sw, W w, double *out) {
   const int nb = f.nb, mb = (int)blocks16(mo);
@@ -794,7 +1373,7 @@ __device__ __noinline__ void fast_density(Team<CL> &tm, int n, Fast &f, int mo, 
     const int ti = t / mb, tj = t % mb;
     const size_t o = ((size_t)ti * nb + tj) * kDig * 32;
     long long r[8];
-    join_block(f.Gp + o, r);
+    join_block(f.Gl + o, r);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int j = 16 * tj + tile_col(e);
@@ -803,25 +1382,10 @@ __device__ __noinline__ void fast_density(Team<CL> &tm, int n, Fast &f, int mo, 
     }
     uint32_t d[kDig][4];
     cut_block<kDig>(r, d);
-    put_block<kDig>(f.Fp + o, d);
+    put_right<kDig>(f.Fr + o, d);
   }
   tm.sync();
-  for (int t = team_warp(tm); t < nb * (nb + 1) / 2; t += team_warps(tm)) {
-    int ti, tj;
-    lower_tile(t, ti, tj);
-    long long c[8];
-    tile_nt<kDig, kDig, kDig>(f.Gp + (size_t)ti * nb * kDig * 32, f.Fp + (size_t)tj * nb * kDig * 32, 0, mb, c);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
-      if (i < n && j <= i) {
-        const double v = unfix(c[e], ldi<CL>(f.xte + i) + ldi<CL>(f.xte + j) + sw - 56);
-        out[(size_t)i * n + j] = v;
-        out[(size_t)j * n + i] = v;
-      }
-    }
-  }
-  tm.sync();
+  tiles<kDig>(tm, n, f, out != nullptr ? kWeighted : kDensity, mo, sw, out);
 }
 
 // The mo lowest orbitals' coefficients, row j of C (n x n, the rest zero).
@@ -831,7 +1395,7 @@ __device__ __noinline__ void fast_orbitals(Team<CL> &tm, int n, const Fast &f, i
   for (int t = team_warp(tm); t < nb * mb; t += team_warps(tm)) {
     const int ti = t / mb, tj = t % mb;
     long long r[8];
-    join_block(f.Gp + ((size_t)ti * nb + tj) * kDig * 32, r);
+    join_block(f.Gl + ((size_t)ti * nb + tj) * kDig * 32, r);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);

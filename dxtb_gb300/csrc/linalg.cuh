@@ -102,6 +102,23 @@ __device__ double team_sum(Team<CL> &tm, double v, double *red) {
   return s;
 }
 
+// Maximum of non-negative values over the team (a NaN is dropped).
+template <bool CL>
+__device__ double team_max(Team<CL> &tm, double v, double *red) {
+  double s = block_max(v, red);
+  if constexpr (CL) {
+    if (tm.size > 1) {
+      double *slot = tm.gred + 16 * (tm.phase & 1);
+      ++tm.phase;
+      if (threadIdx.x == 0) slot[tm.rank] = s;
+      tm.sync();
+      s = 0.0;
+      for (int c = 0; c < tm.size; ++c) s = fmax(s, __ldcg(slot + c));
+    }
+  }
+  return s;
+}
+
 // Shapes of the k-loop for triangular operands.
 enum KRange : int {
   kFull = 0,     // k in [0, K)

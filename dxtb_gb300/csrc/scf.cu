@@ -26,6 +26,7 @@ constexpr double kOccCut = 1e-15;    // orbitals below this occupation carry no 
 constexpr int kLuSlots = 1024;       // concurrent inverse-iteration factorisations per molecule
 // size classes (kClasses, common.cuh): 0 small, 1 one SM, 2..5 clusters of 2..16
 constexpr int kMaxCluster = 16;
+constexpr int kTinyN = 12;           // largest order of the float64 path by choice
 // dynamic shared memory: 32 n bytes, plus the rows of the Householder
 // reduction where they fit (one-SM and cluster teams), next to ~10 KB of
 // static arrays, within the 227 KB of a CTA
@@ -52,7 +53,7 @@ __host__ __device__ inline int64_t ws_size_base(int64_t n, int64_t nat) {
 }
 // with the digit planes of the tensor-core path (eigemm.cuh)
 __host__ __device__ inline int64_t ws_size_mol(int64_t n, int64_t nat) {
-  return ws_size_base(n, nat) + fast_size(n);
+  return ws_size_base(n, nat) + fast_size(n, nat);
 }
 
 struct Ws {
@@ -96,8 +97,12 @@ __device__ inline Ws ws_carve(double *base, int n, int nat) {
 // Fermi-Dirac occupations of singly occupied orbitals summing to nel
 // (filling.py:428-742 converges to the same unique root): Newton steps on
 // the electron count, safeguarded by a bisection bracket; warp 0 only.
-// eps is sorted ascending. Returns false on failure.
-__device__ bool fermi_warp(int n, const double *eps, double nel, double kt, double *f) {
+// eps is sorted ascending; eh, el: eps as float32 pairs. Orbitals beyond 45 kT
+// from mu (by float32) have f = 0 or 1 to 3e-20 and are counted in integers:
+// only the window around mu, empty for most molecules, takes float64 (a warp
+// issues one float64 instruction per ~64 cycles). Returns false on failure.
+__device__ bool fermi_warp(int n, const double *eps, const float *eh, const float *el, double nel, double kt,
+                           double *f) {
   const int lane = threadIdx.x & 31;
   if (nel <= 0.0) {
     for (int j = lane; j < n; j += 32) f[j] = 0.0;
@@ -111,10 +116,10 @@ __device__ bool fermi_warp(int n, const double *eps, double nel, double kt, doub
   const int khomo = min(max((int)ceil(nel) - 1, 0), n - 1);
   double mu = 0.5 * (eps[khomo] + eps[min(khomo + 1, n - 1)]);
   const double ikt = 1.0 / kt;
+  const float iktf = (float)ikt;
   // f(x) = 1 / (1 + e^x) from one exp(-|x|) and a reciprocal (rcp_nr: 1 + e
   // lies in [1, 2]); beyond |x| = 40 f is 0 or 1 to 4e-18, below the
-  // electron-count threshold, and the exp is skipped (the eigenvalues are
-  // sorted, so whole warp iterations far from mu skip it together)
+  // electron-count threshold
   auto occ = [](double x) {
     if (x > 40.0) return 0.0;
     if (x < -40.0) return 1.0;
@@ -122,15 +127,37 @@ __device__ bool fermi_warp(int n, const double *eps, double nel, double kt, doub
     const double r = rcp_nr(1.0 + ex);
     return x > 0.0 ? ex * r : r;
   };
-  for (int it = 0; it < 200; ++it) {
-    double s = 0.0, ds = 0.0;
+  // electrons (less nel) and their derivative at mu; with `f` the occupations
+  auto count = [&](bool write, double &ds) -> double {
+    const float mh = (float)mu, ml = (float)(mu - (double)mh);
+    int full = 0;
+    double s = 0.0;
+    ds = 0.0;
+    bool window = false;
     for (int j = lane; j < n; j += 32) {
-      const double v = occ((eps[j] - mu) * ikt);
-      s += v;
-      ds = fma(v, 1.0 - v, ds);
+      const float x = ((eh[j] - mh) + (el[j] - ml)) * iktf;
+      double v = 0.0;
+      if (x < -45.0f) {
+        ++full;
+        v = 1.0;
+      } else if (!(x > 45.0f)) {
+        window = true;
+        v = occ((eps[j] - mu) * ikt);
+        s += v;
+        ds = fma(v, 1.0 - v, ds);
+      }
+      if (write) f[j] = v;
     }
-    s = warp_sum(s) - nel;
-    ds = warp_sum(ds) * ikt;
+    full = __reduce_add_sync(0xffffffffu, full);
+    if (__any_sync(0xffffffffu, window)) {
+      s = warp_sum(s);
+      ds = warp_sum(ds) * ikt;
+    }
+    return s + ((double)full - nel);
+  };
+  double ds;
+  for (int it = 0; it < 200; ++it) {
+    const double s = count(false, ds);
     if (fabs(s) < 1e-13 * fmax(1.0, nel)) break;
     if (s > 0.0) hi = mu; else lo = mu;
     double next = ds > 0.0 ? mu - s / ds : 0.5 * (lo + hi);
@@ -138,14 +165,7 @@ __device__ bool fermi_warp(int n, const double *eps, double nel, double kt, doub
     if (hi - lo < 1e-15 * fmax(1.0, fabs(mu))) break;
     mu = next;
   }
-  double s = 0.0;
-  for (int j = lane; j < n; j += 32) {
-    const double v = occ((eps[j] - mu) * ikt);
-    f[j] = v;
-    s += v;
-  }
-  s = warp_sum(s);
-  return fabs(s - nel) < 1e-6;
+  return fabs(count(true, ds)) < 1e-6;
 }
 
 __device__ __forceinline__ double ent(double f) {
@@ -171,29 +191,109 @@ struct ScfArgs {
   int fast;           // the workspace has room for the digit planes
 };
 
-// Potential x = (vorb [n], vdp [nat][3], vqp [nat][6]) from the orbital
-// charges qo and atomic multipoles dpa/qpa (interactions/base.py:135-181).
-// One CTA (the team's lead); qo, dpa, qpa may come from the whole team.
+// Potential x = (vorb [n], vdp [nat][3], vqp [nat][6]) from the shell and atom
+// charges and the atomic multipoles (interactions/base.py:135-181). The team's
+// warps share the rows of gamma and of the atom-pair matrices; their column
+// sums are cut into `nc` chunks of rows whose partial sums go to part (9 nat
+// nc doubles). Ends with a team barrier.
 template <bool CL>
-__device__ void potential_from_charges(const ScfArgs &a, const MolView &mv, const double *qo,
-                                       const double *dpa, const double *qpa, double *qsh,
-                                       double *qat, double *vsh, double *vat, double *xout,
-                                       int multipole, int es3_shell) {
+__device__ __noinline__ void potential_from_charges(const ScfArgs &a, const MolView &mv, Team<CL> &tm,
+                                                    const double *qsh, const double *qat, const double *dpa,
+                                                    const double *qpa, double *vsh, double *vat, double *part,
+                                                    int64_t room, double *xout, int multipole, int es3_shell) {
   const dxtb_batch &b = a.b;
   const int n = mv.n, nat = mv.nat, nsh = mv.nsh;
-  for (int s = threadIdx.x; s < nsh; s += blockDim.x) {
-    const int t = b.shell_type[mv.s0 + s];
-    const int o = b.shell_ao[mv.s0 + s], no = 2 * pi_(a.pi, DXTB_I_L + t) + 1;
+  const int lane = threadIdx.x & 31, tw = team_warps(tm);
+  for (int r = team_warp(tm); r < nsh + nat; r += tw) {
     double v = 0.0;
-    for (int k = 0; k < no; ++k) v += ld<CL>(qo + o + k);
-    qsh[s] = v;
+    if (r < nsh) {
+      // shell potential: ES2 gamma q_sh (+ shell-resolved ES3)
+      const double *gr = a.gamma + mv.g0 + (size_t)r * nsh;
+      for (int t = lane; t < nsh; t += 32) v = fma(gr[t], ld<CL>(qsh + t), v);
+      v = warp_sum(v);
+      if (lane == 0) {
+        if (es3_shell) {
+          const double q = ld<CL>(qsh + r);
+          v += a.hd[mv.s0 + r] * q * q;
+        }
+        vsh[r] = v;
+      }
+    } else {
+      // atom potential: atom-resolved ES3, AES2 monopole terms, GB
+      const int i = r - nsh;
+      if (multipole || a.gb != nullptr) {
+        for (int j = lane; j < nat; j += 32) {
+          const int64_t o = mv.n2off + (int64_t)i * nat + j;
+          if (multipole) {
+            for (int c = 0; c < 3; ++c) v = fma(a.sd[c * mv.n2tot + o], ld<CL>(dpa + 3 * j + c), v);
+            for (int c = 0; c < 6; ++c) v = fma(a.sq[c * mv.n2tot + o], ld<CL>(qpa + 6 * j + c), v);
+          }
+          if (a.gb != nullptr) v = fma(a.gb[o], ld<CL>(qat + j), v);
+        }
+        v = warp_sum(v);
+      }
+      if (lane == 0) {
+        if (!es3_shell) {
+          const double q = ld<CL>(qat + i);
+          v += a.hd[mv.a0 + i] * q * q;
+        }
+        vat[i] = v;
+      }
+    }
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < nat; i += blockDim.x) qat[i] = 0.0;
-  __syncthreads();
-  if (threadIdx.x == 0)
-    for (int s = 0; s < nsh; ++s) qat[b.shell_atom[mv.s0 + s]] += qsh[s];
-  __syncthreads();
+  const int jg = (nat + 31) >> 5;
+  const int nc = multipole ? (int)max((int64_t)1, min(min((int64_t)(tw + jg - 1) / jg, (int64_t)(nat + 3) / 4),
+                                                      room / (9 * (int64_t)nat)))
+                           : 1;
+  if (multipole) {
+    for (int t = team_warp(tm); t < jg * nc; t += tw) {
+      const int j = 32 * (t % jg) + lane, ch = t / jg;
+      if (j >= nat) continue;
+      const int i0 = nat * ch / nc, i1 = nat * (ch + 1) / nc;
+      double vd[3] = {0, 0, 0}, vq[6] = {0, 0, 0, 0, 0, 0};
+      for (int i = i0; i < i1; ++i) {
+        const int64_t o = mv.n2off + (int64_t)i * nat + j;
+        const double qi = ld<CL>(qat + i);
+        for (int c = 0; c < 3; ++c) vd[c] = fma(a.sd[c * mv.n2tot + o], qi, vd[c]);
+        for (int x = 0; x < 3; ++x) {
+          const double d = ld<CL>(dpa + 3 * i + x);
+          for (int y = 0; y < 3; ++y) vd[y] = fma(a.dd[(3 * x + y) * mv.n2tot + o], d, vd[y]);
+        }
+        for (int c = 0; c < 6; ++c) vq[c] = fma(a.sq[c * mv.n2tot + o], qi, vq[c]);
+      }
+      for (int c = 0; c < 3; ++c) part[((size_t)ch * 9 + c) * nat + j] = vd[c];
+      for (int c = 0; c < 6; ++c) part[((size_t)ch * 9 + 3 + c) * nat + j] = vq[c];
+    }
+  }
+  tm.sync();
+  for (int o = tm.tid; o < n; o += tm.nthr) {
+    const int s = b.ao_shell[mv.o0 + o];
+    xout[o] = ld<CL>(vsh + s) + ld<CL>(vat + b.shell_atom[mv.s0 + s]);
+  }
+  if (multipole) {
+    for (int t = tm.tid; t < 9 * nat; t += tm.nthr) {
+      const int c = t / nat, j = t % nat;
+      const int zj = b.numbers[mv.a0 + j];
+      // qscale of the components xx, yx, yy, zx, zy, zz
+      double v = c < 3 ? 2.0 * pf(a.pf, DXTB_P_DKERNEL + zj) * ld<CL>(dpa + 3 * j + c)
+                       : 2.0 * pf(a.pf, DXTB_P_QKERNEL + zj) * ld<CL>(qpa + 6 * j + c - 3) *
+                             ((c == 4 || c == 6 || c == 7) ? 2.0 : 1.0);
+      for (int h = 0; h < nc; ++h) v += ld<CL>(part + ((size_t)h * 9 + c) * nat + j);
+      xout[c < 3 ? n + 3 * j + c : n + 3 * nat + 6 * j + c - 3] = v;
+    }
+  }
+  tm.sync();
+}
+
+// The same by one CTA, a thread per row or column in one running sum: for a
+// few atoms, where the split sums' reductions cost more than they share.
+constexpr int kFewAtoms = 8;
+__device__ __noinline__ void potential_few_atoms(const ScfArgs &a, const MolView &mv, const double *qsh,
+                                                 const double *qat, const double *dpa, const double *qpa,
+                                                 double *vsh, double *vat, double *xout, int multipole,
+                                                 int es3_shell) {
+  const dxtb_batch &b = a.b;
+  const int n = mv.n, nat = mv.nat, nsh = mv.nsh;
   // shell potential: ES2 gamma q_sh (+ shell-resolved ES3)
   for (int s = threadIdx.x; s < nsh; s += blockDim.x) {
     const double *gr = a.gamma + mv.g0 + (size_t)s * nsh;
@@ -208,8 +308,8 @@ __device__ void potential_from_charges(const ScfArgs &a, const MolView &mv, cons
     if (multipole) {
       for (int j = 0; j < nat; ++j) {
         const int64_t o = mv.n2off + (int64_t)i * nat + j;
-        for (int c = 0; c < 3; ++c) v += a.sd[c * mv.n2tot + o] * ld<CL>(dpa + 3 * j + c);
-        for (int c = 0; c < 6; ++c) v += a.sq[c * mv.n2tot + o] * ld<CL>(qpa + 6 * j + c);
+        for (int c = 0; c < 3; ++c) v += a.sd[c * mv.n2tot + o] * ld<false>(dpa + 3 * j + c);
+        for (int c = 0; c < 6; ++c) v += a.sq[c * mv.n2tot + o] * ld<false>(qpa + 6 * j + c);
       }
     }
     if (a.gb != nullptr) {
@@ -229,13 +329,13 @@ __device__ void potential_from_charges(const ScfArgs &a, const MolView &mv, cons
       const int zj = b.numbers[mv.a0 + j];
       const double dk = pf(a.pf, DXTB_P_DKERNEL + zj), qk = pf(a.pf, DXTB_P_QKERNEL + zj);
       double vd[3], vq[6];
-      for (int c = 0; c < 3; ++c) vd[c] = 2.0 * dk * ld<CL>(dpa + 3 * j + c);
-      for (int c = 0; c < 6; ++c) vq[c] = 2.0 * qk * ld<CL>(qpa + 6 * j + c) * qscale[c];
+      for (int c = 0; c < 3; ++c) vd[c] = 2.0 * dk * ld<false>(dpa + 3 * j + c);
+      for (int c = 0; c < 6; ++c) vq[c] = 2.0 * qk * ld<false>(qpa + 6 * j + c) * qscale[c];
       for (int i = 0; i < nat; ++i) {
         const int64_t o = mv.n2off + (int64_t)i * nat + j;
         for (int c = 0; c < 3; ++c) vd[c] += a.sd[c * mv.n2tot + o] * qat[i];
         for (int x = 0; x < 3; ++x)
-          for (int y = 0; y < 3; ++y) vd[y] += a.dd[(3 * x + y) * mv.n2tot + o] * ld<CL>(dpa + 3 * i + x);
+          for (int y = 0; y < 3; ++y) vd[y] += a.dd[(3 * x + y) * mv.n2tot + o] * ld<false>(dpa + 3 * i + x);
         for (int c = 0; c < 6; ++c) vq[c] += a.sq[c * mv.n2tot + o] * qat[i];
       }
       for (int c = 0; c < 3; ++c) xout[n + 3 * j + c] = vd[c];
@@ -257,24 +357,28 @@ __device__ double interaction_energy(const ScfArgs &a, const MolView &mv, const 
   for (int s = threadIdx.x; s < nsh; s += blockDim.x) {
     const double *gr = a.gamma + mv.g0 + (size_t)s * nsh;
     double v = 0.0;
-    for (int t = 0; t < nsh; ++t) v = fma(gr[t], qsh[t], v);
-    e += 0.5 * qsh[s] * v;
-    if (es3_shell) e += a.hd[mv.s0 + s] * qsh[s] * qsh[s] * qsh[s] / 3.0;
+    for (int t = 0; t < nsh; ++t) v = fma(gr[t], ld<CL>(qsh + t), v);
+    const double q = ld<CL>(qsh + s);
+    e += 0.5 * q * v;
+    if (es3_shell) e += a.hd[mv.s0 + s] * q * q * q / 3.0;
   }
   const double qscale[6] = {1.0, 2.0, 1.0, 2.0, 2.0, 1.0};
   for (int j = threadIdx.x; j < nat; j += blockDim.x) {
-    if (!es3_shell) e += a.hd[mv.a0 + j] * qat[j] * qat[j] * qat[j] / 3.0;
+    if (!es3_shell) {
+      const double q = ld<CL>(qat + j);
+      e += a.hd[mv.a0 + j] * q * q * q / 3.0;
+    }
     if (multipole) {
       const int zj = b.numbers[mv.a0 + j];
       const double dk = pf(a.pf, DXTB_P_DKERNEL + zj), qk = pf(a.pf, DXTB_P_QKERNEL + zj);
       double vd[3] = {0, 0, 0}, vq[6] = {0, 0, 0, 0, 0, 0};
       for (int i = 0; i < nat; ++i) {
         const int64_t o = mv.n2off + (int64_t)i * nat + j;
-        for (int c = 0; c < 3; ++c) vd[c] += a.sd[c * mv.n2tot + o] * qat[i];
+        for (int c = 0; c < 3; ++c) vd[c] += a.sd[c * mv.n2tot + o] * ld<CL>(qat + i);
         for (int x = 0; x < 3; ++x)
           for (int y = 0; y < 3; ++y)
             vd[y] += 0.5 * a.dd[(3 * x + y) * mv.n2tot + o] * ld<CL>(dpa + 3 * i + x);
-        for (int c = 0; c < 6; ++c) vq[c] += a.sq[c * mv.n2tot + o] * qat[i];
+        for (int c = 0; c < 6; ++c) vq[c] += a.sq[c * mv.n2tot + o] * ld<CL>(qat + i);
       }
       for (int c = 0; c < 3; ++c) {
         const double dj = ld<CL>(dpa + 3 * j + c);
@@ -288,16 +392,16 @@ __device__ double interaction_energy(const ScfArgs &a, const MolView &mv, const 
     if (a.gb != nullptr) {
       const double *gr = a.gb + mv.n2off + (size_t)j * nat;
       double v = 0.0;
-      for (int i = 0; i < nat; ++i) v += gr[i] * qat[i];
-      e += 0.5 * qat[j] * v;
+      for (int i = 0; i < nat; ++i) v += gr[i] * ld<CL>(qat + i);
+      e += 0.5 * ld<CL>(qat + j) * v;
     }
   }
   return block_sum(e, red);
 }
 
-// State of the root solver, held by the lead CTA only. final_eval: one more
-// pass evaluates the energy at the iterate left in x (hit_max: with status
-// MAXITER); base: the Anderson history ring's entry 0.
+// State of the root solver, the same on every CTA of the team. final_eval:
+// one more pass evaluates the energy at the iterate left in x (hit_max: with
+// status MAXITER); base: the Anderson history ring's entry 0.
 struct Broyden {
   int nrank = 0, final_eval = 0, hit_max = 0, base = 0;
   double resid = 0.0, best_ynorm = 1e308, dx_norm = 0.0;
@@ -310,117 +414,129 @@ enum ScfAction : int { kNext = 0, kStop = 1 };
 // damped steps x += damp * dx, dx = -Gm F (the broyden1 of exlibs/xitorch/
 // _impls/optimize/root/{rootsolver.py:42-265, _jacobian.py:51-120} with
 // alpha = -0.5, damp = 0.5, line_search = False, scf/base.py:267-292);
-// stop when |dx|_2 < x_tol and |F|_2 < f_tol. Lead CTA only.
-__device__ int broyden_step(const ScfArgs &a, Ws &w, int N, int it, Broyden &br, int &status,
-                            double *red) {
-  double *sdot = w.sdot;         // [kRank] dot products
-  double *sdot2 = sdot + kRank;  // [kRank]
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int nw = (int)(blockDim.x >> 5);
+// stop when |dx|_2 < x_tol and |F|_2 < f_tol. The whole team: an element of
+// the vectors is always the same thread's, a history vector's dot products a
+// warp's. The history is read once for the three products of each vector
+// (with dx, dy and F), once for the update and the step.
+template <bool CL>
+__device__ __noinline__ int broyden_step(const ScfArgs &a, Team<CL> &tm, Ws &w, int N, int it, Broyden &br,
+                                         int &status, double *red) {
+  double *sdot = w.sdot;          // [kRank] c_k . dx
+  double *sdot2 = sdot + kRank;   // [kRank] d_k . dy
+  double *sdot3 = sdot2 + kRank;  // [kRank] d_k . F
+  const int lane = threadIdx.x & 31;
   // |F|^2 with F = x - G(x)
   double part = 0.0;
-  for (int t = threadIdx.x; t < N; t += blockDim.x) {
-    const double y = w.x[t] - w.g[t];
+  for (int t = tm.tid; t < N; t += tm.nthr) {
+    const double y = w.x[t] - ld<CL>(w.g + t);
     part += y * y;
   }
-  const double ynorm = sqrt(block_sum(part, red));
+  const double ynorm = sqrt(team_sum(tm, part, red));
   br.resid = ynorm;
   if (it == 1) {
     if (ynorm <= a.ftol * kEps) return kStop;
     br.nrank = 0;
-  } else {
-    if (ynorm < br.best_ynorm) {
-      br.best_ynorm = ynorm;
-      for (int t = threadIdx.x; t < N; t += blockDim.x) w.xbest[t] = w.x[t];
-    }
-    // Broyden update with dx = x - x_prev, dy = F - F_prev:
-    // v = Gm^T dx, c = dx - Gm dy, d = v / (dy . v)
-    if (br.nrank >= kRank) br.nrank = 0;  // "restart" reduction of a full memory (not reached: kRank >= maxiter)
-    const int nrank = br.nrank;
-    // dx and dy once (into the x_prev / F_prev slots, rewritten below): a
-    // float64 instruction costs a warp ~64 cycles, so the dot products below
-    // read them instead of forming the differences again per history vector
-    for (int t = threadIdx.x; t < N; t += blockDim.x) {
+  } else if (ynorm < br.best_ynorm) {
+    br.best_ynorm = ynorm;
+    for (int t = tm.tid; t < N; t += tm.nthr) w.xbest[t] = w.x[t];
+  }
+  if (br.nrank >= kRank) br.nrank = 0;  // "restart" reduction of a full memory (not reached: kRank >= maxiter)
+  const int nrank = br.nrank;
+  // dx = x - x_prev and dy = F - F_prev into the x_prev / F_prev slots
+  if (it > 1) {
+    for (int t = tm.tid; t < N; t += tm.nthr) {
       const double xt = w.x[t];
-      w.rold[t] = (xt - w.g[t]) - w.rold[t];
+      w.rold[t] = (xt - ld<CL>(w.g + t)) - w.rold[t];
       w.xold[t] = xt - w.xold[t];
     }
-    __syncthreads();
-    for (int k = wid; k < 2 * nrank; k += nw) {
+    tm.sync();
+    for (int k = team_warp(tm); k < 2 * nrank; k += team_warps(tm)) {
       const int kk = k >> 1;
-      double s = 0.0;
+      double s = 0.0, r = 0.0;
       if ((k & 1) == 0) {
         const double *ck = w.hx + (size_t)kk * N;
-        for (int t = lane; t < N; t += 32) s = fma(ck[t], w.xold[t], s);
+        for (int t = lane; t < N; t += 32) s = fma(ld<CL>(ck + t), ld<CL>(w.xold + t), s);
       } else {
         const double *dk = w.hr + (size_t)kk * N;
-        for (int t = lane; t < N; t += 32) s = fma(dk[t], w.rold[t], s);
+        for (int t = lane; t < N; t += 32) {
+          const double d = ld<CL>(dk + t);
+          s = fma(d, ld<CL>(w.rold + t), s);
+          r = fma(d, ld<CL>(w.x + t) - ld<CL>(w.g + t), r);
+        }
+        r = warp_sum(r);
       }
       s = warp_sum(s);
       if (lane == 0) {
-        if ((k & 1) == 0) sdot[kk] = s; else sdot2[kk] = s;
+        if ((k & 1) == 0) {
+          sdot[kk] = s;
+        } else {
+          sdot2[kk] = s;
+          sdot3[kk] = r;
+        }
       }
     }
-    __syncthreads();
-    double *cn = w.hx + (size_t)nrank * N, *dn = w.hr + (size_t)nrank * N;
-    double pdv = 0.0;
-    for (int t = threadIdx.x; t < N; t += blockDim.x) {
-      const double dxt = w.xold[t];
-      const double dyt = w.rold[t];
+    tm.sync();
+  }
+  // Broyden update: v = Gm^T dx, c = dx - Gm dy, d = v / (dy . v); beside it
+  // g = Gm F of the old memory (in the new F_prev slot)
+  double *cn = w.hx + (size_t)nrank * N, *dn = w.hr + (size_t)nrank * N;
+  double pdv = 0.0, pfv = 0.0;
+  for (int t = tm.tid; t < N; t += tm.nthr) {
+    const double y = w.x[t] - ld<CL>(w.g + t);
+    double step = 0.5 * y;
+    if (it > 1) {
+      const double dxt = w.xold[t], dyt = w.rold[t];
       double v = 0.5 * dxt, gdy = 0.5 * dyt;
       for (int k = 0; k < nrank; ++k) {
-        v += w.hr[(size_t)k * N + t] * sdot[k];
-        gdy += w.hx[(size_t)k * N + t] * sdot2[k];
+        const double d = w.hr[(size_t)k * N + t], c = w.hx[(size_t)k * N + t];
+        v = fma(d, ld<CL>(sdot + k), v);
+        gdy = fma(c, ld<CL>(sdot2 + k), gdy);
+        step = fma(c, ld<CL>(sdot3 + k), step);
       }
       cn[t] = dxt - gdy;
       dn[t] = v;
-      pdv += dyt * v;
+      pdv = fma(dyt, v, pdv);
+      pfv = fma(y, v, pfv);
     }
-    const double dyv = block_sum(pdv, red);
+    w.rold[t] = step;
+  }
+  double fd = 0.0;  // d . F of the new vector
+  if (it > 1) {
+    const double dyv = team_sum(tm, pdv, red);
+    const double fv = team_sum(tm, pfv, red);
     if (dyv == 0.0 || !isfinite(dyv)) {
       status = DXTB_ERR_NAN;
       return kStop;
     }
     const double idyv = 1.0 / dyv;
-    for (int t = threadIdx.x; t < N; t += blockDim.x) dn[t] *= idyv;
+    fd = fv * idyv;
+    for (int t = tm.tid; t < N; t += tm.nthr) dn[t] *= idyv;
     ++br.nrank;
-    __syncthreads();
     if (br.dx_norm < a.xtol && ynorm < a.ftol) return kStop;  // converged at x
   }
   if (it >= a.maxiter) {
     // not converged: evaluate once more at the best iterate, which the root
     // solver returns with a warning (rootsolver.py:250-259)
     if (br.best_ynorm < ynorm) {
-      for (int t = threadIdx.x; t < N; t += blockDim.x) w.x[t] = w.xbest[t];
+      for (int t = tm.tid; t < N; t += tm.nthr) w.x[t] = w.xbest[t];
       br.final_eval = 1;
       br.hit_max = 1;
-      __syncthreads();
       return kNext;
     }
     br.hit_max = 1;
     return kStop;
   }
-  // F_prev = F, x_prev = x; dx = -Gm F = -(0.5 F + sum_k c_k (d_k . F))
-  const int nrank = br.nrank;
-  for (int k = wid; k < nrank; k += nw) {
-    const double *dk = w.hr + (size_t)k * N;
-    double s = 0.0;
-    for (int t = lane; t < N; t += 32) s += dk[t] * (w.x[t] - w.g[t]);
-    s = warp_sum(s);
-    if (lane == 0) sdot[k] = s;
-  }
-  __syncthreads();
+  // F_prev = F, x_prev = x; dx = -Gm F
   double pdx = 0.0;
-  for (int t = threadIdx.x; t < N; t += blockDim.x) {
-    const double y = w.x[t] - w.g[t];
-    double dx = -0.5 * y;
-    for (int k = 0; k < nrank; ++k) dx -= w.hx[(size_t)k * N + t] * sdot[k];
-    w.rold[t] = y;
-    w.xold[t] = w.x[t];
-    w.x[t] += a.damp * dx;
-    pdx += dx * dx;
+  for (int t = tm.tid; t < N; t += tm.nthr) {
+    const double xt = w.x[t];
+    const double dx = it > 1 ? -fma(cn[t], fd, w.rold[t]) : -w.rold[t];
+    w.rold[t] = xt - ld<CL>(w.g + t);
+    w.xold[t] = xt;
+    w.x[t] = fma(a.damp, dx, xt);
+    pdx = fma(dx, dx, pdx);
   }
-  br.dx_norm = sqrt(block_sum(pdx, red));
+  br.dx_norm = sqrt(team_sum(tm, pdx, red));
   if (br.dx_norm == 0.0) {
     status = DXTB_ERR_NAN;
     return kStop;
@@ -472,25 +588,25 @@ __device__ bool small_solve(int n, double *A, double *r) {
 // start) or the first call, else x_bar + damp F_bar with the coefficients th
 // of (dF_i . dF_j)(1 + offset^2 on the diagonal) th = dF_i . F, dF_i = F -
 // F_i over the last min(call - 1, generations) entries. The histories X (in
-// hx) and F (in hr) are rings of generations + 1 vectors. Lead CTA only.
-__device__ int anderson_step(const ScfArgs &a, Ws &w, int N, int it, Broyden &br, int &status,
-                             double *red) {
+// hx) and F (in hr) are rings of generations + 1 vectors. The whole team.
+template <bool CL>
+__device__ __noinline__ int anderson_step(const ScfArgs &a, Team<CL> &tm, Ws &w, int N, int it, Broyden &br,
+                                          int &status, double *red) {
   const int G = a.generations, H = G + 1;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int nw = (int)(blockDim.x >> 5);
+  const int lane = threadIdx.x & 31;
   auto X = [&](int h) { return w.hx + (size_t)((br.base + h) % H) * N; };
   auto F = [&](int h) { return w.hr + (size_t)((br.base + h) % H) * N; };
   double *x0 = X(0), *f0 = F(0);
   double p2 = 0.0, pm = 0.0;
-  for (int t = threadIdx.x; t < N; t += blockDim.x) {
-    const double xt = w.x[t], ft = w.g[t] - xt;
+  for (int t = tm.tid; t < N; t += tm.nthr) {
+    const double xt = w.x[t], ft = ld<CL>(w.g + t) - xt;
     x0[t] = xt;
     f0[t] = ft;
     p2 = fma(ft, ft, p2);
     pm = fmax(pm, fabs(ft));
   }
-  const double l2 = sqrt(block_sum(p2, red));
-  const double mx = block_max(pm, red);
+  const double l2 = sqrt(team_sum(tm, p2, red));
+  const double mx = team_max(tm, pm, red);
   br.resid = l2;
   if (!isfinite(l2)) {
     status = DXTB_ERR_NAN;
@@ -499,10 +615,9 @@ __device__ int anderson_step(const ScfArgs &a, Ws &w, int N, int it, Broyden &br
   // the loop ends after maxiter calls beyond the guess-mixing one
   const bool conv = it >= 2 && l2 < a.xtol && mx < a.xtol_max;
   if (conv || it >= a.maxiter + 1) {
-    for (int t = threadIdx.x; t < N; t += blockDim.x) w.x[t] = w.g[t];
+    for (int t = tm.tid; t < N; t += tm.nthr) w.x[t] = ld<CL>(w.g + t);
     br.final_eval = 1;
     br.hit_max = conv ? 0 : 1;
-    __syncthreads();
     return kNext;
   }
   double *sdot = w.sdot;  // [0, n(n+1)/2 + n): the system; then th
@@ -510,7 +625,8 @@ __device__ int anderson_step(const ScfArgs &a, Ws &w, int N, int it, Broyden &br
     const int n = min(it - 1, G);
     const int npair = n * (n + 1) / 2;
     // task k < npair: (dF_i . dF_j), i <= j; then dF_i . F
-    for (int k = wid; k < npair + n; k += nw) {
+    tm.sync();
+    for (int k = team_warp(tm); k < npair + n; k += team_warps(tm)) {
       int i, j;
       if (k < npair) {
         i = 0;
@@ -523,40 +639,40 @@ __device__ int anderson_step(const ScfArgs &a, Ws &w, int N, int it, Broyden &br
       const double *fi = F(i + 1), *fj = j >= 0 ? F(j + 1) : nullptr;
       double s = 0.0;
       for (int t = lane; t < N; t += 32) {
-        const double di = f0[t] - fi[t];
-        s = fma(di, j >= 0 ? f0[t] - fj[t] : f0[t], s);
+        const double f = ld<CL>(f0 + t), di = f - ld<CL>(fi + t);
+        s = fma(di, j >= 0 ? f - ld<CL>(fj + t) : f, s);
       }
       s = warp_sum(s);
       if (lane == 0) sdot[k] = s;
     }
-    __syncthreads();
+    tm.sync();
     double *A = sdot + npair + n, *th = A + n * n;
-    if (threadIdx.x == 0) {
+    if (tm.lead() && threadIdx.x == 0) {
       for (int i = 0; i < n; ++i) {
         for (int j = 0; j <= i; ++j) {
-          const double v = sdot[i * (i + 1) / 2 + j];
+          const double v = ld<CL>(sdot + i * (i + 1) / 2 + j);
           A[i * n + j] = v;
           A[j * n + i] = v;
         }
         A[i * n + i] *= 1.0 + a.offset * a.offset;
-        th[i] = sdot[npair + i];
+        th[i] = ld<CL>(sdot + npair + i);
       }
       w.team[48] = small_solve(n, A, th) ? 1.0 : 0.0;
     }
-    __syncthreads();
-    if (w.team[48] == 0.0) {
+    tm.sync();
+    if (ld<CL>(w.team + 48) == 0.0) {
       status = DXTB_ERR_NAN;
       return kStop;
     }
     // x_mix = X0 + damp F0 + sum_i th_i ((X_i - X0) + damp (F_i - F0))
-    for (int t = threadIdx.x; t < N; t += blockDim.x) {
+    for (int t = tm.tid; t < N; t += tm.nthr) {
       const double xt = x0[t], ft = f0[t];
       double v = fma(a.damp, ft, xt);
-      for (int i = 0; i < n; ++i) v = fma(th[i], (X(i + 1)[t] - xt) + a.damp * (F(i + 1)[t] - ft), v);
+      for (int i = 0; i < n; ++i) v = fma(ld<CL>(th + i), (X(i + 1)[t] - xt) + a.damp * (F(i + 1)[t] - ft), v);
       w.x[t] = v;
     }
   } else {
-    for (int t = threadIdx.x; t < N; t += blockDim.x) w.x[t] = fma(a.damp_init, f0[t], x0[t]);
+    for (int t = tm.tid; t < N; t += tm.nthr) w.x[t] = fma(a.damp_init, f0[t], x0[t]);
   }
   br.base = (br.base + H - 1) % H;  // entry 0 of this call becomes entry 1
   __syncthreads();
@@ -572,27 +688,34 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
   __shared__ double red[32];
   __shared__ double spart[kPart];
   __shared__ float4 sfour[32];
+  // what every thread reads and none changes: one copy per CTA (per-thread
+  // copies handed to functions live in local memory and fill the L1)
+  __shared__ MolView mv;
+  __shared__ Ws w;
+  __shared__ Fast f;
   const dxtb_batch &b = a.b;
-  MolView mv;
-  mv.m = m_;
-  const int m = mv.m;
-  mv.a0 = b.atom_off[m];
-  mv.s0 = b.shell_off[m];
-  mv.o0 = b.ao_off[m];
-  mv.moff = b.mat_off[m];
-  mv.mtot = b.mat_off[b.nmol];
-  mv.n2off = b.nat2_off[m];
-  mv.n2tot = b.nat2_off[b.nmol];
-  mv.g0 = b.nsh2_off[m];
-  mv.n = (int)(b.ao_off[m + 1] - mv.o0);
-  mv.nat = (int)(b.atom_off[m + 1] - mv.a0);
-  mv.nsh = (int)(b.shell_off[m + 1] - mv.s0);
-  const int n = mv.n, nat = mv.nat;
+  const int m = m_;
   const int multipole = pi_(a.pi, DXTB_I_SCAL + DXTB_IS_MULTIPOLE);
   const int es3_shell = pi_(a.pi, DXTB_I_SCAL + DXTB_IS_ES3_SHELL);
-  const int N = n + (multipole ? 9 * nat : 0);
-  mv.N = N;
-  Ws w = ws_carve(a.ws + a.ws_off[m], n, nat);
+  if (threadIdx.x == 0) {
+    mv.m = m;
+    mv.a0 = b.atom_off[m];
+    mv.s0 = b.shell_off[m];
+    mv.o0 = b.ao_off[m];
+    mv.moff = b.mat_off[m];
+    mv.mtot = b.mat_off[b.nmol];
+    mv.n2off = b.nat2_off[m];
+    mv.n2tot = b.nat2_off[b.nmol];
+    mv.g0 = b.nsh2_off[m];
+    mv.n = (int)(b.ao_off[m + 1] - mv.o0);
+    mv.nat = (int)(b.atom_off[m + 1] - mv.a0);
+    mv.nsh = (int)(b.shell_off[m + 1] - mv.s0);
+    mv.N = mv.n + (multipole ? 9 * mv.nat : 0);
+    w = ws_carve(a.ws + a.ws_off[m], mv.n, mv.nat);
+    if (a.fast) f = fast_carve(a.ws + a.ws_off[m] + ws_size_base(mv.n, mv.nat), mv.n, mv.nat, multipole);
+  }
+  __syncthreads();
+  const int n = mv.n, nat = mv.nat, N = mv.N;
   tm.gred = w.team;
   tm.gctl = reinterpret_cast<int *>(w.team + 32);
   tm.phase = 0;
@@ -617,65 +740,139 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
   for (int t = tm.tid; t < N; t += tm.nthr) w.x[t] = 0.0;
   tm.sync();
   // The products and the eigenproblem run on digit planes; where a norm is not
-  // finite or the vectors do not settle, or without the workspace for the
-  // planes, the float64 path takes over for the rest of this SCF.
-  Fast f = {};
-  bool fast = a.fast != 0 && status == DXTB_OK;
+  // finite or the vectors do not settle the float64 path takes an iteration,
+  // after three such iterations, or without the workspace for the planes, all.
+  // Up to kTinyN orbitals (less than a block) float64 stays: as quick at 6
+  // (1.87 ms against 1.92 for water), 5.9 ms against ~3.9 at 12, but SCFs of so
+  // few degrees of freedom on the default 1e-4 end where the rounding takes
+  // them (a 3-atom molecule's Anderson system is singular to working
+  // precision: 1e-16 in its charges moves its forces by 1e-6).
+  bool fast = a.fast != 0 && status == DXTB_OK && n > kTinyN;
   if (fast) {
-    f = fast_carve(a.ws + a.ws_off[m] + ws_size_base(n, nat), n);
-    fast = fast_setup(tm, n, w.Linv, f, sfour);
+    fast = fast_setup(tm, n, w.Linv, f, sfour) &&
+           fast_integrals(tm, n, f, S, H0, multipole ? a.D + mv.moff : nullptr,
+                          multipole ? a.Q + mv.moff : nullptr, mv.mtot, sfour);
   }
 
-  int it = 0, mo = 1;
+  int it = 0, mo = 1, misses = fast ? 0 : 3;
   Broyden br;
   while (status == DXTB_OK) {
     ++it;
-    // ---- Fock matrix F(x) into Zt (conversions.py:255-297) ----
-    // The multipole part -1/2 (T + T^T) with T_ij = sum_c M_c,ij v_c(atom of j)
-    // is formed in two coalesced passes (T into A, then the transposed read),
-    // the orbital -> atom map and the orbital potential staged in shared
-    // memory (free here: df and sd are used later in the iteration).
-    {
+    fast = misses < 3;
+    // ---- F' = X F X^T and its eigenvalues (ascending, sw) and vectors ----
+    double tnorm = 0.0;
+    double *fa = w.fa, *fb = w.fb;  // occupations: per CTA in shared memory on the fast path
+    if (fast) {
       int *aoat = reinterpret_cast<int *>(df);
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        aoat[i] = b.shell_atom[mv.s0 + b.ao_shell[mv.o0 + i]];
-        sd[i] = ld<CL>(w.x + i);
+      for (int i = threadIdx.x; i < n; i += blockDim.x) aoat[i] = b.shell_atom[mv.s0 + b.ao_shell[mv.o0 + i]];
+      __syncthreads();
+      int s2;
+      fast = fast_fock(tm, n, f, H0, w.x, aoat, s2, sfour) && fast_eigen(tm, n, f, sd, se, df, e2f, sfour);
+      if (fast) {
+        const double scale = ldexp(1.0, s2);
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+          const double v = sd[i] * scale;
+          sw[i] = v;
+          df[i] = (float)v;
+          e2f[i] = (float)(v - (double)(float)v);
+        }
+      } else {
+        ++misses;
       }
       __syncthreads();
-      if (multipole) {
-        const double *xd = w.x + n, *xq = w.x + n + 3 * nat;
-        const double *Dm = a.D + mv.moff, *Qm = a.Q + mv.moff;
-        for (int64_t t = tm.tid; t < (int64_t)n * n; t += tm.nthr) {
-          const int aj = aoat[(int)(t % n)];
-          double acc = 0.0;
-#pragma unroll
-          for (int c = 0; c < 3; ++c) acc = fma(Dm[c * mv.mtot + t], ld<CL>(xd + 3 * aj + c), acc);
-#pragma unroll
-          for (int c = 0; c < 6; ++c) acc = fma(Qm[c * mv.mtot + t], ld<CL>(xq + 6 * aj + c), acc);
-          w.A[t] = acc;
+    }
+    if (fast) {
+      // ---- Fermi occupations (filling.py:428-742), both spin channels: every
+      // CTA for itself ----
+      fa = sd;
+      fb = se;
+      __shared__ int s_ok, s_mo;
+      if (threadIdx.x < 32) {
+        bool ok = fermi_warp(n, sw, df, e2f, nel_a, a.kt, fa);
+        if (nel_b != nel_a) ok = ok && fermi_warp(n, sw, df, e2f, nel_b, a.kt, fb);
+        int first = n;  // orbitals with non-vanishing occupation (decreasing with j)
+        for (int j = threadIdx.x; j < n; j += 32) {
+          if (nel_b == nel_a) fb[j] = fa[j];
+          if (first == n && !(fa[j] + fb[j] > kOccCut)) first = j;
         }
-        tm.sync();
+        first = __reduce_min_sync(0xffffffffu, first);
+        if (threadIdx.x == 0) {
+          s_ok = ok ? 1 : 0;
+          s_mo = first > 0 ? first : 1;
+        }
       }
-      for (int64_t t = tm.tid; t < (int64_t)n * n; t += tm.nthr) {
-        const int i = (int)(t / n), j = (int)(t % n);
-        double f = H0[t] - 0.5 * S[t] * (sd[i] + sd[j]);
-        if (multipole) f -= 0.5 * (ld<CL>(w.A + t) + ld<CL>(w.A + (size_t)j * n + i));
-        w.Zt[t] = f;
+      __syncthreads();
+      if (!s_ok) {
+        status = DXTB_ERR_FERMI;
+        break;
+      }
+      mo = s_mo;
+      // ---- C^T, then P = C diag(occ) C^T (scf/utils.py:29-52) ----
+      tiles<kDig>(tm, n, f, kCoeff, mo, 0, nullptr);
+      fast_density(tm, n, f, mo, 1, [&](int j) { return fa[j] + fb[j]; }, (double *)nullptr);
+      // ---- Mulliken charges and atomic multipoles (conversions.py:203-251) ----
+      const int u = f.xtm + 1 - 50 - fast_populations(tm, n, f);
+      // orbital o's sum with matrix c counts 2^(u + xte[o] + exponent of the matrix)
+      auto pop = [&](int c, int o) {
+        return unfix(__ldcg(f.pop + (size_t)c * n + o), u + f.xte[o] + (c == 0 ? f.eS : c < 4 ? f.eD : f.eQ));
+      };
+      for (int i = tm.tid; i < n; i += tm.nthr) qo[i] = n0[i] - pop(0, i);
+      for (int t = tm.tid; t < f.nm * mv.nsh; t += tm.nthr) {
+        const int c = t / mv.nsh, sh0 = t % mv.nsh;
+        auto orbitals = [&](int s) { return 2 * pi_(a.pi, DXTB_I_L + b.shell_type[mv.s0 + s]) + 1; };
+        if (c == 0) {
+          const int o = b.shell_ao[mv.s0 + sh0], no = orbitals(sh0);
+          double v = 0.0;
+          for (int k = 0; k < no; ++k) v += n0[o + k] - pop(0, o + k);
+          qsh[sh0] = v;
+        }
+        // the first shell of an atom sums the atom (its shells are consecutive)
+        const int at = b.shell_atom[mv.s0 + sh0];
+        if (sh0 > 0 && b.shell_atom[mv.s0 + sh0 - 1] == at) continue;
+        double v = 0.0;
+        for (int s = sh0; s < mv.nsh && b.shell_atom[mv.s0 + s] == at; ++s) {
+          const int o = b.shell_ao[mv.s0 + s], no = orbitals(s);
+          for (int k = 0; k < no; ++k) v += c == 0 ? n0[o + k] - pop(0, o + k) : -pop(c, o + k);
+        }
+        (c == 0 ? qat + at : c < 4 ? dpa + 3 * at + c - 1 : qpa + 6 * at + c - 4)[0] = v;
       }
       tm.sync();
     }
-    // ---- F' = X F X^T and its eigenvalues (ascending, sw) and vectors ----
-    double tnorm = 0.0;
-    if (fast) {
-      int s2;
-      fast = fast_transform(tm, n, f, w.Zt, w.A, s2, sfour) && fast_eigen(tm, n, f, sd, se, df, e2f, sfour);
-      if (fast) {
-        const double scale = ldexp(1.0, s2);
-        for (int i = threadIdx.x; i < n; i += blockDim.x) sw[i] = sd[i] * scale;
-      }
-      __syncthreads();
-    }
     if (!fast) {
+      // ---- Fock matrix F(x) into Zt (conversions.py:255-297) ----
+      // The multipole part -1/2 (T + T^T) with T_ij = sum_c M_c,ij v_c(atom of j)
+      // is formed in two coalesced passes (T into A, then the transposed read),
+      // the orbital -> atom map and the orbital potential staged in shared
+      // memory (free here: df and sd are used later in the iteration).
+      {
+        int *aoat = reinterpret_cast<int *>(df);
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+          aoat[i] = b.shell_atom[mv.s0 + b.ao_shell[mv.o0 + i]];
+          sd[i] = ld<CL>(w.x + i);
+        }
+        __syncthreads();
+        if (multipole) {
+          const double *xd = w.x + n, *xq = w.x + n + 3 * nat;
+          const double *Dm = a.D + mv.moff, *Qm = a.Q + mv.moff;
+          for (int64_t t = tm.tid; t < (int64_t)n * n; t += tm.nthr) {
+            const int aj = aoat[(int)(t % n)];
+            double acc = 0.0;
+  #pragma unroll
+            for (int c = 0; c < 3; ++c) acc = fma(Dm[c * mv.mtot + t], ld<CL>(xd + 3 * aj + c), acc);
+  #pragma unroll
+            for (int c = 0; c < 6; ++c) acc = fma(Qm[c * mv.mtot + t], ld<CL>(xq + 6 * aj + c), acc);
+            w.A[t] = acc;
+          }
+          tm.sync();
+        }
+        for (int64_t t = tm.tid; t < (int64_t)n * n; t += tm.nthr) {
+          const int i = (int)(t / n), j = (int)(t % n);
+          double f = H0[t] - 0.5 * S[t] * (sd[i] + sd[j]);
+          if (multipole) f -= 0.5 * (ld<CL>(w.A + t) + ld<CL>(w.A + (size_t)j * n + i));
+          w.Zt[t] = f;
+        }
+        tm.sync();
+      }
       // ---- F' = X F X^T (exlibs/xitorch/_impls/linalg/symeig.py:57-61) ----
       // X = L^-1 is lower triangular: A = X F needs k <= i; only the lower
       // triangle of (X F) X^T is formed (k <= j), then mirrored.
@@ -705,39 +902,39 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
       tnorm = 0.0;
       for (int j = threadIdx.x; j < n; j += blockDim.x) tnorm = fmax(tnorm, fabs(sd[j]) + 2.0 * fabs(se[j]));
       tnorm = block_max(tnorm, red);  // also orders the sw writes
-    }
-    // ---- Fermi occupations (filling.py:428-742), both spin channels ----
-    if (tm.lead() && threadIdx.x < 32) {
-      bool ok = fermi_warp(n, sw, nel_a, a.kt, w.fa);
-      if (nel_b == nel_a) {
-        for (int j = threadIdx.x; j < n; j += 32) w.fb[j] = w.fa[j];
-      } else {
-        ok = ok && fermi_warp(n, sw, nel_b, a.kt, w.fb);
+      // float32 pairs of the eigenvalues for the Fermi search
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        df[i] = (float)sw[i];
+        e2f[i] = (float)(sw[i] - (double)df[i]);
       }
-      __syncwarp();
-      if (threadIdx.x == 0) {
-        // orbitals with non-vanishing occupation (occupations decrease with
-        // j), extended to the end of their eigenvalue cluster
-        int mm = 0;
-        while (mm < n && w.fa[mm] + w.fb[mm] > kOccCut) ++mm;
-        mm = mm > 0 ? mm : 1;
-        const double ctol = 1e-6 * fmax(tnorm, 1.0);
-        while (!fast && mm < n && sw[mm] - sw[mm - 1] <= ctol) ++mm;
-        tm.gctl[0] = ok ? 1 : 0;
-        tm.gctl[1] = mm;
+      __syncthreads();
+      // ---- Fermi occupations (filling.py:428-742), both spin channels ----
+      if (tm.lead() && threadIdx.x < 32) {
+        bool ok = fermi_warp(n, sw, df, e2f, nel_a, a.kt, w.fa);
+        if (nel_b == nel_a) {
+          for (int j = threadIdx.x; j < n; j += 32) w.fb[j] = w.fa[j];
+        } else {
+          ok = ok && fermi_warp(n, sw, df, e2f, nel_b, a.kt, w.fb);
+        }
+        __syncwarp();
+        if (threadIdx.x == 0) {
+          // orbitals with non-vanishing occupation (occupations decrease with
+          // j), extended to the end of their eigenvalue cluster
+          int mm = 0;
+          while (mm < n && w.fa[mm] + w.fb[mm] > kOccCut) ++mm;
+          mm = mm > 0 ? mm : 1;
+          const double ctol = 1e-6 * fmax(tnorm, 1.0);
+          while (mm < n && sw[mm] - sw[mm - 1] <= ctol) ++mm;
+          tm.gctl[0] = ok ? 1 : 0;
+          tm.gctl[1] = mm;
+        }
       }
-    }
-    tm.sync();
-    if (!ldi<CL>(tm.gctl + 0)) {
-      status = DXTB_ERR_FERMI;
-      break;
-    }
-    mo = ldi<CL>(tm.gctl + 1);
-    if (fast) {
-      // ---- C^T, then P = C diag(occ) C^T (scf/utils.py:29-52) ----
-      fast_coefficients(tm, f, mo);
-      fast_density(tm, n, f, mo, 1, [&](int j) { return ld<CL>(w.fa + j) + ld<CL>(w.fb + j); }, P);
-    } else {
+      tm.sync();
+      if (!ldi<CL>(tm.gctl + 0)) {
+        status = DXTB_ERR_FERMI;
+        break;
+      }
+      mo = ldi<CL>(tm.gctl + 1);
       // ---- eigenvectors of the mo lowest orbitals only ----
       team_tri_vectors(tm, n, sd, se, sw, mo, tnorm, w.Zt, w.lu, (int)min((int64_t)tm.nthr, lu_slots(n)), w.cl,
                        reinterpret_cast<double *>(df));
@@ -752,56 +949,71 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
       tm.sync();
       team_gemm<true, false>(tm, n, n, mo, 1.0, C, n, w.A, n, 0.0, P, n, kFull, true);
       team_mirror_lower(tm, n, P);
-    }
-    // ---- Mulliken charges and atomic multipoles (conversions.py:203-251) ----
-    for (int i = tm.tid; i < n; i += tm.nthr) {
-      double pop = 0.0;
-      for (int k = 0; k < n; ++k) pop = fma(ld<CL>(P + (size_t)k * n + i), S[(size_t)k * n + i], pop);
-      qo[i] = n0[i] - pop;
-    }
-    if (multipole) {
-      for (int t = tm.tid; t < 3 * nat; t += tm.nthr) dpa[t] = 0.0;
-      for (int t = tm.tid; t < 6 * nat; t += tm.nthr) qpa[t] = 0.0;
-      tm.sync();
-      // -sum_k P_ik M[c][k][i] per orbital i, reduced onto the atom of i
+      // ---- Mulliken charges and atomic multipoles (conversions.py:203-251) ----
       for (int i = tm.tid; i < n; i += tm.nthr) {
-        double acc[9];
-        for (int c = 0; c < 9; ++c) acc[c] = 0.0;
-        for (int k = 0; k < n; ++k) {
-          const double pk = ld<CL>(P + (size_t)k * n + i);
-          const int64_t e = mv.moff + (int64_t)k * n + i;
-          for (int c = 0; c < 3; ++c) acc[c] -= pk * a.D[c * mv.mtot + e];
-          for (int c = 0; c < 6; ++c) acc[3 + c] -= pk * a.Q[c * mv.mtot + e];
+        double pop = 0.0;
+        for (int k = 0; k < n; ++k) pop = fma(ld<CL>(P + (size_t)k * n + i), S[(size_t)k * n + i], pop);
+        qo[i] = n0[i] - pop;
+      }
+      if (multipole) {
+        for (int t = tm.tid; t < 3 * nat; t += tm.nthr) dpa[t] = 0.0;
+        for (int t = tm.tid; t < 6 * nat; t += tm.nthr) qpa[t] = 0.0;
+        tm.sync();
+        // -sum_k P_ik M[c][k][i] per orbital i, reduced onto the atom of i
+        for (int i = tm.tid; i < n; i += tm.nthr) {
+          double acc[9];
+          for (int c = 0; c < 9; ++c) acc[c] = 0.0;
+          for (int k = 0; k < n; ++k) {
+            const double pk = ld<CL>(P + (size_t)k * n + i);
+            const int64_t e = mv.moff + (int64_t)k * n + i;
+            for (int c = 0; c < 3; ++c) acc[c] -= pk * a.D[c * mv.mtot + e];
+            for (int c = 0; c < 6; ++c) acc[3 + c] -= pk * a.Q[c * mv.mtot + e];
+          }
+          const int ai = b.shell_atom[mv.s0 + b.ao_shell[mv.o0 + i]];
+          for (int c = 0; c < 3; ++c) atomicAdd(&dpa[3 * ai + c], acc[c]);
+          for (int c = 0; c < 6; ++c) atomicAdd(&qpa[6 * ai + c], acc[3 + c]);
         }
-        const int ai = b.shell_atom[mv.s0 + b.ao_shell[mv.o0 + i]];
-        for (int c = 0; c < 3; ++c) atomicAdd(&dpa[3 * ai + c], acc[c]);
-        for (int c = 0; c < 6; ++c) atomicAdd(&qpa[6 * ai + c], acc[3 + c]);
       }
+      tm.sync();
+      for (int s = tm.tid; s < mv.nsh; s += tm.nthr) {
+        const int o = b.shell_ao[mv.s0 + s], no = 2 * pi_(a.pi, DXTB_I_L + b.shell_type[mv.s0 + s]) + 1;
+        double v = 0.0;
+        for (int k = 0; k < no; ++k) v += ld<CL>(qo + o + k);
+        qsh[s] = v;
+      }
+      tm.sync();
+      for (int s = tm.tid; s < mv.nsh; s += tm.nthr) {
+        const int at = b.shell_atom[mv.s0 + s];
+        if (s > 0 && b.shell_atom[mv.s0 + s - 1] == at) continue;
+        double v = 0.0;
+        for (int k = s; k < mv.nsh && b.shell_atom[mv.s0 + k] == at; ++k) v += ld<CL>(qsh + k);
+        qat[at] = v;
+      }
+      tm.sync();
+    }
+    // ---- new potential G(x) and the root-solver step ----
+    if (!CL && nat <= kFewAtoms)
+      potential_few_atoms(a, mv, qsh, qat, dpa, qpa, vsh, vat, w.g, multipole, es3_shell);
+    else
+      potential_from_charges(a, mv, tm, qsh, qat, dpa, qpa, vsh, vat, w.lu, lu_size(n), w.g, multipole, es3_shell);
+    int act;
+    if (br.final_eval) {
+      act = kStop;  // hit_max as set when the final evaluation was scheduled
+    } else if (a.mixer == DXTB_MIXER_ANDERSON) {
+      act = anderson_step(a, tm, w, N, it, br, status, red);
+    } else {
+      act = broyden_step(a, tm, w, N, it, br, status, red);
     }
     tm.sync();
-    // ---- new potential G(x) and the root-solver step (lead CTA) ----
-    if (tm.lead()) {
-      potential_from_charges<CL>(a, mv, qo, dpa, qpa, qsh, qat, vsh, vat, w.g, multipole, es3_shell);
-      int act;
-      if (br.final_eval) {
-        act = kStop;  // hit_max as set when the final evaluation was scheduled
-      } else if (a.mixer == DXTB_MIXER_ANDERSON) {
-        act = anderson_step(a, w, N, it, br, status, red);
-      } else {
-        act = broyden_step(a, w, N, it, br, status, red);
-      }
-      if (threadIdx.x == 0) {
-        tm.gctl[3] = act;
-        tm.gctl[4] = (act == kStop && br.hit_max && status == DXTB_OK) ? DXTB_ERR_MAXITER : status;
-      }
+    if (act == kStop) {
+      if (br.hit_max && status == DXTB_OK) status = DXTB_ERR_MAXITER;
+      break;
     }
-    tm.sync();
-    status = ldi<CL>(tm.gctl + 4);
-    if (ldi<CL>(tm.gctl + 3) == kStop) break;
   }
 
   // ---- outputs ----
   if (status == DXTB_OK || status == DXTB_ERR_MAXITER) {
+    if (fast) fast_store_density(tm, n, f, P);
     // energies (scf/base.py:510-619): E_h0 + E_int and -TS
     double part = 0.0;
     for (int64_t t = tm.tid; t < (int64_t)n * n; t += tm.nthr) part += ld<CL>(P + t) * H0[t];
@@ -809,7 +1021,8 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
     if (tm.lead()) {
       const double eint = interaction_energy<CL>(a, mv, qsh, qat, dpa, qpa, multipole, es3_shell, red);
       double ts = 0.0;
-      for (int j = threadIdx.x; j < n; j += blockDim.x) ts += ent(w.fa[j]) + ent(w.fb[j]);
+      const double *fa = fast ? sd : w.fa, *fb = fast ? se : w.fb;
+      for (int j = threadIdx.x; j < n; j += blockDim.x) ts += ent(fa[j]) + ent(fb[j]);
       ts = a.kt * block_sum(ts, red);
       if (threadIdx.x == 0) {
         a.energies[4 * m + 0] = eh0 + eint;
@@ -820,18 +1033,18 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
       }
       for (int j = threadIdx.x; j < n; j += blockDim.x) {
         a.evals[mv.o0 + j] = sw[j];
-        a.occ[mv.o0 + j] = w.fa[j] + w.fb[j];
+        a.occ[mv.o0 + j] = fa[j] + fb[j];
         a.q[mv.o0 + j] = ld<CL>(qo + j);
       }
       // potentials of the final charges (for the gradient)
-      for (int t = threadIdx.x; t < n; t += blockDim.x) a.vorb[mv.o0 + t] = w.g[t];
+      for (int t = threadIdx.x; t < n; t += blockDim.x) a.vorb[mv.o0 + t] = ld<CL>(w.g + t);
       if (multipole) {
         for (int t = threadIdx.x; t < 3 * nat; t += blockDim.x) {
-          a.vdp[3 * mv.a0 + t] = w.g[n + t];
+          a.vdp[3 * mv.a0 + t] = ld<CL>(w.g + n + t);
           a.dp[3 * mv.a0 + t] = ld<CL>(dpa + t);
         }
         for (int t = threadIdx.x; t < 6 * nat; t += blockDim.x) {
-          a.vqp[6 * mv.a0 + t] = w.g[n + 3 * nat + t];
+          a.vqp[6 * mv.a0 + t] = ld<CL>(w.g + n + 3 * nat + t);
           a.qp[6 * mv.a0 + t] = ld<CL>(qpa + t);
         }
       }
@@ -840,7 +1053,7 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
     if (a.W != nullptr && fast) {
       const double top = fmax(fabs(sw[0]), fabs(sw[n - 1]));
       const int e2 = top > 1e-30 ? exp_above((float)top) + 1 : 0;
-      fast_density(tm, n, f, mo, e2, [&](int j) { return (ld<CL>(w.fa + j) + ld<CL>(w.fb + j)) * sw[j]; },
+      fast_density(tm, n, f, mo, e2, [&](int j) { return (sd[j] + se[j]) * sw[j]; },
                    a.W + mv.moff);
     } else if (a.W != nullptr) {
       for (int64_t t = tm.tid; t < (int64_t)mo * n; t += tm.nthr) {
@@ -862,7 +1075,7 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
 // One CTA per molecule of size class `cls` (0: NT = 256, two per SM;
 // 1: NT = 512, one per SM); CTA i takes the i-th molecule of the launch order.
 template <int NT, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_scf(ScfArgs a, int cls) {
+__global__ void __launch_bounds__(NT, MINB) k_scf(const __grid_constant__ ScfArgs a, int cls) {
   extern __shared__ double dsm[];
   const int i = blockIdx.x;
   const int m = a.order ? a.order[i] : i;
@@ -880,7 +1093,7 @@ __global__ void __launch_bounds__(NT, MINB) k_scf(ScfArgs a, int cls) {
 // clusters of the launch take the molecules of the class in launch order,
 // round robin. Every CTA of a cluster walks the same list, so the team's
 // control flow is uniform.
-__global__ void __launch_bounds__(kScfBigThreads, 1) k_scf_cluster(ScfArgs a, int cls) {
+__global__ void __launch_bounds__(kScfBigThreads, 1) k_scf_cluster(const __grid_constant__ ScfArgs a, int cls) {
   extern __shared__ double dsm[];
   Team<true> tm;
   tm.rank = (int)cluster_ctarank();
