@@ -35,11 +35,11 @@ DEFAULT = (112, 136, 160, 320, 640)
 # thresholds of classes 1..5 (one-SM CTA, clusters of 2, 4, 8, 16)
 CANDIDATES = [
     DEFAULT,
-    (100, 136, 160, 320, 640),
-    (124, 136, 160, 320, 640),
-    (112, 144, 176, 320, 640),
-    (112, 128, 160, 320, 640),
-    (112, 136, 192, 384, 768),
+    (96, 136, 160, 320, 640),
+    (80, 112, 140, 320, 640),
+    (96, 136, 180, 240, 320),
+    (112, 160, 220, 260, 320),
+    (30, 80, 110, 140, 640),
 ]
 _applied: dict = {}
 

@@ -396,6 +396,7 @@ struct Fast {
   int2 *vm;                  // atomic dipole and quadrupole potential, [9][nat]
   long long *pop;            // populations: charge and moments per orbital, [10][n]
   int eS, eD, eQ, eH;        // |S| <= 2^eS, ...
+  int own_tables;            // vo and vm are in shared memory
   int nat, nm;               // atoms; 10 matrices in M, or 1 without multipoles
   int xtm;                   // largest xte
   int cur;                   // VT in use
@@ -441,6 +442,7 @@ __device__ inline Fast fast_carve(double *base, int n, int nat, bool multipole) 
   f.vo = (long long *)take(8 * (int64_t)n);
   f.vm = (int2 *)take(8 * 9 * (int64_t)nat);
   f.pop = (long long *)take(8 * 10 * (int64_t)n);
+  f.own_tables = 0;
   f.nat = nat;
   f.nm = multipole ? 10 : 1;
   f.cur = 0;
@@ -1000,7 +1002,7 @@ __device__ bool fast_eigen(Team<CL> &tm, int n, Fast &f, double *lam, double *sk
     step_update_planes(tm, n, f, sc, ke);
     // a coarse step that no longer shrinks the rotations has met its own rounding
     // (pairs closer than ~2^-17 of the norm): full steps from here on
-    if (low && zm < 0.125f && zm > 0.7f * zprev) stalled = true;
+    if (low && zm < 0x1p-6f && zm > 0.9f * zprev) stalled = true;
     zprev = zm;
     low = !last && !stalled && zm > kZLow;
     tiles<kDigLow>(tm, n, f, kApply, ke, low ? 0 : 1, nullptr);
@@ -1107,7 +1109,8 @@ __device__ __noinline__ bool fast_fock(Team<CL> &tm, int n, Fast &f, const doubl
     if (f.nm > 1) E = max(E, max(f.eD + ex(vd), f.eQ + ex(vq)));
     s = E;
     for (int t = tm.tid; t < f.nm * n; t += tm.nthr) f.pop[t] = 0;  // for this iteration's populations
-    for (int t = tm.tid; t < N; t += tm.nthr) {
+    // tables in shared memory are every CTA's own
+    for (int t = f.own_tables ? (int)threadIdx.x : tm.tid; t < N; t += f.own_tables ? (int)blockDim.x : tm.nthr) {
       const double v = ld<CL>(x + t);
       if (t < n) {
         f.vo[t] = fix(v, 53 - E + f.eS);
@@ -1138,64 +1141,54 @@ __device__ __noinline__ bool fast_fock(Team<CL> &tm, int n, Fast &f, const doubl
       for (int k = 0; k < 2; ++k) ar[k] = aoat[r[k]];
 #pragma unroll
       for (int k = 0; k < 4; ++k) ac[k] = aoat[c[k]];
-      // two matrices at a time: a 16-byte word of the pair (i, j) and of (j, i);
-      // the words of the next two are loaded ahead (their latency bounds this)
+      // two matrices at a time (matrix 0 is S), first the pairs (i, j) with the
+      // column atom's potential, then the mirrors (j, i) with the row atom's
       const int4 *M = f.M + (size_t)t * kPairWords + (threadIdx.x & 31);
-#pragma unroll 1
-      for (int h = 0; h < 2; ++h) {
-        long long b0[4], b1[4];
-        int4 x[4], y[4];
+      long long a1[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) a0[e] = a1[e] = 0;
+#pragma unroll
+      for (int m = 0; m < 5; ++m) {
+        int4 x[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = M[m * 512 + e * 32];
+        const int2 *u = f.vm + 2 * m * nat;
+        int2 vc[4], uc[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          b0[k] = b1[k] = 0;
-          x[k] = M[(4 * h + k) * 32];
-          y[k] = M[(8 + 4 * h + k) * 32];
-        }
-        const int h2 = 2 * h;
-        const int c0 = h ? c[2] : c[0], c1 = h ? c[3] : c[1], q0 = h ? ac[2] : ac[0], q1 = h ? ac[3] : ac[1];
-#pragma unroll
-        for (int m = 0; m < 5; ++m) {
-          int4 xn[4], yn[4];
-          if (m < 4) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              xn[k] = M[(m + 1) * 512 + (4 * h + k) * 32];
-              yn[k] = M[(m + 1) * 512 + (8 + 4 * h + k) * 32];
-            }
-          }
-          const int2 *v = f.vm + (2 * m - 1) * nat, *u = v + nat;  // matrix 0 is S
-          int2 vr[2], vc[2], ur[2], uc[2];
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            vr[k] = m ? v[ar[k]] : make_int2(0, 0);
-            ur[k] = u[ar[k]];
-            vc[k] = m ? v[k ? q1 : q0] : make_int2(0, 0);
-            uc[k] = u[k ? q1 : q0];
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int kr = k >> 1, kc = k & 1;
-            if (m == 0) mul_add(b0[k], b1[k], make_int2(x[k].x, x[k].y), halves(f.vo[r[kr]] + f.vo[kc ? c1 : c0]));
-            else mul_add(b0[k], b1[k], make_int2(x[k].x, x[k].y), vc[kc]);
-            if (m) mul_add(b0[k], b1[k], make_int2(y[k].x, y[k].y), vr[kr]);
-            mul_add(b0[k], b1[k], make_int2(x[k].z, x[k].w), uc[kc]);
-            mul_add(b0[k], b1[k], make_int2(y[k].z, y[k].w), ur[kr]);
-          }
-          if (m < 4) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              x[k] = xn[k];
-              y[k] = yn[k];
-            }
-          }
+          if (m) vc[k] = u[ac[k] - nat];
+          uc[k] = u[ac[k]];
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          // |b0| < 20 2^50: the sum in units of 2^(E - 58) fits
-          const long long acc = b0[k] * 256 + (b1[k] >> 20);
-          if (h2) a0[4 + k] = acc; else a0[k] = acc;
+        for (int e = 0; e < 8; ++e) {
+          const int kc = (e >> 2) * 2 + (e & 1);
+          mul_add(a0[e], a1[e], make_int2(x[e].x, x[e].y),
+                  m ? vc[kc] : halves(f.vo[r[(e >> 1) & 1]] + f.vo[c[kc]]));
+          mul_add(a0[e], a1[e], make_int2(x[e].z, x[e].w), uc[kc]);
         }
       }
+#pragma unroll
+      for (int m = 0; m < 5; ++m) {
+        int4 y[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) y[e] = M[m * 512 + 256 + e * 32];
+        const int2 *u = f.vm + 2 * m * nat;
+        int2 vr[2], ur[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          if (m) vr[k] = u[ar[k] - nat];
+          ur[k] = u[ar[k]];
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const int kr = (e >> 1) & 1;
+          if (m) mul_add(a0[e], a1[e], make_int2(y[e].x, y[e].y), vr[kr]);
+          mul_add(a0[e], a1[e], make_int2(y[e].z, y[e].w), ur[kr]);
+        }
+      }
+      // |a0| < 20 2^50: the sum in units of 2^(E - 58) fits
+#pragma unroll
+      for (int e = 0; e < 8; ++e) a0[e] = a0[e] * 256 + (a1[e] >> 20);
     } else {
 #pragma unroll
       for (int e = 0; e < 8; ++e) {

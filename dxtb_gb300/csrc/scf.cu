@@ -712,7 +712,16 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
     mv.nsh = (int)(b.shell_off[m + 1] - mv.s0);
     mv.N = mv.n + (multipole ? 9 * mv.nat : 0);
     w = ws_carve(a.ws + a.ws_off[m], mv.n, mv.nat);
-    if (a.fast) f = fast_carve(a.ws + a.ws_off[m] + ws_size_base(mv.n, mv.nat), mv.n, mv.nat, multipole);
+    if (a.fast) {
+      f = fast_carve(a.ws + a.ws_off[m] + ws_size_base(mv.n, mv.nat), mv.n, mv.nat, multipole);
+      uint32_t dyn;
+      asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
+      if ((size_t)8 * (5 * mv.n + 9 * mv.nat) <= dyn) {
+        f.vo = reinterpret_cast<long long *>(dsm + 4 * mv.n);
+        f.vm = reinterpret_cast<int2 *>(dsm + 5 * mv.n);
+        f.own_tables = 1;
+      }
+    }
   }
   __syncthreads();
   const int n = mv.n, nat = mv.nat, N = mv.N;
@@ -1122,7 +1131,17 @@ namespace dxtb {
 
 // Size-class thresholds (smallest n of classes 1..5), process-wide.
 static std::mutex g_policy_mutex;
+static constexpr int kDefaultThr[kClasses] = {0, 112, 136, 160, 320, 640};
 static int g_thr[kClasses] = {0, 112, 136, 160, 320, 640};
+// One or two molecules leave most SMs idle: under the default policy they take
+// larger teams. Energy + forces of one GFN2 molecule, ms, by team (256 threads,
+// 512, clusters of 4, 8, 16): n = 33 7.9 7.4 8.7 8.9 9.6; 49 12.6 10.4 10.9
+// 11.2 11.9; 72 16.1 12.9 11.9 12.2 13.0; 106 33.4 25.3 17.1 16.1 16.8; 150 -
+// 65 29.6 25.5 24.1; 233 - - 60.9 41.0 35.3. From nine molecules on clusters
+// of 16 no longer run at once; two keep within a quarter of the SMs, which
+// leaves callers with several such batches in flight (a serving loop) theirs.
+static constexpr int kFewThr[kClasses] = {0, 30, 60, 60, 90, 130};
+constexpr int kFewMolecules = 2;
 
 // Side streams and fork/join events per (device, caller stream), created once
 // (no device memory is allocated); all launches stay inside a caller's
@@ -1242,13 +1261,18 @@ static int32_t class_gradient(const ScfArgs &a, const GradArgs *g, int c, cudaSt
 static int32_t launch_scf(ScfArgs a, int nmol, cudaStream_t st, const GradArgs *g = nullptr) {
   {
     std::lock_guard<std::mutex> lock(g_policy_mutex);
-    for (int c = 0; c < kClasses; ++c) a.thr[c] = g_thr[c];
+    bool preset = nmol <= kFewMolecules;
+    for (int c = 0; c < kClasses; ++c) {
+      a.thr[c] = g_thr[c];
+      preset = preset && g_thr[c] == kDefaultThr[c];
+    }
+    if (preset)
+      for (int c = 0; c < kClasses; ++c) a.thr[c] = min(a.thr[c], kFewThr[c]);
   }
   int sms = 0;
   if (device_sms(&sms) != DXTB_OK) return DXTB_ERR_LAUNCH;
   const int nmax = a.b.max_nao;
-  const size_t smem = (size_t)nmax * (3 * sizeof(double) + 2 * sizeof(float));
-  if (smem > kMaxDynSmem) return DXTB_ERR_TOO_LARGE;
+  if ((size_t)nmax * 32 > kMaxDynSmem) return DXTB_ERR_TOO_LARGE;
   // clusters need the launch order; classes beyond the cluster cap fold down
   int top = a.order ? 5 : 1;
   if (top > 1 && scf_class(a.thr, nmax) >= 2) {
@@ -1281,7 +1305,13 @@ static int32_t launch_scf(ScfArgs a, int nmol, cudaStream_t st, const GradArgs *
       }) != DXTB_OK)
     return DXTB_ERR_LAUNCH;
   // shared memory of every class: the base. The L1 serves the digit planes.
-  auto class_smem = [&](int) -> size_t { return smem; };
+  // shared memory of class c: 4 n doubles and, while that leaves most of the
+  // L1, the tables of the potential (n + 9 nat)
+  auto class_smem = [&](int c) -> size_t {
+    const size_t nub = c + 1 < kClasses ? (size_t)min(nmax, a.thr[c + 1]) : (size_t)nmax;
+    const size_t tables = 8 * nub + 72 * (size_t)a.b.max_nat;
+    return 32 * nub + (32 * nub + tables <= 64 * 1024 ? tables : 0);
+  };
   // largest classes first: clusters, then one-SM CTAs, then the shared SMs
   for (int c = cmax; c >= 2; --c) {
     const int csize = 1 << (c - 1);
@@ -1324,9 +1354,8 @@ static int32_t launch_scf(ScfArgs a, int nmol, cudaStream_t st, const GradArgs *
     const int32_t rc = launch_cta_class(k_scf<kScfBigThreads, 1>, 1, kScfBigThreads, class_smem(1));
     if (rc != DXTB_OK) return rc;
   }
-  const size_t smem0 = (size_t)min(nmax, a.thr[1]) * (3 * sizeof(double) + 2 * sizeof(float));
   {
-    const int32_t rc = launch_cta_class(k_scf<kScfThreads, 2>, 0, kScfThreads, smem0);
+    const int32_t rc = launch_cta_class(k_scf<kScfThreads, 2>, 0, kScfThreads, class_smem(0));
     if (rc != DXTB_OK) return rc;
   }
   if (ss) {

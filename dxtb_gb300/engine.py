@@ -204,12 +204,14 @@ def _seg_sum(values: torch.Tensor, seg: torch.Tensor, nmol: int) -> torch.Tensor
 GB_KERNELS = {"p16": 0, "still": 1}
 
 
-def scf_launches(L, nmax: int) -> int:
-    """Kernels launched by dxtb_scf for a batch whose largest molecule has
-    nmax orbitals: one per cluster class up to the largest one present, the
-    one-SM launch, the shared-SM launch."""
+def scf_launches(L, nmax: int, nmol: int = 0) -> int:
+    """Kernels launched by dxtb_scf for a batch (of nmol molecules) whose
+    largest has nmax orbitals: one per cluster class up to the largest one
+    present, the one-SM launch, the shared-SM launch."""
     thr = (C.c_int32 * 5)()
     _lib.check(L.dxtb_scf_get_size_classes(thr), "size classes")
+    if 0 < nmol <= 2 and tuple(thr) == (112, 136, 160, 320, 640):
+        thr = (30, 60, 60, 90, 130)  # the library's teams for one or two molecules
     cmax = sum(1 for t in thr if nmax >= t)
     return 1 + (1 if cmax >= 1 else 0) + max(0, cmax - 1)
 
@@ -358,7 +360,7 @@ def run(pb: PackedBatch, *, etemp: float = 300.0, maxiter: int = 250, tol: float
                 _lib.ptr(W), Cm.data_ptr(), ev.data_ptr(), occ.data_ptr(), q.data_ptr(),
                 dp.data_ptr(), qp.data_ptr(), vorb.data_ptr(), vdp.data_ptr(), vqp.data_ptr(),
                 en.data_ptr(), status.data_ptr())
-    n_scf = scf_launches(L, int(pb.nao.max()))
+    n_scf = scf_launches(L, int(pb.nao.max()), pb.nmol)
     grad = None
     if forces:
         # SCF and gradient fused per size class: each class's forces overlap
