@@ -18,9 +18,10 @@
 // of 16 x 16 values is one 16-byte word per lane and plane. The four registers
 // of an A operand (rows i, inner index k) in the order 0, 2, 1, 3 are those of
 // two B operands (C = A B^T), so a matrix is stored in the order of the side
-// it stands on ("left" or "right"; X and V stand on both), and no register is
-// moved between a load and the instruction. A result tile has the layout of
-// an A operand, transposed blocks come from movmatrix.
+// it stands on ("left" or "right") and no register is moved between a load and
+// the instruction; X and V stand on both and are stored for the left only (a
+// second copy cost more in L2 misses than the moves). A result tile has the
+// layout of an A operand, transposed blocks come from movmatrix.
 //
 // Eigenvectors are iterated (Ogita and Aishima, Japan J. Indust. Appl. Math.
 // 35 (2018) 1007, here with the first-order rotation clamped): for approximate
@@ -70,6 +71,21 @@ __device__ __forceinline__ uint4 ld_plane(const uint4 *p) {
                : "l"(__cvta_generic_to_global(p)));
   return v;
 }
+// A word read once per pass over data that exceeds the caches (the integrals,
+// 80 bytes a pair): kept out of the L1 and first to leave the L2, where the
+// planes of the running steps should stay.
+__device__ __forceinline__ uint64_t stream_policy() {
+  uint64_t pol;
+  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+  return pol;
+}
+__device__ __forceinline__ int4 ld_stream(const int4 *p, uint64_t pol) {
+  int4 v;
+  asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v4.s32 {%0,%1,%2,%3}, [%4], %5;"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(__cvta_generic_to_global(p)), "l"(pol));
+  return v;
+}
 __device__ __forceinline__ void st_plane(uint4 *p, const uint4 &v) {
   asm volatile("st.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(__cvta_generic_to_global(p)), "r"(v.x), "r"(v.y),
                "r"(v.z), "r"(v.w)
@@ -83,7 +99,7 @@ __device__ __forceinline__ void st_plane(uint4 *p, const uint4 &v) {
 // 8 (e >> 2) + 2 q + (e & 1) for lane 4 g + q. Every 128 terms the orders are
 // carried into the one above (multiples of 512), which keeps them exact.
 template <int NP>
-__device__ __forceinline__ void tile_nt(const uint4 *A, int sa, const uint4 *B, int sb, int k0, int k1,
+__device__ __forceinline__ void tile_nt(const uint4 *A, int sa, const uint4 *B, int sb, bool left_b, int k0, int k1,
                                         float (&acc)[NP][8]) {
   const int lane = threadIdx.x & 31;
   const uint4 *pa = A + (size_t)k0 * sa + lane, *pb = B + (size_t)k0 * sb + lane;
@@ -100,7 +116,12 @@ __device__ __forceinline__ void tile_nt(const uint4 *A, int sa, const uint4 *B, 
     for (int p = 0; p < NP; ++p) a[p] = ld_plane(pa + p * 32);
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
-      const uint4 b = ld_plane(pb + q * 32);
+      uint4 b = ld_plane(pb + q * 32);
+      if (left_b) {  // the order of the left side: swap the middle words
+        const uint32_t y = b.y;
+        b.y = b.z;
+        b.z = y;
+      }
 #pragma unroll
       for (int p = 0; p < NP - q; ++p) {
         mma16816(acc[p + q], a[p], b.x, b.y);
@@ -373,7 +394,7 @@ __host__ __device__ inline int64_t fast_size(int64_t n, int64_t nat) {
   const int64_t nb = blocks16(n), np2 = 256 * nb * nb;
   // planes of six digits are 12 bytes a value (3/2 doubles), of three 3/4;
   // the integrals S, D, Q in fixed point; potential and population tables
-  return (7 * 3 * np2) / 2 + (3 * 3 * np2) / 4 + 2 * np2 + 6 * 16 * nb + 64 + 64 +
+  return (5 * 3 * np2) / 2 + (2 * 3 * np2) / 4 + 2 * np2 + 6 * 16 * nb + 64 + 64 +
          nb * (nb + 1) / 2 * kPairWords * 2 + (n + 9 * nat) + 10 * n + 8;
 }
 
@@ -381,9 +402,9 @@ __host__ __device__ inline int64_t fast_size(int64_t n, int64_t nat) {
 // its 300 bytes a thread filled the L1. Written by thread 0 between barriers.
 struct Fast {
   int nb;
-  uint4 *Xl, *Xr, *XTl;      // X = L^-1 for both sides, X^T for the left
+  uint4 *Xl, *XTl;           // X = L^-1 and its transpose
   uint4 *Fr, *Gl;            // F, F', weighted C^T (right); H, G, C^T (left)
-  uint4 *Vl, *Vr, *VT[2], *El;  // V for both sides, V^T (right), E^T (left)
+  uint4 *Vl, *VT[2], *El;    // V (left), V^T (right), E^T (left, in G's memory)
   long long *Vm, *Vm2;       // vectors, weight 2^-60, tile layout
   float *T, *R;              // tile layout (Vm2's memory)
   long long *td, *rd;        // diagonals of T and R
@@ -416,15 +437,13 @@ __device__ inline Fast fast_carve(double *base, int n, int nat, bool multipole) 
     return r;
   };
   f.Xl = (uint4 *)take(12 * np2);
-  f.Xr = (uint4 *)take(12 * np2);
   f.XTl = (uint4 *)take(12 * np2);
   f.Fr = (uint4 *)take(12 * np2);
   f.Gl = (uint4 *)take(12 * np2);
   f.Vl = (uint4 *)take(12 * np2);
-  f.Vr = (uint4 *)take(12 * np2);
   f.VT[0] = (uint4 *)take(6 * np2);
   f.VT[1] = (uint4 *)take(6 * np2);
-  f.El = (uint4 *)take(6 * np2);
+  f.El = f.Gl;
   f.Vm = (long long *)take(8 * np2);
   f.Vm2 = (long long *)take(8 * np2);
   f.T = (float *)f.Vm2;
@@ -476,9 +495,9 @@ __device__ __forceinline__ int tile_row(int e) { return ((threadIdx.x & 31) >> 2
 __device__ __forceinline__ int tile_col(int e) { return 8 * (e >> 2) + 2 * (threadIdx.x & 3) + (e & 1); }
 
 // Digit planes of the row-major n x n matrix M (TR: of its transpose) whose
-// row i is scaled by 2^-e[i], for the left side and, if given, the right.
+// row i is scaled by 2^-e[i], for the left side.
 template <bool TR, bool CL>
-__device__ __noinline__ void planes_of(Team<CL> &tm, int n, int nb, const double *M, uint4 *left, uint4 *right,
+__device__ __noinline__ void planes_of(Team<CL> &tm, int n, int nb, const double *M, uint4 *left,
                                        const int *ex) {
   for (int t = team_warp(tm); t < nb * nb; t += team_warps(tm)) {
     const int ti = t / nb, tj = t % nb;
@@ -492,7 +511,6 @@ __device__ __noinline__ void planes_of(Team<CL> &tm, int n, int nb, const double
     uint32_t w[kDig][4];
     cut_block<kDig>(r, w);
     put_left<kDig>(left + (size_t)t * kDig * 32, w);
-    if (right != nullptr) put_right<kDig>(right + (size_t)t * kDig * 32, w);
   }
 }
 
@@ -596,8 +614,8 @@ __device__ __noinline__ bool fast_setup(Team<CL> &tm, int n, const double *X, Fa
   const Four r = team_four(tm, Four{bad, top, 0.0f, 0.0f}, sm, f.red);
   if (r.m0 > 0.0f) return false;
   if (threadIdx.x == 0) f.xtm = (int)r.m1 - 128;
-  planes_of<false>(tm, n, f.nb, X, f.Xl, f.Xr, f.xe);
-  planes_of<true>(tm, n, f.nb, X, f.XTl, (uint4 *)nullptr, f.xte);
+  planes_of<false>(tm, n, f.nb, X, f.Xl, f.xe);
+  planes_of<true>(tm, n, f.nb, X, f.XTl, f.xte);
   tm.sync();
   return true;
 }
@@ -619,7 +637,6 @@ __device__ __noinline__ void fast_identity(Team<CL> &tm, int n, Fast &f) {
     uint32_t w[kDig][4];
     cut_block<kDig>(r, w);
     put_left<kDig>(f.Vl + (size_t)t * kDig * 32, w);
-    put_right<kDig>(f.Vr + (size_t)t * kDig * 32, w);
     put_right_t<kDigLow>(f.VT[0] + ((size_t)tj * nb + ti) * kDigLow * 32, w);
   }
   if (threadIdx.x == 0) f.cur = 0;
@@ -678,6 +695,7 @@ __device__ __noinline__ float tiles(Team<CL> &tm, int n, const Fast &f, Product 
   for (int t = team_warp(tm); t < ntile; t += team_warps(tm)) {
     int ti, tj, k0 = 0, k1 = nb, sa = S6, sb = S6;
     const uint4 *A, *B;
+    bool left_b = false;   // B is stored for the left side
     bool square = false;  // a tile of the full matrix (else of the lower triangle)
     if (what == kApply || what == kHalf || (what == kStep && t < nb * nb)) {
       ti = t / nb;
@@ -703,21 +721,22 @@ __device__ __noinline__ float tiles(Team<CL> &tm, int n, const Fast &f, Product 
       B = VT + (size_t)tj * row3;
     } else {
       A = (what == kStep ? f.Vl : what == kHalf ? f.Xl : what == kCoeff ? f.XTl : f.Gl) + (size_t)ti * row6;
-      B = (what == kStep ? (square ? f.Fr : f.Vr)
+      B = (what == kStep ? (square ? f.Fr : f.Vl)
            : what == kHalf || dens ? f.Fr
-           : what == kFockX ? f.Xr : f.Vr) + (size_t)tj * row6;
+           : what == kFockX ? f.Xl : f.Vl) + (size_t)tj * row6;
+      left_b = !(what == kHalf || dens || (what == kStep && square));
     }
     longlong2 vm[4];  // kApply: the vectors to update, loaded ahead
     if (NP == kDigLow && what == kApply) {
-      const longlong2 *pv = reinterpret_cast<const longlong2 *>(f.Vm) + (size_t)t * 128 + lane;
+      const longlong2 *pv = reinterpret_cast<const longlong2 *>(f.Vm) + (size_t)(ti * nb + tj) * 128 + lane;
 #pragma unroll
       for (int h = 0; h < 4; ++h) vm[h] = pv[32 * h];
     }
     float acc[NP][8];
-    tile_nt<NP>(A, sa, B, sb, k0, k1, acc);
+    tile_nt<NP>(A, sa, B, sb, left_b, k0, k1, acc);
     const size_t blk = (size_t)ti * row6 + (size_t)tj * S6;
     if (NP == kDigLow && what == kApply) {
-      longlong2 *pv = reinterpret_cast<longlong2 *>(f.Vm) + (size_t)t * 128 + lane;
+      longlong2 *pv = reinterpret_cast<longlong2 *>(f.Vm) + (size_t)(ti * nb + tj) * 128 + lane;
       long long c[8];
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
@@ -733,13 +752,11 @@ __device__ __noinline__ float tiles(Team<CL> &tm, int n, const Fast &f, Product 
         uint32_t w[kDig][4];
         cut_block<kDig>(c, w);
         put_left<kDig>(f.Vl + blk, w);
-        put_right<kDig>(f.Vr + blk, w);
         put_right_t<kDigLow>(vt, w);
       } else {
         uint32_t w[kDigLow][4];
         cut_block<kDigLow>(c, w);
         put_left<kDigLow>(f.Vl + blk, w);
-        put_right<kDigLow>(f.Vr + blk, w);
         put_right_t<kDigLow>(vt, w);
       }
     } else if (square) {
@@ -939,7 +956,6 @@ __device__ __noinline__ void fast_sort(Team<CL> &tm, int n, Fast &f, double *lam
     uint32_t w[kDig][4];
     cut_block<kDig>(v, w);
     put_left<kDig>(f.Vl + (size_t)t * kDig * 32, w);
-    put_right<kDig>(f.Vr + (size_t)t * kDig * 32, w);
     put_right_t<kDigLow>(f.VT[f.cur ^ 1] + ((size_t)tj * nb + ti) * kDigLow * 32, w);
   }
   tm.sync();
@@ -1125,6 +1141,7 @@ __device__ __noinline__ bool fast_fock(Team<CL> &tm, int n, Fast &f, const doubl
     tm.sync();
   }
   const int E = s;
+  const uint64_t pol = stream_policy();
   Four sum = {0.0f, 0.0f, 0.0f, 0.0f};
   for (int t = team_warp(tm); t < nlow; t += team_warps(tm)) {
     int ti, tj;
@@ -1151,7 +1168,7 @@ __device__ __noinline__ bool fast_fock(Team<CL> &tm, int n, Fast &f, const doubl
       for (int m = 0; m < 5; ++m) {
         int4 x[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = M[m * 512 + e * 32];
+        for (int e = 0; e < 8; ++e) x[e] = ld_stream(M + m * 512 + e * 32, pol);
         const int2 *u = f.vm + 2 * m * nat;
         int2 vc[4], uc[4];
 #pragma unroll
@@ -1171,7 +1188,7 @@ __device__ __noinline__ bool fast_fock(Team<CL> &tm, int n, Fast &f, const doubl
       for (int m = 0; m < 5; ++m) {
         int4 y[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) y[e] = M[m * 512 + 256 + e * 32];
+        for (int e = 0; e < 8; ++e) y[e] = ld_stream(M + m * 512 + 256 + e * 32, pol);
         const int2 *u = f.vm + 2 * m * nat;
         int2 vr[2], ur[2];
 #pragma unroll
@@ -1193,7 +1210,7 @@ __device__ __noinline__ bool fast_fock(Team<CL> &tm, int n, Fast &f, const doubl
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const int i = r[(e >> 1) & 1], j = c[(e >> 2) * 2 + (e & 1)];
-        const int4 x = f.M[(size_t)t * kPairWords + e * 32 + (threadIdx.x & 31)];
+        const int4 x = ld_stream(f.M + (size_t)t * kPairWords + e * 32 + (threadIdx.x & 31), pol);
         long long b0 = 0, b1 = 0;
         mul_add(b0, b1, make_int2(x.x, x.y), halves(f.vo[i] + f.vo[j]));
         a0[e] = b0 * 256 + (b1 >> 20);
@@ -1236,6 +1253,7 @@ __device__ __noinline__ int fast_populations(Team<CL> &tm, int n, Fast &f) {
   int sh = 12;  // sums over n products of at most 2^50 in units of 2^(56 - sh)
   while (sh > 0 && ((int64_t)n << sh) > (int64_t(1) << 12)) --sh;
   const int nw = f.nm > 1 ? 5 : 1;
+  const uint64_t pol = stream_policy();
   for (int t = team_warp(tm); t < nlow; t += team_warps(tm)) {
     int ti, tj;
     lower_tile(t, ti, tj);
@@ -1252,7 +1270,7 @@ __device__ __noinline__ int fast_populations(Team<CL> &tm, int n, Fast &f) {
     const int mirror = f.nm > 1 ? 256 : 0;
     int4 x[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) x[e] = M[e * 32];
+    for (int e = 0; e < 8; ++e) x[e] = ld_stream(M + e * 32, pol);
 #pragma unroll 1
     for (int m = 0; m < nw; ++m) {
 #pragma unroll
@@ -1263,7 +1281,7 @@ __device__ __noinline__ int fast_populations(Team<CL> &tm, int n, Fast &f) {
           const bool turn = half == 1 || ti == tj;
           const int4 *next = M + (turn ? (m + 1 < nw ? (m + 1) * 512 : 0) : m * 512 + mirror);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) xn[e] = next[e * 32];
+          for (int e = 0; e < 8; ++e) xn[e] = ld_stream(next + e * 32, pol);
         }
         long long s[4][2];
         {
