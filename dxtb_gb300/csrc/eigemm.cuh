@@ -419,7 +419,6 @@ struct Fast {
   int eS, eD, eQ, eH;        // |S| <= 2^eS, ...
   int own_tables;            // vo and vm are in shared memory
   int nat, nm;               // atoms; 10 matrices in M, or 1 without multipoles
-  int xtm;                   // largest xte
   int cur;                   // VT in use
   bool warm;                 // V holds vectors of an earlier problem
   float z0;                  // first rotation of the last problem
@@ -593,7 +592,7 @@ __device__ __noinline__ bool fast_integrals(Team<CL> &tm, int n, Fast &f, const 
 template <bool CL>
 __device__ __noinline__ bool fast_setup(Team<CL> &tm, int n, const double *X, Fast &f, float4 *sm) {
   const int lane = threadIdx.x & 31;
-  float bad = 0.0f, top = 0.0f;
+  float bad = 0.0f;
   for (int q = team_warp(tm); q < 2 * n; q += team_warps(tm)) {
     const int i = q >> 1;
     const bool tr = q & 1;
@@ -608,12 +607,10 @@ __device__ __noinline__ bool fast_setup(Team<CL> &tm, int n, const double *X, Fa
     const bool ok = nrm > 0x1p-60f && nrm < 0x1p60f;
     if (!ok) bad = 1.0f;
     const int ex = ok ? exp_above(nrm) : 0;
-    if (tr) top = fmaxf(top, (float)(ex + 128));
     if (lane == 0) (tr ? f.xte : f.xe)[i] = ex;
   }
-  const Four r = team_four(tm, Four{bad, top, 0.0f, 0.0f}, sm, f.red);
+  const Four r = team_four(tm, Four{bad, 0.0f, 0.0f, 0.0f}, sm, f.red);
   if (r.m0 > 0.0f) return false;
-  if (threadIdx.x == 0) f.xtm = (int)r.m1 - 128;
   planes_of<false>(tm, n, f.nb, X, f.Xl, f.xe);
   planes_of<true>(tm, n, f.nb, X, f.XTl, f.xte);
   tm.sync();
@@ -667,6 +664,7 @@ __device__ __forceinline__ long long shift(long long x, int left) {
 // The products of a step, a Fock build and a density: which tiles, what
 // becomes of a result. One function per digit count: the instruction cache
 // does not hold a copy of the tile loop for each product.
+constexpr int kExpBias = 512;
 enum Product : int {
   kStep,    // G = V F (planes), R = I - V V^T (float32, lower tiles)
   kProject, // T = G V^T (float32, lower tiles)
@@ -674,7 +672,7 @@ enum Product : int {
   kHalf,    // H = X F (planes), X lower triangular
   kFockX,    // F' = H X^T (fixed point, lower tiles)
   kCoeff,   // C^T = X^T V^T (planes), the mo lowest vectors
-  kDensity, // P = C w C^T (fixed point, lower tiles)
+  kDensity, // P = C w C^T (fixed point, lower tiles); the diagonal's largest exponent + kExpBias
   kWeighted // the same in float64, both triangles
 };
 
@@ -801,7 +799,12 @@ __device__ __noinline__ float tiles(Team<CL> &tm, int n, const Fast &f, Product 
     } else if (what == kDensity) {
       long long c[8];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) c[e] = tile_fix(acc, e);
+      for (int e = 0; e < 8; ++e) {
+        c[e] = tile_fix(acc, e);
+        const int i = 16 * ti + tile_row(e);
+        if (ti == tj && tile_row(e) == tile_col(e) && i < n && c[e] > 0)
+          sum = fmaxf(sum, (float)(kExpBias + 2 * f.xte[i] + arg2 - 56 + 64 - __clzll(c[e])));
+      }
       put_tile(f.Ft, t, c);
     } else {
 #pragma unroll
@@ -815,7 +818,7 @@ __device__ __noinline__ float tiles(Team<CL> &tm, int n, const Fast &f, Product 
       }
     }
   }
-  if (what != kFockX) tm.sync();
+  if (what != kFockX && what != kDensity) tm.sync();  // these two are followed by a team_four
   return sum;
 }
 
@@ -1241,14 +1244,17 @@ __device__ __noinline__ bool fast_fock(Team<CL> &tm, int n, Fast &f, const doubl
 }
 
 // Populations sum_k P_ki M_c,ki of every orbital i for the 10 (1) matrices,
-// from the density in f.Ft (C w C^T with |w| <= 2): f.pop[c n + i] in units of
-// 2^(xte_i + xtm + 1 + eM - 106 + 56 - sh), sh returned. A lower tile serves the
+// from the density in f.Ft (C w C^T with 0 <= w <= 2): f.pop[c n + i] in units
+// of 2^(eP + eM - 106 + 56 - sh), sh returned. eP: every |P_ii| < 2^eP, hence
+// every |P_ij|: one unit for all of P. (Units by the row norms of X, from which
+// P is built, lose as many bits as these norms exceed P's entries, that is for
+// an ill-conditioned S.) A lower tile serves the
 // sums of its columns with the pairs and of its rows with their mirrors. Exact
 // sums of 53-bit factors: the order of the atomics does not matter.
 // In float64 (10 FMA a pair) this was bound by the FP64 pipe; here by the
 // loads, 80 bytes a pair, which the tile order makes contiguous.
 template <bool CL>
-__device__ __noinline__ int fast_populations(Team<CL> &tm, int n, Fast &f) {
+__device__ __noinline__ int fast_populations(Team<CL> &tm, int n, Fast &f, int eP) {
   const int lane = threadIdx.x & 31, nlow = f.nb * (f.nb + 1) / 2;
   int sh = 12;  // sums over n products of at most 2^50 in units of 2^(56 - sh)
   while (sh > 0 && ((int64_t)n << sh) > (int64_t(1) << 12)) --sh;
@@ -1259,12 +1265,11 @@ __device__ __noinline__ int fast_populations(Team<CL> &tm, int n, Fast &f) {
     lower_tile(t, ti, tj);
     long long p[8];
     get_tile(f.Ft, t, p);
-    int2 pc[8], pr[8];  // for the column sums (scaled by the row's exponent) and the row sums
+    int2 q[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int i = min(16 * ti + tile_row(e), n - 1), j = min(16 * tj + tile_col(e), n - 1);
-      pc[e] = halves(shift(p[e], f.xte[i] - f.xtm - 3));
-      pr[e] = ti == tj ? make_int2(0, 0) : halves(shift(p[e], f.xte[j] - f.xtm - 3));
+      q[e] = halves(shift(p[e], f.xte[i] + f.xte[j] + 1 - 56 + 53 - eP));
     }
     const int4 *M = f.M + (size_t)t * kPairWords + lane;
     const int mirror = f.nm > 1 ? 256 : 0;
@@ -1289,14 +1294,13 @@ __device__ __noinline__ int fast_populations(Team<CL> &tm, int n, Fast &f) {
 #pragma unroll
           for (int k = 0; k < 4; ++k)
 #pragma unroll
-            for (int c = 0; c < 2; ++c) a0[k][c] = a1[k][c] = 0;
+            for (int c = 0; c < 2; ++c) a0[k][c] = 0, a1[k][c] = 1ll << (27 - sh);  // to round
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             // columns: (e >> 2, e & 1); rows: (e >> 1) & 1
             const int k = half ? (e >> 1) & 1 : (e >> 2) * 2 + (e & 1);
-            const int2 q = half ? pr[e] : pc[e];
-            mul_add(a0[k][0], a1[k][0], q, make_int2(x[e].x, x[e].y));
-            mul_add(a0[k][1], a1[k][1], q, make_int2(x[e].z, x[e].w));
+            mul_add(a0[k][0], a1[k][0], q[e], make_int2(x[e].x, x[e].y));
+            mul_add(a0[k][1], a1[k][1], q[e], make_int2(x[e].z, x[e].w));
           }
 #pragma unroll
           for (int k = 0; k < 4; ++k)
@@ -1376,9 +1380,11 @@ __device__ __forceinline__ void join_block(const uint4 *blk, long long (&r)[8]) 
 
 // C diag(w) C^T over the mo lowest orbitals from the planes of C^T in f.Gl;
 // w(j): weight of orbital j, |w| <= 2^sw. To out (both triangles), or without
-// it to f.Ft in units of 2^(xte_i + xte_j + sw - 56).
+// it to f.Ft in units of 2^(xte_i + xte_j + sw - 56); the returned eP bounds
+// this P, every |P_ii| < 2^eP.
 template <bool CL, typename W>
-__device__ __noinline__ void fast_density(Team<CL> &tm, int n, Fast &f, int mo, int sw, W w, double *out) {
+__device__ __noinline__ int fast_density(Team<CL> &tm, int n, Fast &f, int mo, int sw, W w, double *out,
+                                         float4 *sm) {
   const int nb = f.nb, mb = (int)blocks16(mo);
   for (int t = team_warp(tm); t < nb * mb; t += team_warps(tm)) {
     const int ti = t / mb, tj = t % mb;
@@ -1396,7 +1402,10 @@ __device__ __noinline__ void fast_density(Team<CL> &tm, int n, Fast &f, int mo, 
     put_right<kDig>(f.Fr + o, d);
   }
   tm.sync();
-  tiles<kDig>(tm, n, f, out != nullptr ? kWeighted : kDensity, mo, sw, out);
+  const float top = tiles<kDig>(tm, n, f, out != nullptr ? kWeighted : kDensity, mo, sw, out);
+  if (out != nullptr) return 0;
+  const Four r = team_four(tm, Four{top, 0.0f, 0.0f, 0.0f}, sm, f.red);
+  return max((int)r.m0 - kExpBias, -60);
 }
 
 // The mo lowest orbitals' coefficients, row j of C (n x n, the rest zero).

@@ -818,12 +818,12 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
       mo = s_mo;
       // ---- C^T, then P = C diag(occ) C^T (scf/utils.py:29-52) ----
       tiles<kDig>(tm, n, f, kCoeff, mo, 0, nullptr);
-      fast_density(tm, n, f, mo, 1, [&](int j) { return fa[j] + fb[j]; }, (double *)nullptr);
+      const int eP = fast_density(tm, n, f, mo, 1, [&](int j) { return fa[j] + fb[j]; }, (double *)nullptr, sfour);
       // ---- Mulliken charges and atomic multipoles (conversions.py:203-251) ----
-      const int u = f.xtm + 1 - 50 - fast_populations(tm, n, f);
-      // orbital o's sum with matrix c counts 2^(u + xte[o] + exponent of the matrix)
+      const int u = eP - 50 - fast_populations(tm, n, f, eP);
+      // orbital o's sum with matrix c counts 2^(u + exponent of the matrix)
       auto pop = [&](int c, int o) {
-        return unfix(__ldcg(f.pop + (size_t)c * n + o), u + f.xte[o] + (c == 0 ? f.eS : c < 4 ? f.eD : f.eQ));
+        return unfix(__ldcg(f.pop + (size_t)c * n + o), u + (c == 0 ? f.eS : c < 4 ? f.eD : f.eQ));
       };
       for (int i = tm.tid; i < n; i += tm.nthr) qo[i] = n0[i] - pop(0, i);
       for (int t = tm.tid; t < f.nm * mv.nsh; t += tm.nthr) {
@@ -1063,7 +1063,7 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
       const double top = fmax(fabs(sw[0]), fabs(sw[n - 1]));
       const int e2 = top > 1e-30 ? exp_above((float)top) + 1 : 0;
       fast_density(tm, n, f, mo, e2, [&](int j) { return (sd[j] + se[j]) * sw[j]; },
-                   a.W + mv.moff);
+                   a.W + mv.moff, sfour);
     } else if (a.W != nullptr) {
       for (int64_t t = tm.tid; t < (int64_t)mo * n; t += tm.nthr) {
         const int j = (int)(t / n);
