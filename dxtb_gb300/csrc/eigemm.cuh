@@ -3,16 +3,21 @@
 //
 // The FP64 pipe of this part issues 1.7 FMA per clock and SM, the 16-bit
 // tensor instruction (mma.sync m16n8k16) 1020 (both measured): a product of
-// 54-bit fixed-point operands cut into six digits of nine bits takes 21 digit
-// products (those above 2^-54 of the largest), still ~28 times the FP64 rate,
-// and is exact but for the digits left out: a digit product sum over 128
-// terms stays below 2^24, where the float32 accumulator holds every integer.
-// Sums over more terms are drained into 64-bit integers every 128.
+// 60-bit fixed-point operands cut into six digits of ten bits takes 21 digit
+// products (orders p + q <= 5), still ~28 times the FP64 rate. The orders left
+// out are 2^-64 sqrt(5 n) of the operands' norms. The digit product sums are
+// integers in float32 accumulators, exact below 2^24: the orders 0 to 2 for any
+// operands of norm <= 1 (order 2 is carried upwards every 32 terms), the orders
+// from 3 on, of weight <= 2^-50, every 64 terms and for digits that are not all
+// at their limit (they would round, not overflow).
+// Nine-bit digits (54 bits) lost 2^-58 sqrt(5 n), with a sign on a diagonal: SCF
+// residuals then end at 6e-12 (n = 181) to 6e-10 (n = 1145), where float64 ends
+// at 6e-13 to 4e-12.
 //
-// Fixed point: an operand's value is sum_p digit_p 2^(-9 (p + 1)) times a
+// Fixed point: an operand's value is sum_p digit_p 2^(-10 (p + 1)) times a
 // power of two kept beside the matrix (per matrix or per row); digits are
-// balanced (|digit| <= 256) but the first, which takes the rest (|.| <= 2047,
-// exact in fp16, so |value| < 4). Results are 64-bit integers of weight 2^-56.
+// balanced (|digit| <= 512) but the first, which takes the rest (|.| <= 2048,
+// exact in fp16, so |value| <= 2). Results are 64-bit integers of weight 2^-58.
 //
 // Digit planes are stored in the register layout of the instruction: a block
 // of 16 x 16 values is one 16-byte word per lane and plane. The four registers
@@ -47,12 +52,12 @@ namespace dxtb {
 
 constexpr int kDig = 6;          // digits of a full operand
 constexpr int kDigLow = 3;       // digits of the coarse steps and of the rotations
-constexpr int kDrain = 8;        // k blocks of 16 per float32 accumulation
+constexpr int kW = 60, kR = 58;  // an operand's last digit weighs 2^-kW, results 2^-kR
 constexpr int kMaxSteps = 160;   // steps of one eigenproblem before it is given up
 constexpr float kZMax = 0.4f;    // largest rotation of one pair in one step
 constexpr float kZNorm = 1.2f;   // largest Frobenius norm (over sqrt 2) of the rotations of a small problem
-constexpr float kZFinal = 0x1p-30f;  // a full step below this is the last (its error is quadratic)
-constexpr float kZLow = 0x1p-10f;    // above this the next step is coarse
+constexpr float kFinal = 0x1p-28f;   // a full step of this Frobenius norm is the last (its error is quadratic)
+constexpr float kZLow = 0x1p-7f;    // above this the next step is coarse
 
 __host__ __device__ inline int64_t blocks16(int64_t n) { return (n + 15) / 16; }
 
@@ -93,11 +98,11 @@ __device__ __forceinline__ void st_plane(uint4 *p, const uint4 &v) {
 }
 
 // The 16 x 16 tile sum_k A[i][k] B[j][k] over the k blocks [k0, k1) with NP
-// digits, as the sums of each order (acc[d], weight 2^(-9 (d + 2)), exact
+// digits, as the sums of each order (acc[d], weight 2^(-10 (d + 2)), exact
 // integers): A, B are the first blocks of the two block rows, sa, sb the words
 // per block (planes stored x 32). Value e: row g + 8 ((e >> 1) & 1), column
-// 8 (e >> 2) + 2 q + (e & 1) for lane 4 g + q. Every 128 terms the orders are
-// carried into the one above (multiples of 512), which keeps them exact.
+// 8 (e >> 2) + 2 q + (e & 1) for lane 4 g + q. Orders are carried into the one
+// above (multiples of 1024), which keeps them exact.
 template <int NP>
 __device__ __forceinline__ void tile_nt(const uint4 *A, int sa, const uint4 *B, int sb, bool left_b, int k0, int k1,
                                         float (&acc)[NP][8]) {
@@ -107,6 +112,7 @@ __device__ __forceinline__ void tile_nt(const uint4 *A, int sa, const uint4 *B, 
   for (int p = 0; p < NP; ++p)
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[p][e] = 0.0f;
+  constexpr int kDrain = NP == kDigLow ? 8 : 4;  // k blocks of 16 between carries of all orders
   int left = kDrain;
   constexpr int kUnroll = NP == kDigLow ? 2 : 1;  // loads of two k blocks in flight where registers allow
 #pragma unroll kUnroll
@@ -130,24 +136,26 @@ __device__ __forceinline__ void tile_nt(const uint4 *A, int sa, const uint4 *B, 
     }
     pa += sa;
     pb += sb;
+    auto carry = [&](int p) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float c = fmaf(acc[p][e], 0x1p-10f, 0x1.8p23f) - 0x1.8p23f;  // rounded to an integer
+        acc[p - 1][e] += c;
+        acc[p][e] = fmaf(-1024.0f, c, acc[p][e]);
+      }
+    };
     if (--left == 0) {
       left = kDrain;
       if (kb + 1 < k1) {
 #pragma unroll
-        for (int p = NP - 1; p > 0; --p)
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float c = fmaf(acc[p][e], 0x1p-9f, 0x1.8p23f) - 0x1.8p23f;  // rounded to an integer
-            acc[p - 1][e] += c;
-            acc[p][e] = fmaf(-512.0f, c, acc[p][e]);
-          }
+        for (int p = NP - 1; p > 0; --p) carry(p);
       }
+    } else if (NP == kDig && left == 2) {
+      carry(2);
     }
   }
 }
 
-// x rounded to an integer (|x| < 2^22)
-__device__ __forceinline__ float rint_f(float x) { return (x + 0x1.8p23f) - 0x1.8p23f; }
 // an integer in float32 (|x| < 2^22) as an int: no conversion (those run at
 // an eighth of the rate)
 __device__ __forceinline__ int int_f(float x) { return __float_as_int(x + 0x1.8p23f) - 0x4b400000; }
@@ -156,61 +164,61 @@ __device__ __forceinline__ int int_f(float x) { return __float_as_int(x + 0x1.8p
 // cancel the partial results are exact integers, so the error is relative.
 template <int NP>
 __device__ __forceinline__ float tile_float(const float (&acc)[NP][8], int e, bool less_one) {
-  float v = less_one ? acc[0][e] - 0x1p18f : acc[0][e];
+  float v = less_one ? acc[0][e] - 0x1p20f : acc[0][e];
 #pragma unroll
-  for (int p = 1; p < NP; ++p) v = fmaf(v, 512.0f, acc[p][e]);
-  return v * (NP == 6 ? 0x1p-63f : 0x1p-36f);
+  for (int p = 1; p < NP; ++p) v = fmaf(v, 1024.0f, acc[p][e]);
+  return v * (NP == 6 ? 0x1p-70f : 0x1p-40f);
 }
 
 // A tile's value e as the NP digits of an operand, and the rest below the last
-// (weight 2^(-9 (NP + 1)), |rest| <= 256). Carries in float32, all exact.
+// (weight 2^(-10 (NP + 1)), |rest| <= 512). Carries in float32, all exact.
 template <int NP>
 __device__ __forceinline__ float tile_digits(const float (&acc)[NP][8], int e, float (&d)[NP]) {
-  float c = fmaf(acc[NP - 1][e], 0x1p-9f, 0x1.8p23f) - 0x1.8p23f;
-  const float rest = fmaf(-512.0f, c, acc[NP - 1][e]);
+  float c = fmaf(acc[NP - 1][e], 0x1p-10f, 0x1.8p23f) - 0x1.8p23f;
+  const float rest = fmaf(-1024.0f, c, acc[NP - 1][e]);
 #pragma unroll
   for (int i = NP - 1; i > 0; --i) {
     const float x = acc[i - 1][e] + c;
-    c = fmaf(x, 0x1p-9f, 0x1.8p23f) - 0x1.8p23f;
-    d[i] = fmaf(-512.0f, c, x);
+    c = fmaf(x, 0x1p-10f, 0x1.8p23f) - 0x1.8p23f;
+    d[i] = fmaf(-1024.0f, c, x);
   }
   d[0] = c;
   return rest;
 }
 
-// A tile's value e as an integer of weight 2^-56.
+// A tile's value e as an integer of weight 2^-kR (|value| < 16).
 template <int NP>
 __device__ __forceinline__ long long tile_fix(const float (&acc)[NP][8], int e) {
   float d[NP];
   const float rest = tile_digits<NP>(acc, e, d);
-  const int hi = (int_f(d[0]) * 512 + int_f(d[1])) * 512 + int_f(d[2]);  // weight 2^-27
+  const long long hi = (long long)int_f(d[0]) * (1 << 20) + (int_f(d[1]) * 1024 + int_f(d[2]));  // weight 2^-30
   if constexpr (NP > 3) {
-    const int lo = ((int_f(d[3]) * 512 + int_f(d[4])) * 512 + int_f(d[5])) * 4 + int_f(fmaf(rest, 0x1p-7f, 0.0f));
-    return (long long)hi * (1 << 29) + lo;
+    const int lo = (int_f(d[3]) * 1024 + int_f(d[4])) * 1024 + int_f(d[5]);  // weight 2^-60
+    return hi * (1 << 28) + ((lo + 2) >> 2);
   } else {
-    return (long long)hi * (1 << 29) + int_f(rest) * (1 << 20);
+    return hi * (1 << 28) + int_f(rest) * (1 << 18);
   }
 }
 
-// Balanced digits of r (weight 2^-54), first digit first. With NP = 3 the
-// value is rounded to 2^-27, which leaves the first three digits of NP = 6.
+// Balanced digits of r (weight 2^-kW, |r| < 2^61), first digit first. With NP = 3
+// the value is rounded to 2^-30, which leaves the first three digits of NP = 6.
 template <int NP>
 __device__ __forceinline__ void cut(long long r, int (&d)[NP]) {
-  const int hi = (int)((r + (1 << 26)) >> 27);
+  const int hi = (int)((r + (1 << 29)) >> 30);
   if constexpr (NP == 6) {
-    const int lo = (int)(r - ((long long)hi << 27));
-    const int x1 = (lo + 256) >> 9, x2 = (x1 + 256) >> 9;
-    d[5] = lo - (x1 << 9);
-    d[4] = x1 - (x2 << 9);
+    const int lo = (int)(r - ((long long)hi << 30));
+    const int x1 = (lo + 512) >> 10, x2 = (x1 + 512) >> 10;
+    d[5] = lo - (x1 << 10);
+    d[4] = x1 - (x2 << 10);
     d[3] = x2;
   }
-  const int y1 = (hi + 256) >> 9, y2 = (y1 + 256) >> 9;
-  d[2] = hi - (y1 << 9);
-  d[1] = y1 - (y2 << 9);
+  const int y1 = (hi + 512) >> 10, y2 = (y1 + 512) >> 10;
+  d[2] = hi - (y1 << 10);
+  d[1] = y1 - (y2 << 10);
   d[0] = y2;
 }
 
-// Two digits as fp16. |d| <= 256: the bits of 1536 + d (unit spacing there)
+// Two digits as fp16. |d| <= 512: the bits of 1536 + d (unit spacing there)
 // minus 1536; the first digit by conversion.
 __device__ __forceinline__ uint32_t pack_small(int a, int b) {
   const uint32_t w = (uint32_t)(a + 0x6600) | ((uint32_t)(b + 0x6600) << 16);
@@ -236,16 +244,16 @@ __device__ __forceinline__ void cut_block(const long long (&r)[8], uint32_t (&w)
   }
 }
 
-// Digit words of values of weight 2^-27.
+// Digit words of values of weight 2^-30.
 __device__ __forceinline__ void cut_words(const int (&r)[8], uint32_t (&w)[kDigLow][4]) {
 #pragma unroll
   for (int h = 0; h < 4; ++h) {
     int d[2][3];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      const int x = r[2 * h + k], y1 = (x + 256) >> 9, y2 = (y1 + 256) >> 9;
-      d[k][2] = x - (y1 << 9);
-      d[k][1] = y1 - (y2 << 9);
+      const int x = r[2 * h + k], y1 = (x + 512) >> 10, y2 = (y1 + 512) >> 10;
+      d[k][2] = x - (y1 << 10);
+      d[k][1] = y1 - (y2 << 10);
       d[k][0] = y2;
     }
     w[0][h] = pack_first(d[0][0], d[1][0]);
@@ -405,7 +413,7 @@ struct Fast {
   uint4 *Xl, *XTl;           // X = L^-1 and its transpose
   uint4 *Fr, *Gl;            // F, F', weighted C^T (right); H, G, C^T (left)
   uint4 *Vl, *VT[2], *El;    // V (left), V^T (right), E^T (left, in G's memory)
-  long long *Vm, *Vm2;       // vectors, weight 2^-60, tile layout
+  long long *Vm, *Vm2;       // vectors, weight 2^-kW, tile layout
   float *T, *R;              // tile layout (Vm2's memory)
   long long *td, *rd;        // diagonals of T and R
   double *lam;               // eigenvalue of each row of V
@@ -505,7 +513,7 @@ __device__ __noinline__ void planes_of(Team<CL> &tm, int n, int nb, const double
     for (int e = 0; e < 8; ++e) {
       const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
       r[e] = 0;
-      if (i < n && j < n) r[e] = fix(ld<CL>(TR ? M + (size_t)j * n + i : M + (size_t)i * n + j), 54 - ldi<CL>(ex + i));
+      if (i < n && j < n) r[e] = fix(ld<CL>(TR ? M + (size_t)j * n + i : M + (size_t)i * n + j), kW - ldi<CL>(ex + i));
     }
     uint32_t w[kDig][4];
     cut_block<kDig>(r, w);
@@ -521,15 +529,18 @@ __device__ __forceinline__ float mag(double x) {
   return hi < 0x38100000 ? 0.0f : __int_as_float(((hi - 0x38000000) << 3) + 8);
 }
 
-// Fixed point with 53 bits in two signed halves: h 2^28 + l.
+// Fixed point with kFix bits and a sign in two signed halves: h 2^29 + l,
+// |h| <= 2^29, |l| <= 2^28. Five bits more than a float64 holds, since all
+// entries of a matrix share one exponent.
+constexpr int kFix = 58;
 __device__ __forceinline__ int2 halves(long long m) {
-  const int h = (int)((m + (1 << 27)) >> 28);
-  return make_int2(h, (int)(m - ((long long)h << 28)));
+  const int h = (int)((m + (1 << 28)) >> 29);
+  return make_int2(h, (int)(m - ((long long)h << 29)));
 }
 
-// A product of two such numbers without its low x low part (2^-50 of a unit
-// of h x h): three 32-bit multiply-adds in place of a float64 one, which
-// costs nineteen times an IMAD's issue on this part.
+// A product of two such numbers without its low x low part (at most 2^-60):
+// three 32-bit multiply-adds in place of a float64 one, which costs nineteen
+// times an IMAD's issue on this part. 20 products fit: |a0|, |a1| < 20 2^58.
 __device__ __forceinline__ void mul_add(long long &a0, long long &a1, int2 x, int2 y) {
   a0 += (long long)x.x * y.x;
   a1 += (long long)x.x * y.y;
@@ -572,11 +583,11 @@ __device__ __noinline__ bool fast_integrals(Team<CL> &tm, int n, Fast &f, const 
       for (int y = 0; y < (f.nm > 1 ? 2 : 1); ++y) {
         const int64_t o = y ? (int64_t)j * n + i : (int64_t)i * n + j;
         int2 m[10];
-        m[0] = halves(in ? fix(S[o], 53 - f.eS) : 0);
+        m[0] = halves(in ? fix(S[o], kFix - f.eS) : 0);
         int4 *out = f.M + (size_t)t * kPairWords + (y * 8 + e) * 32 + lane;
         if (f.nm > 1) {
-          for (int c = 0; c < 3; ++c) m[1 + c] = halves(in ? fix(D[c * mtot + o], 53 - f.eD) : 0);
-          for (int c = 0; c < 6; ++c) m[4 + c] = halves(in ? fix(Q[c * mtot + o], 53 - f.eQ) : 0);
+          for (int c = 0; c < 3; ++c) m[1 + c] = halves(in ? fix(D[c * mtot + o], kFix - f.eD) : 0);
+          for (int c = 0; c < 6; ++c) m[4 + c] = halves(in ? fix(Q[c * mtot + o], kFix - f.eQ) : 0);
           for (int c = 0; c < 5; ++c) out[c * 512] = make_int4(m[2 * c].x, m[2 * c].y, m[2 * c + 1].x, m[2 * c + 1].y);
         } else {
           *out = make_int4(m[0].x, m[0].y, 0, 0);
@@ -623,16 +634,15 @@ __device__ __noinline__ void fast_identity(Team<CL> &tm, int n, Fast &f) {
   const int nb = f.nb, lane = threadIdx.x & 31;
   for (int t = team_warp(tm); t < nb * nb; t += team_warps(tm)) {
     const int ti = t / nb, tj = t % nb;
-    long long v[8], r[8];
+    long long v[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
-      v[e] = (i == j && i < n) ? 1ll << 60 : 0;
-      r[e] = v[e] >> 6;
+      v[e] = (i == j && i < n) ? 1ll << kW : 0;
       f.Vm[(((size_t)t * 4 + (e >> 1)) * 32 + lane) * 2 + (e & 1)] = v[e];
     }
     uint32_t w[kDig][4];
-    cut_block<kDig>(r, w);
+    cut_block<kDig>(v, w);
     put_left<kDig>(f.Vl + (size_t)t * kDig * 32, w);
     put_right_t<kDigLow>(f.VT[0] + ((size_t)tj * nb + ti) * kDigLow * 32, w);
   }
@@ -739,11 +749,11 @@ __device__ __noinline__ float tiles(Team<CL> &tm, int n, const Fast &f, Product 
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
         longlong2 v = vm[h];
-        v.x += shift(tile_fix(acc, 2 * h), 4 - arg);  // weight 2^-56 2^-ke to 2^-60
-        v.y += shift(tile_fix(acc, 2 * h + 1), 4 - arg);
+        v.x += shift(tile_fix(acc, 2 * h), kW - kR - arg);  // weight 2^-kR 2^-ke to 2^-kW
+        v.y += shift(tile_fix(acc, 2 * h + 1), kW - kR - arg);
         pv[32 * h] = v;
-        c[2 * h] = (v.x + 32) >> 6;
-        c[2 * h + 1] = (v.y + 32) >> 6;
+        c[2 * h] = v.x;
+        c[2 * h + 1] = v.y;
       }
       uint4 *vt = VN + (size_t)tj * row3 + (size_t)ti * S3;
       if (arg2) {
@@ -780,7 +790,7 @@ __device__ __noinline__ float tiles(Team<CL> &tm, int n, const Fast &f, Product 
           const int i = 16 * ti + tile_row(e);
           if (tile_row(e) == tile_col(e)) {
             const long long v = tile_fix(acc, e);
-            if (isr) f.rd[i] = (i < n ? (1ll << 56) : 0) - v; else f.td[i] = v;
+            if (isr) f.rd[i] = (i < n ? (1ll << kR) : 0) - v; else f.td[i] = v;
           }
         }
       }
@@ -803,7 +813,7 @@ __device__ __noinline__ float tiles(Team<CL> &tm, int n, const Fast &f, Product 
         c[e] = tile_fix(acc, e);
         const int i = 16 * ti + tile_row(e);
         if (ti == tj && tile_row(e) == tile_col(e) && i < n && c[e] > 0)
-          sum = fmaxf(sum, (float)(kExpBias + 2 * f.xte[i] + arg2 - 56 + 64 - __clzll(c[e])));
+          sum = fmaxf(sum, (float)(kExpBias + 2 * f.xte[i] + arg2 - kR + 64 - __clzll(c[e])));
       }
       put_tile(f.Ft, t, c);
     } else {
@@ -811,7 +821,7 @@ __device__ __noinline__ float tiles(Team<CL> &tm, int n, const Fast &f, Product 
       for (int e = 0; e < 8; ++e) {
         const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
         if (i < n && j <= i) {
-          const double v = unfix(tile_fix(acc, e), f.xte[i] + f.xte[j] + arg2 - 56);
+          const double v = unfix(tile_fix(acc, e), f.xte[i] + f.xte[j] + arg2 - kR);
           out[(size_t)i * n + j] = v;
           out[(size_t)j * n + i] = v;
         }
@@ -829,17 +839,18 @@ __device__ __noinline__ Four step_rotations(Team<CL> &tm, int n, const Fast &f, 
                                             float *lh, float *ll, float4 *sm) {
   const int nb = f.nb, nlow = nb * (nb + 1) / 2, lane = threadIdx.x & 31;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const double t = (double)(CL ? __ldcg(f.td + i) : f.td[i]) * 0x1p-56;
-    const double r = (double)(CL ? __ldcg(f.rd + i) : f.rd[i]) * 0x1p-56;
+    const double t = (double)(CL ? __ldcg(f.td + i) : f.td[i]) * 0x1p-58;
+    const double r = (double)(CL ? __ldcg(f.rd + i) : f.rd[i]) * 0x1p-58;
     const double v = t * rcp_nr(1.0 - r);
     lam[i] = v;
     lh[i] = (float)v;
     ll[i] = (float)(v - (double)lh[i]);
   }
   __syncthreads();
-  // couplings at the rounding level of T are left alone (inside a degenerate
-  // level their ratio to the gap is noise)
-  const float thr = low ? 0x1p-24f : 0x1p-51f;
+  // inside a degenerate level couplings at the rounding level of T are left
+  // alone (their ratio to the gap is noise); above the gap `far` every coupling
+  // counts, since there thr / far is far below kFinal
+  const float thr = low ? 0x1p-26f : 0x1p-54f, far = low ? 4.0f : 0x1p-22f;
   Four s = {0.0f, 0.0f, 0.0f, 0.0f};
   for (int t = team_warp(tm); t < nlow; t += team_warps(tm)) {
     int ti, tj;
@@ -859,7 +870,7 @@ __device__ __noinline__ Four step_rotations(Team<CL> &tm, int n, const Fast &f, 
         if (i != j) {
           const float num = fmaf(0.5f * (lh[i] + lh[j]), r[e], z[e]);
           const float gap = (lh[j] - lh[i]) + (ll[j] - ll[i]);
-          if (!(fabsf(num) < thr)) {
+          if (!(fabsf(num) < thr && fabsf(gap) < far)) {
             v = fabsf(num) < kZMax * fabsf(gap) ? __fdividef(num, gap)
                                                 : (((__float_as_int(num) ^ __float_as_int(gap)) < 0) ? -kZMax : kZMax);
             if (!isfinite(num)) v = num;
@@ -885,7 +896,7 @@ __device__ __noinline__ Four step_rotations(Team<CL> &tm, int n, const Fast &f, 
 template <bool CL>
 __device__ __noinline__ void step_update_planes(Team<CL> &tm, int n, const Fast &f, float sc, int ke) {
   const int nb = f.nb, nlow = nb * (nb + 1) / 2, lane = threadIdx.x & 31;
-  const float up = ldexpf(1.0f, ke) * 0x1p27f;
+  const float up = ldexpf(1.0f, ke) * 0x1p30f;
   for (int t = team_warp(tm); t < nlow; t += team_warps(tm)) {
     int ti, tj;
     lower_tile(t, ti, tj);
@@ -896,7 +907,7 @@ __device__ __noinline__ void step_update_planes(Team<CL> &tm, int n, const Fast 
     *reinterpret_cast<float4 *>(z + 4) = pt[32];
     *reinterpret_cast<float4 *>(r) = pr[0];
     *reinterpret_cast<float4 *>(r + 4) = pr[32];
-    int a[8], b[8];  // weight 2^-27; zero outside the matrix
+    int a[8], b[8];  // weight 2^-30; zero outside the matrix
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       a[e] = __float2int_rn(fmaf(-sc, z[e], 0.5f * r[e]) * up);  // E_ji
@@ -953,8 +964,6 @@ __device__ __noinline__ void fast_sort(Team<CL> &tm, int n, Fast &f, double *lam
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
       out[32 * h] = make_longlong2(v[2 * h], v[2 * h + 1]);
-      v[2 * h] = (v[2 * h] + 32) >> 6;
-      v[2 * h + 1] = (v[2 * h + 1] + 32) >> 6;
     }
     uint32_t w[kDig][4];
     cut_block<kDig>(v, w);
@@ -976,7 +985,7 @@ __device__ __noinline__ void fast_sort(Team<CL> &tm, int n, Fast &f, double *lam
 
 // Eigenvectors (rows of V, ascending) and eigenvalues (lam, shared, every
 // CTA; in units of 2^s) of the matrix whose planes, scaled by 2^-s to a
-// Frobenius norm in (1, 2], are in f.Fr. False when the steps do not converge.
+// Frobenius norm in (1/2, 1], are in f.Fr. False when the steps do not converge.
 template <bool CL>
 __device__ bool fast_eigen(Team<CL> &tm, int n, Fast &f, double *lam, double *sk, float *lh, float *ll, float4 *sm) {
   const bool warm = f.warm;
@@ -1015,12 +1024,12 @@ __device__ bool fast_eigen(Team<CL> &tm, int n, Fast &f, double *lam, double *sk
     const float sc = zf > lim ? lim / zf : 1.0f;
     const float zm = s.m0 * sc;
     if (it == 0 && threadIdx.x == 0) f.z0 = zm;
-    const bool last = !low && zm < kZFinal && s.m1 < 0x1p-26f;
+    const bool last = !low && fmaxf(zf, rf) < kFinal;
     const float em = zm + 0.5f * s.m1;
     const int ke = em > 0x1p-50f ? -exp_above(em) : 50;
     step_update_planes(tm, n, f, sc, ke);
     // a coarse step that no longer shrinks the rotations has met its own rounding
-    // (pairs closer than ~2^-17 of the norm): full steps from here on
+    // (pairs closer than ~2^-20 of the norm): full steps from here on
     if (low && zm < 0x1p-6f && zm > 0.9f * zprev) stalled = true;
     zprev = zm;
     low = !last && !stalled && zm > kZLow;
@@ -1050,7 +1059,7 @@ __device__ __noinline__ void planes_of_tiles(Team<CL> &tm, int n, const Fast &f,
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
-      int k = c + 54;
+      int k = c + kW;
       if constexpr (ROWS) {
         if (i < n && j < n) k += f.xe[i] + f.xe[j];
       }
@@ -1080,14 +1089,14 @@ __device__ __noinline__ void planes_of_tiles(Team<CL> &tm, int n, const Fast &f,
 }
 
 // Exponent s of a scale 2^-s that puts a matrix of Frobenius norm sqrt(sum) to
-// a norm in (1, 2].
+// a norm in (1/2, 1].
 __device__ __forceinline__ int norm_exp(float sum) {
-  return sum > 0x1p-100f ? exp_above(sqrtf(sum) * 1.0001f) - 1 : 0;
+  return sum > 0x1p-100f ? exp_above(sqrtf(sum) * 1.0001f) : 0;
 }
 
 // The Fock matrix F = H0 - S (v_i + v_j) / 2 - (T + T^T) / 2, T_ij = sum_c
 // M_c,ij v_c(atom of j) (conversions.py:255-297), and F' = X F X^T, whose
-// planes, scaled by 2^-s to a Frobenius norm in (1, 2], go to f.Fr. x: the
+// planes, scaled by 2^-s to a Frobenius norm in (1/2, 1], go to f.Fr. x: the
 // potential (orbitals, atomic dipoles, quadrupoles); aoat: shared, atom of
 // each orbital. All in fixed point: the float64 form (14 FMA a value) was
 // bound by the FP64 pipe. False if a potential or norm is out of range.
@@ -1132,13 +1141,13 @@ __device__ __noinline__ bool fast_fock(Team<CL> &tm, int n, Fast &f, const doubl
     for (int t = f.own_tables ? (int)threadIdx.x : tm.tid; t < N; t += f.own_tables ? (int)blockDim.x : tm.nthr) {
       const double v = ld<CL>(x + t);
       if (t < n) {
-        f.vo[t] = fix(v, 53 - E + f.eS);
+        f.vo[t] = fix(v, kFix - E + f.eS);
       } else if (t < n + 3 * nat) {
         const int u = t - n;
-        f.vm[(u % 3) * nat + u / 3] = halves(fix(v, 53 - E + f.eD));
+        f.vm[(u % 3) * nat + u / 3] = halves(fix(v, kFix - E + f.eD));
       } else {
         const int u = t - n - 3 * nat;
-        f.vm[(3 + u % 6) * nat + u / 6] = halves(fix(v, 53 - E + f.eQ));
+        f.vm[(3 + u % 6) * nat + u / 6] = halves(fix(v, kFix - E + f.eQ));
       }
     }
     tm.sync();
@@ -1206,9 +1215,9 @@ __device__ __noinline__ bool fast_fock(Team<CL> &tm, int n, Fast &f, const doubl
           mul_add(a0[e], a1[e], make_int2(y[e].z, y[e].w), ur[kr]);
         }
       }
-      // |a0| < 20 2^50: the sum in units of 2^(E - 58) fits
+      // in units of 2^(E - kFix)
 #pragma unroll
-      for (int e = 0; e < 8; ++e) a0[e] = a0[e] * 256 + (a1[e] >> 20);
+      for (int e = 0; e < 8; ++e) a0[e] += a1[e] >> 29;
     } else {
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
@@ -1216,14 +1225,14 @@ __device__ __noinline__ bool fast_fock(Team<CL> &tm, int n, Fast &f, const doubl
         const int4 x = ld_stream(f.M + (size_t)t * kPairWords + e * 32 + (threadIdx.x & 31), pol);
         long long b0 = 0, b1 = 0;
         mul_add(b0, b1, make_int2(x.x, x.y), halves(f.vo[i] + f.vo[j]));
-        a0[e] = b0 * 256 + (b1 >> 20);
+        a0[e] = b0 + (b1 >> 29);
       }
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
       long long v = 0;
-      if (i < n && j < n) v = fix(H0[(size_t)i * n + j], 58 - E) - ((a0[e] + 1) >> 1);
+      if (i < n && j < n) v = fix(H0[(size_t)i * n + j], kFix - E) - ((a0[e] + 1) >> 1);
       a0[e] = v;
       const float y = fix_to_float(v);
       sum.s0 = fmaf(ti == tj ? y : 2.0f * y, y, sum.s0);
@@ -1231,33 +1240,33 @@ __device__ __noinline__ bool fast_fock(Team<CL> &tm, int n, Fast &f, const doubl
     put_tile(f.Ft, t, a0);
   }
   const Four q = team_four(tm, sum, sm, f.red);
-  const int sf = norm_exp(q.s0) + E - 2;  // fix_to_float took 2^-56 for 2^(E - 58)
-  planes_of_tiles<false>(tm, n, f, E - 58 - sf);
+  const int sf = norm_exp(q.s0) + E - 2;  // fix_to_float took 2^-56 for 2^(E - kFix)
+  planes_of_tiles<false>(tm, n, f, E - kFix - sf);
   tiles<kDig>(tm, n, f, kHalf, 0, 0, nullptr);
   sum.s0 = tiles<kDig>(tm, n, f, kFockX, 0, 0, nullptr);
   const Four p = team_four(tm, sum, sm, f.red);
   if (!(p.s0 < 0x1p100f)) return false;
   const int sn = norm_exp(p.s0);
-  planes_of_tiles<true>(tm, n, f, -56 - sn);
+  planes_of_tiles<true>(tm, n, f, -kR - sn);
   s = sn + sf;
   return true;
 }
 
 // Populations sum_k P_ki M_c,ki of every orbital i for the 10 (1) matrices,
 // from the density in f.Ft (C w C^T with 0 <= w <= 2): f.pop[c n + i] in units
-// of 2^(eP + eM - 106 + 56 - sh), sh returned. eP: every |P_ii| < 2^eP, hence
+// of 2^(eP + eM - kFix + sh), sh returned. eP: every |P_ii| < 2^eP, hence
 // every |P_ij|: one unit for all of P. (Units by the row norms of X, from which
 // P is built, lose as many bits as these norms exceed P's entries, that is for
 // an ill-conditioned S.) A lower tile serves the
 // sums of its columns with the pairs and of its rows with their mirrors. Exact
-// sums of 53-bit factors: the order of the atomics does not matter.
+// sums of fixed-point factors: the order of the atomics does not matter.
 // In float64 (10 FMA a pair) this was bound by the FP64 pipe; here by the
 // loads, 80 bytes a pair, which the tile order makes contiguous.
 template <bool CL>
 __device__ __noinline__ int fast_populations(Team<CL> &tm, int n, Fast &f, int eP) {
   const int lane = threadIdx.x & 31, nlow = f.nb * (f.nb + 1) / 2;
-  int sh = 12;  // sums over n products of at most 2^50 in units of 2^(56 - sh)
-  while (sh > 0 && ((int64_t)n << sh) > (int64_t(1) << 12)) --sh;
+  int sh = 0;  // sums over n products of at most 2^58
+  while ((16 << sh) < n) ++sh;
   const int nw = f.nm > 1 ? 5 : 1;
   const uint64_t pol = stream_policy();
   for (int t = team_warp(tm); t < nlow; t += team_warps(tm)) {
@@ -1269,7 +1278,7 @@ __device__ __noinline__ int fast_populations(Team<CL> &tm, int n, Fast &f, int e
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int i = min(16 * ti + tile_row(e), n - 1), j = min(16 * tj + tile_col(e), n - 1);
-      q[e] = halves(shift(p[e], f.xte[i] + f.xte[j] + 1 - 56 + 53 - eP));
+      q[e] = halves(shift(p[e], f.xte[i] + f.xte[j] + 1 - kR + kFix - eP));
     }
     const int4 *M = f.M + (size_t)t * kPairWords + lane;
     const int mirror = f.nm > 1 ? 256 : 0;
@@ -1294,7 +1303,7 @@ __device__ __noinline__ int fast_populations(Team<CL> &tm, int n, Fast &f, int e
 #pragma unroll
           for (int k = 0; k < 4; ++k)
 #pragma unroll
-            for (int c = 0; c < 2; ++c) a0[k][c] = 0, a1[k][c] = 1ll << (27 - sh);  // to round
+            for (int c = 0; c < 2; ++c) a0[k][c] = a1[k][c] = 0;
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             // columns: (e >> 2, e & 1); rows: (e >> 1) & 1
@@ -1305,7 +1314,7 @@ __device__ __noinline__ int fast_populations(Team<CL> &tm, int n, Fast &f, int e
 #pragma unroll
           for (int k = 0; k < 4; ++k)
 #pragma unroll
-            for (int c = 0; c < 2; ++c) s[k][c] = (a0[k][c] << sh) + (a1[k][c] >> (28 - sh));
+            for (int c = 0; c < 2; ++c) s[k][c] = (a0[k][c] + (a1[k][c] >> 29) + ((1 << sh) >> 1)) >> sh;
         }
 #pragma unroll
         for (int e = 0; e < 8; ++e) x[e] = xn[e];
@@ -1351,7 +1360,7 @@ __device__ __noinline__ void fast_store_density(Team<CL> &tm, int n, const Fast 
     for (int e = 0; e < 8; ++e) {
       const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
       if (i < n && j <= i) {
-        const double v = unfix(p[e], f.xte[i] + f.xte[j] + 1 - 56);
+        const double v = unfix(p[e], f.xte[i] + f.xte[j] + 1 - kR);
         out[(size_t)i * n + j] = v;
         out[(size_t)j * n + i] = v;
       }
@@ -1360,7 +1369,7 @@ __device__ __noinline__ void fast_store_density(Team<CL> &tm, int n, const Fast 
   tm.sync();
 }
 
-// One block of planes back as integers of weight 2^-54.
+// One block of planes back as integers of weight 2^-kW.
 __device__ __forceinline__ void join_block(const uint4 *blk, long long (&r)[8]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -1372,15 +1381,15 @@ __device__ __forceinline__ void join_block(const uint4 *blk, long long (&r)[8]) 
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
       const __half2 x = *reinterpret_cast<const __half2 *>(&u[h]);
-      r[2 * h] = r[2 * h] * 512 + __half2int_rn(__low2half(x));
-      r[2 * h + 1] = r[2 * h + 1] * 512 + __half2int_rn(__high2half(x));
+      r[2 * h] = r[2 * h] * 1024 + __half2int_rn(__low2half(x));
+      r[2 * h + 1] = r[2 * h + 1] * 1024 + __half2int_rn(__high2half(x));
     }
   }
 }
 
 // C diag(w) C^T over the mo lowest orbitals from the planes of C^T in f.Gl;
 // w(j): weight of orbital j, |w| <= 2^sw. To out (both triangles), or without
-// it to f.Ft in units of 2^(xte_i + xte_j + sw - 56); the returned eP bounds
+// it to f.Ft in units of 2^(xte_i + xte_j + sw - kR); the returned eP bounds
 // this P, every |P_ii| < 2^eP.
 template <bool CL, typename W>
 __device__ __noinline__ int fast_density(Team<CL> &tm, int n, Fast &f, int mo, int sw, W w, double *out,
@@ -1419,7 +1428,7 @@ __device__ __noinline__ void fast_orbitals(Team<CL> &tm, int n, const Fast &f, i
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int i = 16 * ti + tile_row(e), j = 16 * tj + tile_col(e);
-      if (i < n && j < mo) C[(size_t)j * n + i] = unfix(r[e], ldi<CL>(f.xte + i) - 54);
+      if (i < n && j < mo) C[(size_t)j * n + i] = unfix(r[e], ldi<CL>(f.xte + i) - kW);
     }
   }
 }

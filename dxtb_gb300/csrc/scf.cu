@@ -820,7 +820,7 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
       tiles<kDig>(tm, n, f, kCoeff, mo, 0, nullptr);
       const int eP = fast_density(tm, n, f, mo, 1, [&](int j) { return fa[j] + fb[j]; }, (double *)nullptr, sfour);
       // ---- Mulliken charges and atomic multipoles (conversions.py:203-251) ----
-      const int u = eP - 50 - fast_populations(tm, n, f, eP);
+      const int u = eP - kFix + fast_populations(tm, n, f, eP);
       // orbital o's sum with matrix c counts 2^(u + exponent of the matrix)
       auto pop = [&](int c, int o) {
         return unfix(__ldcg(f.pop + (size_t)c * n + o), u + (c == 0 ? f.eS : c < 4 ? f.eD : f.eQ));
