@@ -32,10 +32,11 @@ import torch
 from . import _lib, build
 
 DEFAULT = (112, 136, 160, 320, 640)
-# thresholds of classes 1..5 (one-SM CTA, clusters of 2, 4, 8, 16)
+# thresholds of classes 1..5 (one-SM CTA, clusters of 2, 4, 8, 16); the default
+# stands for the rule by the molecule's share of the batch (dxtb_scf_team_sizes)
 CANDIDATES = [
     DEFAULT,
-    (96, 136, 160, 320, 640),
+    (80, 136, 160, 320, 640),
     (80, 112, 140, 320, 640),
     (96, 136, 180, 240, 320),
     (112, 160, 220, 260, 320),

@@ -1125,6 +1125,7 @@ using namespace dxtb;
 
 extern "C" int64_t dxtb_scf_workspace_mol(int64_t n, int64_t nat) { return ws_size_mol(n, nat); }
 
+#include <cmath>
 #include <mutex>
 
 namespace dxtb {
@@ -1133,14 +1134,14 @@ namespace dxtb {
 static std::mutex g_policy_mutex;
 static constexpr int kDefaultThr[kClasses] = {0, 112, 136, 160, 320, 640};
 static int g_thr[kClasses] = {0, 112, 136, 160, 320, 640};
-// One or two molecules leave most SMs idle: under the default policy they take
-// larger teams. Energy + forces of one GFN2 molecule, ms, by team (256 threads,
-// 512, clusters of 4, 8, 16): n = 33 7.9 7.4 8.7 8.9 9.6; 49 12.6 10.4 10.9
-// 11.2 11.9; 72 16.1 12.9 11.9 12.2 13.0; 106 33.4 25.3 17.1 16.1 16.8; 150 -
-// 65 29.6 25.5 24.1; 233 - - 60.9 41.0 35.3. From nine molecules on clusters
-// of 16 no longer run at once; two keep within a quarter of the SMs, which
-// leaves callers with several such batches in flight (a serving loop) theirs.
+// Where a larger team stops being faster for a molecule alone. SCF of one GFN2
+// molecule, ms, by team (256 threads, 512, clusters of 2, 4, 8, 16): n = 33 6.4
+// 6.1 7.5 7.5 7.8 8.5; 49 10.5 8.5 9.3 9.1 9.4 10.2; 72 13.8 10.7 10.7 10.0 10.3
+// 11.2; 106 31.3 22.3 16.6 14.0 13.2 14.1; 150 94 62 38 25.7 21.6 20.6; 233 -
+// 164 91 53.6 33.8 28.0; 326 - 562 297 158 94 58.7.
 static constexpr int kFewThr[kClasses] = {0, 30, 60, 60, 90, 130};
+// Batches of this size take these teams also where only the number of
+// molecules is known (dxtb_scf, dxtb_scf_gradient).
 constexpr int kFewMolecules = 2;
 
 // Side streams and fork/join events per (device, caller stream), created once
@@ -1258,8 +1259,12 @@ static int32_t class_gradient(const ScfArgs &a, const GradArgs *g, int c, cudaSt
                          a.vqp, a.S, a.D, g->dedcn, g->grad, f, s);
 }
 
-static int32_t launch_scf(ScfArgs a, int nmol, cudaStream_t st, const GradArgs *g = nullptr) {
-  {
+// min_n: thresholds of classes 1..5 for this call, or null: the process-wide ones.
+static int32_t launch_scf(ScfArgs a, int nmol, cudaStream_t st, const int32_t *min_n, const GradArgs *g) {
+  if (min_n != nullptr) {
+    a.thr[0] = 0;
+    for (int c = 1; c < kClasses; ++c) a.thr[c] = min_n[c - 1];
+  } else {
     std::lock_guard<std::mutex> lock(g_policy_mutex);
     bool preset = nmol <= kFewMolecules;
     for (int c = 0; c < kClasses; ++c) {
@@ -1376,12 +1381,54 @@ extern "C" int32_t dxtb_scf_get_size_classes(int32_t *min_n) {
   return DXTB_OK;
 }
 
-extern "C" int32_t dxtb_scf_set_size_classes(const int32_t *min_n) {
-  if (!min_n) return DXTB_ERR_ARGS;
+static bool valid_classes(const int32_t *min_n) {
   for (int c = 1; c < kClasses; ++c)
-    if (min_n[c - 1] < 1 || (c > 1 && min_n[c - 1] < min_n[c - 2])) return DXTB_ERR_ARGS;
+    if (min_n[c - 1] < 1 || (c > 1 && min_n[c - 1] < min_n[c - 2])) return false;
+  return true;
+}
+
+extern "C" int32_t dxtb_scf_set_size_classes(const int32_t *min_n) {
+  if (!min_n || !valid_classes(min_n)) return DXTB_ERR_ARGS;
   std::lock_guard<std::mutex> lock(g_policy_mutex);
   for (int c = 1; c < kClasses; ++c) g_thr[c] = min_n[c - 1];
+  return DXTB_OK;
+}
+
+// Teams by the molecule's share of the batch: the SCF's time on one SM grows
+// about with n^3 over the sizes that matter, so a molecule whose share
+// s(n) = SMs n^3 / sum n^3 is at least r SMs takes the class of r, unless
+// kFewThr says that so large a team is slower. Fixed thresholds leave either
+// SMs idle (small batches) or every molecule on a team whose barriers cost more
+// than its size gains (large ones). Energy and forces of GFN2 batches, ms, fixed
+// {112, 136, 160, 320, 640} -> this rule: 10-60 atoms 8 molecules 47.1 -> 23.3,
+// 37 53.5 -> 25.0, 100 60.3 -> 45.7, 256 90.3 -> 84.1; 30-120 atoms 6 105 -> 52,
+// 24 147 -> 99, 64 188 -> 164. r of half or twice these, and n^2.5, are within
+// 10 % at most sizes and slower by up to 40 % at some.
+// Class 0 ends at n = 136 whatever the share: there two molecules on one SM take
+// as long as one after the other on 512 threads (58 SM ms each).
+extern "C" int32_t dxtb_scf_team_sizes(const int32_t *n, int32_t nmol, int32_t lanes, int32_t *min_n) {
+  if (!n || nmol <= 0 || lanes <= 0 || !min_n) return DXTB_ERR_ARGS;
+  bool preset = true;
+  {
+    std::lock_guard<std::mutex> lock(g_policy_mutex);
+    for (int c = 1; c < kClasses; ++c) {
+      min_n[c - 1] = g_thr[c];
+      preset = preset && g_thr[c] == kDefaultThr[c];
+    }
+  }
+  if (!preset) return DXTB_OK;
+  int sms = 0;
+  if (device_sms(&sms) != DXTB_OK) return DXTB_ERR_LAUNCH;
+  constexpr double share[kClasses] = {0.0, 0.5, 1.5, 3.0, 6.0, 12.0};
+  double work = 0.0;
+  for (int m = 0; m < nmol; ++m) work += (double)n[m] * n[m] * n[m];
+  work *= (double)lanes / sms;
+  for (int c = 1; c < kClasses; ++c) {
+    const double x = std::ceil(std::cbrt(share[c] * work));
+    int v = max(kFewThr[c], x < 1e9 ? (int)x : 1000000000);
+    if (c == 1) v = min(v, 136);
+    min_n[c - 1] = v;
+  }
   return DXTB_OK;
 }
 
@@ -1411,7 +1458,8 @@ static int32_t apply_config(const dxtb_scf_config *c, ScfArgs &a) {
 
 }  // namespace dxtb
 
-// dxtb_scf; fast: the workspace holds ws_size_mol (else ws_size_base) doubles a molecule.
+// dxtb_scf (g: and the gradient); fast: the workspace holds ws_size_mol (else
+// ws_size_base) doubles a molecule; min_n as in launch_scf.
 static int32_t scf_call(const dxtb_batch *b, const double *par_f, const int32_t *par_i,
                         const double *overlap, const double *h0, const double *dipole,
                         const double *quadrupole, const double *gamma, const double *hd,
@@ -1421,11 +1469,13 @@ static int32_t scf_call(const dxtb_batch *b, const double *par_f, const int32_t 
                         double *workspace, double *density, double *wdensity, double *coeff,
                         double *evals, double *occ, double *q, double *dp, double *qp, double *vorb,
                         double *vdp, double *vqp, double *energies, int32_t *status, void *stream,
-                        int fast) {
+                        int fast, const int32_t *min_n = nullptr, const GradArgs *g = nullptr) {
   if (!b || b->nmol <= 0 || !overlap || !h0 || !gamma || !hd || !n0 || !nel || !ws_off ||
       !workspace || !density || !coeff || !evals || !occ || !q || !vorb || !energies || !status)
     return DXTB_ERR_ARGS;
+  if (g != nullptr && (!wdensity || !g->cn || !g->dedcn || !g->grad)) return DXTB_ERR_ARGS;
   if (!(kt > 0.0)) return DXTB_ERR_ARGS;
+  if (g != nullptr && dipole != nullptr && (!vdp || !vqp || !dp || !qp || !g->mrad)) return DXTB_ERR_ARGS;
   ScfArgs a;
   if (apply_config(cfg, a) != DXTB_OK) return DXTB_ERR_ARGS;
   a.b = *b;
@@ -1461,7 +1511,7 @@ static int32_t scf_call(const dxtb_batch *b, const double *par_f, const int32_t 
   a.energies = energies;
   a.status = status;
   a.fast = fast;
-  return launch_scf(a, b->nmol, (cudaStream_t)stream);
+  return launch_scf(a, b->nmol, (cudaStream_t)stream, min_n, g);
 }
 
 extern "C" int32_t dxtb_scf(const dxtb_batch *b, const double *par_f, const int32_t *par_i,
@@ -1488,49 +1538,27 @@ extern "C" int32_t dxtb_scf_gradient(
     double *wdensity, double *coeff, double *evals, double *occ, double *q, double *dp, double *qp,
     double *vorb, double *vdp, double *vqp, double *energies, int32_t *status, const double *cn,
     const double *mrad, double *dedcn, double *grad, void *stream) {
-  if (!b || b->nmol <= 0 || !overlap || !h0 || !gamma || !hd || !n0 || !nel || !ws_off ||
-      !workspace || !density || !wdensity || !coeff || !evals || !occ || !q || !vorb || !energies ||
-      !status || !cn || !dedcn || !grad)
-    return DXTB_ERR_ARGS;
-  if (!(kt > 0.0)) return DXTB_ERR_ARGS;
-  if (dipole != nullptr && (!vdp || !vqp || !dp || !qp || !mrad)) return DXTB_ERR_ARGS;
-  ScfArgs a;
-  if (apply_config(cfg, a) != DXTB_OK) return DXTB_ERR_ARGS;
-  a.b = *b;
-  a.pf = par_f;
-  a.pi = par_i;
-  a.S = overlap;
-  a.H0 = h0;
-  a.D = dipole;
-  a.Q = quadrupole;
-  a.gamma = gamma;
-  a.hd = hd;
-  a.sd = amat_sd;
-  a.dd = amat_dd;
-  a.sq = amat_sq;
-  a.gb = gb_mat;
-  a.n0 = n0;
-  a.nel = nel;
-  a.kt = kt;
-  a.ws_off = ws_off;
-  a.order = order;
-  a.ws = workspace;
-  a.P = density;
-  a.W = wdensity;
-  a.C = coeff;
-  a.evals = evals;
-  a.occ = occ;
-  a.q = q;
-  a.dp = dp;
-  a.qp = qp;
-  a.vorb = vorb;
-  a.vdp = vdp;
-  a.vqp = vqp;
-  a.energies = energies;
-  a.status = status;
-  a.fast = 1;
-  GradArgs g{cn, mrad, dedcn, grad};
-  return launch_scf(a, b->nmol, (cudaStream_t)stream, &g);
+  const GradArgs g{cn, mrad, dedcn, grad};
+  return scf_call(b, par_f, par_i, overlap, h0, dipole, quadrupole, gamma, hd, amat_sd, amat_dd,
+                  amat_sq, gb_mat, n0, nel, kt, cfg, ws_off, order, workspace, density, wdensity,
+                  coeff, evals, occ, q, dp, qp, vorb, vdp, vqp, energies, status, stream, 1, nullptr, &g);
+}
+
+extern "C" int32_t dxtb_scf_teams(
+    const dxtb_batch *b, const double *par_f, const int32_t *par_i, const double *overlap,
+    const double *h0, const double *dipole, const double *quadrupole, const double *gamma,
+    const double *hd, const double *amat_sd, const double *amat_dd, const double *amat_sq,
+    const double *gb_mat, const double *n0, const double *nel, double kt, const dxtb_scf_config *cfg,
+    const int64_t *ws_off, const int32_t *order, double *workspace, double *density,
+    double *wdensity, double *coeff, double *evals, double *occ, double *q, double *dp, double *qp,
+    double *vorb, double *vdp, double *vqp, double *energies, int32_t *status, const double *cn,
+    const double *mrad, double *dedcn, double *grad,
+    const int32_t *min_n, void *stream) {
+  if (!min_n || !valid_classes(min_n)) return DXTB_ERR_ARGS;
+  const GradArgs g{cn, mrad, dedcn, grad};
+  return scf_call(b, par_f, par_i, overlap, h0, dipole, quadrupole, gamma, hd, amat_sd, amat_dd,
+                  amat_sq, gb_mat, n0, nel, kt, cfg, ws_off, order, workspace, density, wdensity,
+                  coeff, evals, occ, q, dp, qp, vorb, vdp, vqp, energies, status, stream, 1, min_n, grad != nullptr ? &g : nullptr);
 }
 
 // ---------------------------------------------------------------------------

@@ -139,6 +139,8 @@ class PackedBatch:
             "par_i": dev(tables.i32, torch.int32),
         }
         self.numbers = nums
+        self.lanes = 1  # batches of about this size in flight at once (they share the SMs)
+        self._nao32 = np.ascontiguousarray(nao, dtype=np.int32)
         self.set_positions(positions)
 
     def set_positions(self, positions: list) -> None:
@@ -204,14 +206,10 @@ def _seg_sum(values: torch.Tensor, seg: torch.Tensor, nmol: int) -> torch.Tensor
 GB_KERNELS = {"p16": 0, "still": 1}
 
 
-def scf_launches(L, nmax: int, nmol: int = 0) -> int:
-    """Kernels launched by dxtb_scf for a batch (of nmol molecules) whose
-    largest has nmax orbitals: one per cluster class up to the largest one
-    present, the one-SM launch, the shared-SM launch."""
-    thr = (C.c_int32 * 5)()
-    _lib.check(L.dxtb_scf_get_size_classes(thr), "size classes")
-    if 0 < nmol <= 2 and tuple(thr) == (112, 136, 160, 320, 640):
-        thr = (30, 60, 60, 90, 130)  # the library's teams for one or two molecules
+def scf_launches(thr, nmax: int) -> int:
+    """SCF kernels launched for a batch whose largest molecule has nmax
+    orbitals under the size classes thr: one per cluster class up to the
+    largest one present, the one-SM launch, the shared-SM launch."""
     cmax = sum(1 for t in thr if nmax >= t)
     return 1 + (1 if cmax >= 1 else 0) + max(0, cmax - 1)
 
@@ -360,7 +358,9 @@ def run(pb: PackedBatch, *, etemp: float = 300.0, maxiter: int = 250, tol: float
                 _lib.ptr(W), Cm.data_ptr(), ev.data_ptr(), occ.data_ptr(), q.data_ptr(),
                 dp.data_ptr(), qp.data_ptr(), vorb.data_ptr(), vdp.data_ptr(), vqp.data_ptr(),
                 en.data_ptr(), status.data_ptr())
-    n_scf = scf_launches(L, int(pb.nao.max()), pb.nmol)
+    thr = (C.c_int32 * 5)()
+    _lib.check(L.dxtb_scf_team_sizes(pb._nao32.ctypes.data, pb.nmol, pb.lanes, thr), "size classes")
+    n_scf = scf_launches(thr, pb.struct.max_nao)
     grad = None
     if forces:
         # SCF and gradient fused per size class: each class's forces overlap
@@ -370,13 +370,13 @@ def run(pb: PackedBatch, *, etemp: float = 300.0, maxiter: int = 250, tol: float
         dedcn = buf("dedcn", na)
         dedcn.zero_()
         mark("scf", 0)
-        _lib.check(L.dxtb_scf_gradient(*scf_args, cn.data_ptr(), _lib.ptr(mrad), dedcn.data_ptr(),
-                                       grad.data_ptr(), st), "SCF and gradient")
+        _lib.check(L.dxtb_scf_teams(*scf_args, cn.data_ptr(), _lib.ptr(mrad), dedcn.data_ptr(),
+                                    grad.data_ptr(), thr, st), "SCF and gradient")
         launches += 3 * n_scf  # per class: SCF, pair adjoint, per-molecule terms
         mark("scf", 1)
     else:
         mark("scf", 0)
-        _lib.check(L.dxtb_scf(*scf_args, st), "SCF")
+        _lib.check(L.dxtb_scf_teams(*scf_args, None, None, None, None, thr, st), "SCF")
         launches += n_scf
         mark("scf", 1)
     if forces:

@@ -487,6 +487,7 @@ class CudaExecutor:
             pb = PackedBatch(self.tables[method], [r.numbers for r in reqs], [r.positions for r in reqs],
                              device=self.device, charges=[r.chrg for r in reqs],
                              spins=[r.spin for r in reqs])
+            pb.lanes = len(self.streams)
             forces = any(r.forces for r in reqs)
             res = run(pb, forces=forces, state=self.state[slot], **self.opts)
             nm = pb.nmol

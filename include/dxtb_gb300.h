@@ -305,8 +305,8 @@ int32_t dxtb_scf(const dxtb_batch *b, const double *par_f, const int32_t *par_i,
  * 8 or 16 CTAs on as many SMs (classes 2-5) that share every O(n^3) phase.
  * min_n[c-1] is the smallest n of class c (non-decreasing); the default is
  * {112, 136, 160, 320, 640}, under which a batch of one or two molecules
- * takes larger teams ({30, 60, 60, 90, 130}); any other setting holds for
- * every batch. Clusters need the launch order of dxtb_scf;
+ * takes larger teams ({30, 60, 60, 90, 130}) and dxtb_scf_team_sizes fits the
+ * teams to the batch; any other setting holds for every batch. Clusters need the launch order of dxtb_scf;
  * cluster sizes the GPU cannot place fold into the largest one it can.
  * Each class runs on a stream of its own, forked from the caller's stream:
  * larger classes get higher stream priorities, unless the caller's stream
@@ -314,6 +314,13 @@ int32_t dxtb_scf(const dxtb_batch *b, const double *par_f, const int32_t *par_i,
 int32_t dxtb_scf_set_size_classes(const int32_t *min_n);
 /* The current thresholds (min_n [5]). */
 int32_t dxtb_scf_get_size_classes(int32_t *min_n);
+
+/* Thresholds min_n [5] for a batch of nmol molecules with n (host array)
+ * orbitals each, of which about `lanes` run at once on the GPU (1: alone):
+ * teams in proportion to each molecule's share of the work. Under
+ * thresholds other than the default it returns those. */
+int32_t dxtb_scf_team_sizes(const int32_t *n, int32_t nmol, int32_t lanes,
+                            int32_t *min_n);
 
 /* dxtb_scf followed by dxtb_gradient, fused per size class: the gradient of
  * a class's molecules is launched on that class's stream right after its
@@ -337,6 +344,25 @@ int32_t dxtb_scf_gradient(const dxtb_batch *b, const double *par_f,
                           double *vqp, double *energies, int32_t *status,
                           const double *cn, const double *mrad, double *dedcn,
                           double *grad, void *stream);
+
+/* dxtb_scf_gradient, or with grad NULL (then cn, mrad and dedcn too) dxtb_scf,
+ * with this call's own thresholds min_n [5] (host) in place of the
+ * process-wide ones. */
+int32_t dxtb_scf_teams(const dxtb_batch *b, const double *par_f,
+                       const int32_t *par_i, const double *overlap,
+                       const double *h0, const double *dipole,
+                       const double *quadrupole, const double *gamma,
+                       const double *hd, const double *amat_sd,
+                       const double *amat_dd, const double *amat_sq,
+                       const double *gb_mat, const double *n0,
+                       const double *nel, double kt, const dxtb_scf_config *cfg,
+                       const int64_t *ws_off, const int32_t *order,
+                       double *workspace, double *density, double *wdensity,
+                       double *coeff, double *evals, double *occ, double *q,
+                       double *dp, double *qp, double *vorb, double *vdp,
+                       double *vqp, double *energies, int32_t *status,
+                       const double *cn, const double *mrad, double *dedcn,
+                       double *grad, const int32_t *min_n, void *stream);
 
 /* Nuclear gradient dE/dR [natoms][3] at the converged SCF (analytic
  * adjoint; the reference differentiates with autograd through

@@ -130,3 +130,44 @@ def test_without_room_for_the_planes():
     assert (out["P"] - s["P"][:nm]).abs().max().item() <= 1e-8
     assert (out["W"] - s["W"][:nm]).abs().max().item() <= 1e-8
     assert (out["ev"] - s["evals"][:n]).abs().max().item() <= 1e-8
+
+
+@pytest.mark.parametrize("lanes", [1, 40])
+def test_teams_by_share_match_one_cta(lanes):
+    """Both sides of every size where the team changes (for a lone batch and
+    for one that shares the SMs) against one CTA per molecule. Residuals of
+    1e-10 enter energies squared and forces times a response of about 10."""
+    from dxtb_gb300 import _lib
+    from dxtb_gb300.calculators import tables
+    from dxtb_gb300.engine import PackedBatch, run, scf_launches
+
+    L = _lib.lib()
+    mols = [_molecule(n) for n in (9, 29, 30, 59, 60, 89, 90, 129, 130, 136)]
+    pb = PackedBatch(tables("gfn2"), [m[0] for m in mols], [torch.tensor(m[1]) for m in mols])
+    pb.lanes = lanes
+    thr = (C.c_int32 * 5)()
+    assert L.dxtb_scf_team_sizes(pb._nao32.ctypes.data, pb.nmol, lanes, thr) == 0
+    got = tuple(thr)
+    assert list(got) == sorted(got) and got[0] <= 136
+    if lanes == 1:  # few molecules: the largest teams that pay
+        assert got[0] <= 32 and got[1:] == (60, 60, 90, 130) and scf_launches(got, 136) == 6
+    else:
+        assert got[1] > 60
+    r = run(pb, forces=True, tol=1e-10)
+    assert (r.status.cpu() == 0).all()
+    e, g = r.energy.cpu().clone(), r.gradient.cpu().clone()
+    saved = (C.c_int32 * 5)()
+    assert L.dxtb_scf_get_size_classes(saved) == 0
+    try:
+        assert L.dxtb_scf_set_size_classes((C.c_int32 * 5)(*range(1000, 1005))) == 0
+        assert L.dxtb_scf_team_sizes(pb._nao32.ctypes.data, pb.nmol, lanes, thr) == 0
+        assert tuple(thr) == (1000, 1001, 1002, 1003, 1004)  # a set policy holds
+        ref = run(pb, forces=True, tol=1e-10)
+    finally:
+        assert L.dxtb_scf_set_size_classes(saved) == 0
+    assert (ref.energy.cpu() - e).abs().max() <= 1e-10
+    assert (ref.gradient.cpu() - g).abs().max() <= 1e-8
+    bad = (C.c_int32 * 5)(3, 2, 4, 5, 6)
+    assert L.dxtb_scf_team_sizes(None, pb.nmol, lanes, thr) != 0
+    assert L.dxtb_scf_team_sizes(pb._nao32.ctypes.data, pb.nmol, 0, thr) != 0
+    assert L.dxtb_scf_teams(*[None] * 15, 0.0, *[None] * 21, bad, None) != 0
