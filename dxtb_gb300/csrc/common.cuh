@@ -137,6 +137,14 @@ __device__ __forceinline__ int find_mol(const int64_t *off, int nmol, int64_t k)
   return lo;
 }
 
+// Row and column (i >= j) of element t of a lower triangle.
+__device__ __forceinline__ void lower_pair(int64_t t, int &i, int &j) {
+  i = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+  while ((int64_t)(i + 1) * (i + 2) / 2 <= t) ++i;
+  while ((int64_t)i * (i + 1) / 2 > t) --i;
+  j = (int)(t - (int64_t)i * (i + 1) / 2);
+}
+
 // Nuclear-gradient kernels of the molecules selected by a filter (gradient.cu).
 int32_t launch_gradient(const dxtb_batch *b, const double *par_f, const int32_t *par_i,
                         const double *cn, const double *mrad, const double *density,

@@ -391,7 +391,7 @@ def run(pb: PackedBatch, *, etemp: float = 300.0, maxiter: int = 250, tol: float
         mark("scf", 0)
         _lib.check(L.dxtb_scf_teams(*scf_args, cn.data_ptr(), _lib.ptr(mrad), dedcn.data_ptr(),
                                     grad.data_ptr(), thr, st), "SCF and gradient")
-        launches += 3 * n_scf  # per class: SCF, pair adjoint, per-molecule terms
+        launches += 4 * n_scf  # per class: SCF, pairs with d shells, other terms, CN chain rule
         mark("scf", 1)
     else:
         mark("scf", 0)
