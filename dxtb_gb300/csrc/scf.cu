@@ -27,9 +27,10 @@ constexpr int kLuSlots = 1024;       // concurrent inverse-iteration factorisati
 // size classes (kClasses, common.cuh): 0 small, 1 one SM, 2..5 clusters of 2..16
 constexpr int kMaxCluster = 16;
 constexpr int kTinyN = 12;           // largest order of the float64 path by choice
-// dynamic shared memory: 32 n bytes, plus the rows of the Householder
-// reduction where they fit (one-SM and cluster teams), next to ~10 KB of
-// static arrays, within the 227 KB of a CTA
+// dynamic shared memory: 32 n bytes, plus the tables of the potential, or
+// without room for the digit planes (dxtb_scf_noalloc) the rows of the
+// Householder reduction where they fit (one-SM and cluster teams), next to
+// ~10 KB of static arrays, within the 227 KB of a CTA
 constexpr int kMaxDynSmem = 208 * 1024;
 
 struct MolView {
@@ -680,9 +681,8 @@ __device__ __noinline__ int anderson_step(const ScfArgs &a, Team<CL> &tm, Ws &w,
 }
 
 // The SCF of molecule m_ by the team tm. dsm: dynamic shared memory of
-// 3 n doubles + 2 n floats (n of this molecule or larger), then room for
-// the rows of the Householder reduction (`rows`: false for teams that
-// share an SM, which keep the rows in the L1).
+// 3 n doubles + 2 n floats (n of this molecule or larger), then the tables of
+// the potential or (`rows`) room for the rows of the Householder reduction.
 template <bool CL>
 __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bool rows) {
   __shared__ double red[32];
@@ -1095,7 +1095,7 @@ __global__ void __launch_bounds__(NT, MINB) k_scf(const __grid_constant__ ScfArg
   tm.tid = threadIdx.x;
   tm.stid = threadIdx.x;
   tm.nthr = blockDim.x;
-  scf_body<false>(a, m, tm, dsm, false);
+  scf_body<false>(a, m, tm, dsm, NT == kScfBigThreads && !a.fast);
 }
 
 // One thread-block cluster per molecule of size class `cls` (2..5); the
@@ -1115,7 +1115,7 @@ __global__ void __launch_bounds__(kScfBigThreads, 1) k_scf_cluster(const __grid_
   for (int i = 0; i < a.b.nmol; ++i) {
     const int m = a.order ? a.order[i] : i;
     if (scf_class(a.thr, (int)(a.b.ao_off[m + 1] - a.b.ao_off[m])) != cls) continue;
-    if (cnt++ % nq == q) scf_body<true>(a, m, tm, dsm, false);
+    if (cnt++ % nq == q) scf_body<true>(a, m, tm, dsm, !a.fast);
   }
 }
 
@@ -1309,11 +1309,19 @@ static int32_t launch_scf(ScfArgs a, int nmol, cudaStream_t st, const int32_t *m
                                     kMaxDynSmem) == cudaSuccess;
       }) != DXTB_OK)
     return DXTB_ERR_LAUNCH;
-  // shared memory of every class: the base. The L1 serves the digit planes.
-  // shared memory of class c: 4 n doubles and, while that leaves most of the
-  // L1, the tables of the potential (n + 9 nat)
+  // shared memory of class c: 4 n doubles and, while that leaves most of the L1
+  // to the digit planes, the tables of the potential (n + 9 nat). Without the
+  // planes every iteration reduces the matrix to a band: then its rows, if 60 %
+  // of them or more fit (fewer gained nothing at n ~ 900-1000).
   auto class_smem = [&](int c) -> size_t {
     const size_t nub = c + 1 < kClasses ? (size_t)min(nmax, a.thr[c + 1]) : (size_t)nmax;
+    if (!a.fast && c >= 1) {
+      const size_t csize = c >= 2 ? (size_t)1 << (c - 1) : 1, own = (nub + csize - 1) / csize, more = c >= 2 ? 1 : 0;
+      const size_t full = 32 * nub + (own + more) * nub * 8;
+      if (full <= (size_t)kMaxDynSmem) return full;
+      const int64_t fit = ((int64_t)kMaxDynSmem / 8 - 4 * (int64_t)nub) / (int64_t)nub - (int64_t)more;
+      return 10 * fit >= 6 * (int64_t)own ? (size_t)kMaxDynSmem : 32 * nub;
+    }
     const size_t tables = 8 * nub + 72 * (size_t)a.b.max_nat;
     return 32 * nub + (32 * nub + tables <= 64 * 1024 ? tables : 0);
   };
