@@ -95,11 +95,45 @@ __device__ double team_sum(Team<CL> &tm, double v, double *red) {
       ++tm.phase;
       if (threadIdx.x == 0) slot[tm.rank] = s;
       tm.sync();
-      s = 0.0;
-      for (int c = 0; c < tm.size; ++c) s += __ldcg(slot + c);
+      // one warp: as every thread's own sum it took 19 cycles of the FP64 pipe
+      // a warp and CTA
+      if (threadIdx.x < 32) {
+        s = warp_sum(threadIdx.x < tm.size ? __ldcg(slot + threadIdx.x) : 0.0);
+        if (threadIdx.x == 0) red[0] = s;
+      }
+      __syncthreads();
+      s = red[0];
+      __syncthreads();
     }
   }
   return s;
+}
+
+// Three sums at once. sm: shared [3 x 33]; slots: global [2][16][3].
+template <bool CL>
+__device__ void team_sum3(Team<CL> &tm, double (&v)[3], double *sm, double *slots) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) v[c] = warp_sum(v[c]);
+  if (lane == 0)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sm[3 * wid + c] = v[c];
+  __syncthreads();
+  double s = 0.0;
+  if (wid < 3) s = warp_sum(lane < nw ? sm[3 * lane + wid] : 0.0);
+  if constexpr (CL) {
+    if (tm.size > 1) {
+      double *slot = slots + 48 * (tm.phase & 1);
+      ++tm.phase;
+      if (wid < 3 && lane == 0) slot[3 * tm.rank + wid] = s;
+      tm.sync();
+      if (wid < 3) s = warp_sum(lane < tm.size ? __ldcg(slot + 3 * lane + wid) : 0.0);
+    }
+  }
+  if (wid < 3 && lane == 0) sm[96 + wid] = s;
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < 3; ++c) v[c] = sm[96 + c];
 }
 
 // Maximum of non-negative values over the team (a NaN is dropped).

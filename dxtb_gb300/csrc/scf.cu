@@ -418,29 +418,19 @@ enum ScfAction : int { kNext = 0, kStop = 1 };
 // stop when |dx|_2 < x_tol and |F|_2 < f_tol. The whole team: an element of
 // the vectors is always the same thread's, a history vector's dot products a
 // warp's. The history is read once for the three products of each vector
-// (with dx, dy and F), once for the update and the step.
+// (with dx, dy and F), once for the update and the step. Bound by the FP64 pipe
+// (six multiply-adds a history element) and by the reductions' barriers: the
+// norms are summed together. (Gm F = Gm dy - dx_prev would need four, but its
+// rounding errors add up: a molecule of 89 steps no longer reached 1e-10.)
 template <bool CL>
 __device__ __noinline__ int broyden_step(const ScfArgs &a, Team<CL> &tm, Ws &w, int N, int it, Broyden &br,
                                          int &status, double *red) {
-  double *sdot = w.sdot;          // [kRank] c_k . dx
-  double *sdot2 = sdot + kRank;   // [kRank] d_k . dy
-  double *sdot3 = sdot2 + kRank;  // [kRank] d_k . F
+  __shared__ double s3[99];
+  double *sdot = w.sdot;           // [kRank] c_k . dx
+  double *sdot2 = sdot + kRank;    // [kRank] d_k . dy
+  double *sdot3 = sdot2 + kRank;   // [kRank] d_k . F
+  double *slots = sdot3 + kRank;   // [2][16][3] partial sums
   const int lane = threadIdx.x & 31;
-  // |F|^2 with F = x - G(x)
-  double part = 0.0;
-  for (int t = tm.tid; t < N; t += tm.nthr) {
-    const double y = w.x[t] - ld<CL>(w.g + t);
-    part += y * y;
-  }
-  const double ynorm = sqrt(team_sum(tm, part, red));
-  br.resid = ynorm;
-  if (it == 1) {
-    if (ynorm <= a.ftol * kEps) return kStop;
-    br.nrank = 0;
-  } else if (ynorm < br.best_ynorm) {
-    br.best_ynorm = ynorm;
-    for (int t = tm.tid; t < N; t += tm.nthr) w.xbest[t] = w.x[t];
-  }
   if (br.nrank >= kRank) br.nrank = 0;  // "restart" reduction of a full memory (not reached: kRank >= maxiter)
   const int nrank = br.nrank;
   // dx = x - x_prev and dy = F - F_prev into the x_prev / F_prev slots
@@ -479,9 +469,9 @@ __device__ __noinline__ int broyden_step(const ScfArgs &a, Team<CL> &tm, Ws &w, 
     tm.sync();
   }
   // Broyden update: v = Gm^T dx, c = dx - Gm dy, d = v / (dy . v); beside it
-  // g = Gm F of the old memory (in the new F_prev slot)
+  // Gm F of the old memory (in the new F_prev slot)
   double *cn = w.hx + (size_t)nrank * N, *dn = w.hr + (size_t)nrank * N;
-  double pdv = 0.0, pfv = 0.0;
+  double sum[3] = {0.0, 0.0, 0.0};  // F . F, dy . v, F . v
   for (int t = tm.tid; t < N; t += tm.nthr) {
     const double y = w.x[t] - ld<CL>(w.g + t);
     double step = 0.5 * y;
@@ -496,21 +486,30 @@ __device__ __noinline__ int broyden_step(const ScfArgs &a, Team<CL> &tm, Ws &w, 
       }
       cn[t] = dxt - gdy;
       dn[t] = v;
-      pdv = fma(dyt, v, pdv);
-      pfv = fma(y, v, pfv);
+      sum[1] = fma(dyt, v, sum[1]);
+      sum[2] = fma(y, v, sum[2]);
     }
+    sum[0] = fma(y, y, sum[0]);
     w.rold[t] = step;
+  }
+  team_sum3(tm, sum, s3, slots);
+  const double ynorm = sqrt(sum[0]);
+  br.resid = ynorm;
+  if (it == 1) {
+    if (ynorm <= a.ftol * kEps) return kStop;
+  } else if (ynorm < br.best_ynorm) {
+    br.best_ynorm = ynorm;
+    for (int t = tm.tid; t < N; t += tm.nthr) w.xbest[t] = w.x[t];
   }
   double fd = 0.0;  // d . F of the new vector
   if (it > 1) {
-    const double dyv = team_sum(tm, pdv, red);
-    const double fv = team_sum(tm, pfv, red);
+    const double dyv = sum[1];
     if (dyv == 0.0 || !isfinite(dyv)) {
       status = DXTB_ERR_NAN;
       return kStop;
     }
     const double idyv = 1.0 / dyv;
-    fd = fv * idyv;
+    fd = sum[2] * idyv;
     for (int t = tm.tid; t < N; t += tm.nthr) dn[t] *= idyv;
     ++br.nrank;
     if (br.dx_norm < a.xtol && ynorm < a.ftol) return kStop;  // converged at x
