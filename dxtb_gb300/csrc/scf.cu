@@ -1412,7 +1412,15 @@ extern "C" int32_t dxtb_scf_set_size_classes(const int32_t *min_n) {
 // 24 147 -> 99, 64 188 -> 164. r of half or twice these, and n^2.5, are within
 // 10 % at most sizes and slower by up to 40 % at some.
 // Class 0 ends at n = 136 whatever the share: there two molecules on one SM take
-// as long as one after the other on 512 threads (58 SM ms each).
+// as long as one after the other on 512 threads (58 SM ms each). The other
+// classes start at kShareTop at the latest: there the next larger team costs at
+// most a quarter more SM time, and a molecule on one SM would keep all others
+// of its batch waiting (n = 326: 562 ms on one SM, 59 ms on 16). Batches that
+// share the SMs keep the fixed thresholds as the latest: with the share alone
+// packs of molecules of 500 to 930 orbitals ran on one SM each, 118 s instead of
+// 13 s for the slowest of 200 requests of 8-300 atoms.
+static constexpr int kShareTop[kClasses] = {0, 136, 200, 260, 400, 640};
+
 extern "C" int32_t dxtb_scf_team_sizes(const int32_t *n, int32_t nmol, int32_t lanes, int32_t *min_n) {
   if (!n || nmol <= 0 || lanes <= 0 || !min_n) return DXTB_ERR_ARGS;
   bool preset = true;
@@ -1432,9 +1440,8 @@ extern "C" int32_t dxtb_scf_team_sizes(const int32_t *n, int32_t nmol, int32_t l
   work *= (double)lanes / sms;
   for (int c = 1; c < kClasses; ++c) {
     const double x = std::ceil(std::cbrt(share[c] * work));
-    int v = max(kFewThr[c], x < 1e9 ? (int)x : 1000000000);
-    if (c == 1) v = min(v, 136);
-    min_n[c - 1] = v;
+    const int top = lanes > 1 ? kDefaultThr[c] : kShareTop[c];
+    min_n[c - 1] = max(kFewThr[c], x < top ? (int)x : top);
   }
   return DXTB_OK;
 }
