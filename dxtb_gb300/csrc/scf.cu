@@ -27,6 +27,7 @@ constexpr int kLuSlots = 1024;       // concurrent inverse-iteration factorisati
 // size classes (kClasses, common.cuh): 0 small, 1 one SM, 2..5 clusters of 2..16
 constexpr int kMaxCluster = 16;
 constexpr int kTinyN = 12;           // largest order of the float64 path by choice
+constexpr int kLooseN = 32;          // the same under Anderson mixing
 // dynamic shared memory: 32 n bytes, plus the tables of the potential, or
 // without room for the digit planes (dxtb_scf_noalloc) the rows of the
 // Householder reduction where they fit (one-SM and cluster teams), next to
@@ -101,7 +102,12 @@ __device__ inline Ws ws_carve(double *base, int n, int nat) {
 // eps is sorted ascending; eh, el: eps as float32 pairs. Orbitals beyond 45 kT
 // from mu (by float32) have f = 0 or 1 to 3e-20 and are counted in integers:
 // only the window around mu, empty for most molecules, takes float64 (a warp
-// issues one float64 instruction per ~64 cycles). Returns false on failure.
+// issues one float64 instruction per ~64 cycles). IN_ORDER: inside the window
+// the electrons are summed with the full orbitals, in their order, the sum that
+// float64 gives without a window (the float64 path: where the gap is below kT
+// and the SCF ends on 1e-4, its last bit shows in the forces by 1e-7); else
+// apart from them, which rounds less. Returns false on failure.
+template <bool IN_ORDER>
 __device__ bool fermi_warp(int n, const double *eps, const float *eh, const float *el, double nel, double kt,
                            double *f) {
   const int lane = threadIdx.x & 31;
@@ -142,6 +148,7 @@ __device__ bool fermi_warp(int n, const double *eps, const float *eh, const floa
         ++full;
         v = 1.0;
       } else if (!(x > 45.0f)) {
+        if (IN_ORDER && !window) s = (double)full;  // the lane's full orbitals come first
         window = true;
         v = occ((eps[j] - mu) * ikt);
         s += v;
@@ -149,12 +156,11 @@ __device__ bool fermi_warp(int n, const double *eps, const float *eh, const floa
       }
       if (write) f[j] = v;
     }
-    full = __reduce_add_sync(0xffffffffu, full);
-    if (__any_sync(0xffffffffu, window)) {
-      s = warp_sum(s);
-      ds = warp_sum(ds) * ikt;
-    }
-    return s + ((double)full - nel);
+    const int all = __reduce_add_sync(0xffffffffu, full);
+    if (!__any_sync(0xffffffffu, window)) return (double)all - nel;
+    ds = warp_sum(ds) * ikt;
+    if constexpr (IN_ORDER) return warp_sum(window ? s : (double)full) - nel;
+    return warp_sum(s) + ((double)all - nel);
   };
   double ds;
   for (int it = 0; it < 200; ++it) {
@@ -750,12 +756,19 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
   // The products and the eigenproblem run on digit planes; where a norm is not
   // finite or the vectors do not settle the float64 path takes an iteration,
   // after three such iterations, or without the workspace for the planes, all.
-  // Up to kTinyN orbitals (less than a block) float64 stays: as quick at 6
-  // (1.87 ms against 1.92 for water), 5.9 ms against ~3.9 at 12, but SCFs of so
-  // few degrees of freedom on the default 1e-4 end where the rounding takes
-  // them (a 3-atom molecule's Anderson system is singular to working
-  // precision: 1e-16 in its charges moves its forces by 1e-6).
-  bool fast = a.fast != 0 && status == DXTB_OK && n > kTinyN;
+  // Up to kTinyN orbitals (less than a block) float64 stays: as quick at 6 (1.87
+  // ms against 1.92 for water), 5.9 ms against ~3.9 at 12. Anderson mixing keeps
+  // it up to kLooseN, bit for bit as without the planes (one CTA, potential and
+  // Fermi sum in their order): SCFs of few degrees of freedom and a small gap
+  // take 30 to 57 steps to its 1e-4, their mixing systems become singular to
+  // working precision, and the last bit of any product then shows in the
+  // forces. Largest change of a molecule's forces (norm, Eh/Bohr) between the
+  // two paths, 64 geometries of each of 618 molecules: n = 13-32 3e-7, 33-49
+  // 8e-11, 50-63 1e-7 (one molecule; 2e-10 without it); float64 against itself
+  // with the last bit of the positions changed moves as far. 256 molecules of
+  // 3-9 atoms take 11.3 ms here, 7.4 ms on the planes.
+  const bool small = n <= (a.mixer == DXTB_MIXER_ANDERSON ? kLooseN : kTinyN);
+  bool fast = a.fast != 0 && status == DXTB_OK && !small;
   if (fast) {
     fast = fast_setup(tm, n, w.Linv, f, sfour) &&
            fast_integrals(tm, n, f, S, H0, multipole ? a.D + mv.moff : nullptr,
@@ -796,8 +809,8 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
       fb = se;
       __shared__ int s_ok, s_mo;
       if (threadIdx.x < 32) {
-        bool ok = fermi_warp(n, sw, df, e2f, nel_a, a.kt, fa);
-        if (nel_b != nel_a) ok = ok && fermi_warp(n, sw, df, e2f, nel_b, a.kt, fb);
+        bool ok = fermi_warp<false>(n, sw, df, e2f, nel_a, a.kt, fa);
+        if (nel_b != nel_a) ok = ok && fermi_warp<false>(n, sw, df, e2f, nel_b, a.kt, fb);
         int first = n;  // orbitals with non-vanishing occupation (decreasing with j)
         for (int j = threadIdx.x; j < n; j += 32) {
           if (nel_b == nel_a) fb[j] = fa[j];
@@ -918,11 +931,11 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
       __syncthreads();
       // ---- Fermi occupations (filling.py:428-742), both spin channels ----
       if (tm.lead() && threadIdx.x < 32) {
-        bool ok = fermi_warp(n, sw, df, e2f, nel_a, a.kt, w.fa);
+        bool ok = fermi_warp<true>(n, sw, df, e2f, nel_a, a.kt, w.fa);
         if (nel_b == nel_a) {
           for (int j = threadIdx.x; j < n; j += 32) w.fb[j] = w.fa[j];
         } else {
-          ok = ok && fermi_warp(n, sw, df, e2f, nel_b, a.kt, w.fb);
+          ok = ok && fermi_warp<true>(n, sw, df, e2f, nel_b, a.kt, w.fb);
         }
         __syncwarp();
         if (threadIdx.x == 0) {
@@ -1000,7 +1013,7 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
       tm.sync();
     }
     // ---- new potential G(x) and the root-solver step ----
-    if (!CL && nat <= kFewAtoms)
+    if (!CL && (nat <= kFewAtoms || small))
       potential_few_atoms(a, mv, qsh, qat, dpa, qpa, vsh, vat, w.g, multipole, es3_shell);
     else
       potential_from_charges(a, mv, tm, qsh, qat, dpa, qpa, vsh, vat, w.lu, lu_size(n), w.g, multipole, es3_shell);
@@ -1258,6 +1271,13 @@ static int32_t class_gradient(const ScfArgs &a, const GradArgs *g, int c, cudaSt
                          a.vqp, a.S, a.D, g->dedcn, g->grad, f, s);
 }
 
+static bool default_policy() {
+  std::lock_guard<std::mutex> lock(g_policy_mutex);
+  for (int c = 1; c < kClasses; ++c)
+    if (g_thr[c] != kDefaultThr[c]) return false;
+  return true;
+}
+
 // min_n: thresholds of classes 1..5 for this call, or null: the process-wide ones.
 static int32_t launch_scf(ScfArgs a, int nmol, cudaStream_t st, const int32_t *min_n, const GradArgs *g) {
   if (min_n != nullptr) {
@@ -1273,6 +1293,9 @@ static int32_t launch_scf(ScfArgs a, int nmol, cudaStream_t st, const int32_t *m
     if (preset)
       for (int c = 0; c < kClasses; ++c) a.thr[c] = min(a.thr[c], kFewThr[c]);
   }
+  // the float64 path of a loose SCF (scf_body) on the team whose bits it keeps
+  if (a.mixer == DXTB_MIXER_ANDERSON && default_policy())
+    for (int c = 1; c < kClasses; ++c) a.thr[c] = max(a.thr[c], kLooseN + 1);
   int sms = 0;
   if (device_sms(&sms) != DXTB_OK) return DXTB_ERR_LAUNCH;
   const int nmax = a.b.max_nao;
