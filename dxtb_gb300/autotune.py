@@ -4,14 +4,16 @@ classes (``dxtb_scf_set_size_classes``), i.e. which molecules run as one CTA
 of 256 threads two per SM, one CTA of 512 threads per SM, or a thread-block
 cluster of 2, 4, 8 or 16 CTAs.
 
-``tune(pb)`` times the packed batch ``pb`` (energy + forces, CUDA events on
-the current stream, the median of ``reps`` runs after one warm-up) under each
-candidate threshold set, keeps the fastest, applies it process-wide and
-caches it on disk, keyed by the GPU (name, SM count), the library build and
-a signature of the batch's size distribution. ``ensure(pb)`` applies a
-cached choice or tunes once per process and device. Setting
-``DXTB_AUTOTUNE=0`` keeps the library's defaults. The choice changes only
-the team each molecule runs on, so results agree to rounding.
+``ensure(pb)`` gives the packed batch ``pb`` its thresholds (``pb.classes``):
+a choice cached for this GPU and batch shape, or one tuned once per process and
+device. No other batch sees them. ``tune(pb)`` is the explicit call: it times
+the batch (energy + forces, CUDA events on the current stream, the median of
+``reps`` runs after one warm-up) under each candidate threshold set, sets the
+fastest for the whole process (``set_classes``) and caches it on disk, keyed by
+the GPU (name, SM count), the library build and a signature of the batch's size
+distribution. While such a process-wide set is in force ``ensure`` leaves it.
+Setting ``DXTB_AUTOTUNE=0`` keeps the library's defaults. The choice changes
+only the team each molecule runs on, so results agree to rounding.
 
 The reference has no counterpart: its batched SCF is a padded tensor
 program whose shapes PyTorch dispatches.
@@ -92,51 +94,73 @@ def _time(pb, state: dict, reps: int) -> float:
     return float(np.median(times))
 
 
-def tune(pb, candidates=None, reps: int = 3, save: bool = True) -> dict:
-    """Times every candidate on ``pb``, applies and returns the fastest:
-    {"thresholds": [...], "ms": {candidate: median ms}, "source": "tuned"}."""
-    cands = [tuple(c) for c in (candidates or CANDIDATES)]
+def _measure(pb, candidates, reps: int) -> dict:
+    """Times every candidate on ``pb`` and returns the choice; ``pb`` and the
+    process keep their thresholds. Only to be called under the default set."""
     state: dict = {}
     ms = {}
-    for c in cands:
-        set_classes(c)
-        ms[c] = _time(pb, state, reps)
+    before = pb.classes
+    try:
+        for c in candidates:
+            pb.classes = None if c == DEFAULT else c
+            ms[c] = _time(pb, state, reps)
+    finally:
+        pb.classes = before
     best = min(ms, key=ms.get)
-    # a set policy holds for every later batch of the process, where the rule
-    # fits each: it gives way for 5 % or more (256 molecules of 10-60 atoms: 72.5
-    # against 74.5 ms, but then 64 larger ones 178 against 149 ms)
+    # the rule gives way for 5 % or more: runs of one candidate differ by up to 3 %
     if DEFAULT in ms and ms[best] > 0.95 * ms[DEFAULT]:
         best = DEFAULT
-    set_classes(best)
-    out = {"thresholds": list(best), "ms": {",".join(map(str, c)): v for c, v in ms.items()},
-           "source": "tuned", "when": time.strftime("%Y-%m-%dT%H:%M:%S")}
+    return {"thresholds": list(best), "ms": {",".join(map(str, c)): v for c, v in ms.items()},
+            "source": "tuned", "when": time.strftime("%Y-%m-%dT%H:%M:%S")}
+
+
+def _save(pb, out: dict) -> None:
+    path = cache_path()
+    try:
+        path.parent.mkdir(parents=True, exist_ok=True)
+        data = json.loads(path.read_text()) if path.exists() else {}
+        data.setdefault(_device_key(pb.device), {})[_batch_key(pb)] = out
+        path.write_text(json.dumps(data, indent=1))
+    except OSError:
+        pass  # a read-only cache location only costs a re-tune
+
+
+def tune(pb, candidates=None, reps: int = 3, save: bool = True) -> dict:
+    """Times every candidate on ``pb``, applies the fastest process-wide and
+    returns it: {"thresholds": [...], "ms": {candidate: median ms}, "source":
+    "tuned"}."""
+    before = get_classes()
+    set_classes(DEFAULT)
+    try:
+        out = _measure(pb, [tuple(c) for c in (candidates or CANDIDATES)], reps)
+    except BaseException:
+        set_classes(before)
+        raise
+    set_classes(out["thresholds"])
     if save:
-        path = cache_path()
-        try:
-            path.parent.mkdir(parents=True, exist_ok=True)
-            data = json.loads(path.read_text()) if path.exists() else {}
-            data.setdefault(_device_key(pb.device), {})[_batch_key(pb)] = out
-            path.write_text(json.dumps(data, indent=1))
-        except OSError:
-            pass  # a read-only cache location only costs a re-tune
+        _save(pb, out)
     return out
 
 
 def ensure(pb, min_molecules: int = 32) -> dict:
-    """Applies the cached policy for this GPU and batch shape, tuning once if
-    none is cached. Batches below ``min_molecules`` keep the current policy."""
+    """Gives ``pb`` the cached thresholds for this GPU and batch shape, tuning
+    once if none are cached. Batches below ``min_molecules``, and all while a
+    set other than the default is in force for the process, keep theirs."""
+    now = get_classes()
     if os.environ.get("DXTB_AUTOTUNE", "1") == "0" or pb.nmol < min_molecules:
-        return {"thresholds": list(get_classes()), "source": "default"}
+        return {"thresholds": list(now), "source": "default"}
+    if now != DEFAULT:
+        return {"thresholds": list(now), "source": "set"}
     dkey, bkey = _device_key(pb.device), _batch_key(pb)
-    if (dkey, bkey) in _applied:
-        set_classes(_applied[(dkey, bkey)]["thresholds"])
-        return _applied[(dkey, bkey)]
-    try:
-        data = json.loads(cache_path().read_text())
-        hit = data[dkey][bkey]
-        set_classes(hit["thresholds"])
-        res = dict(hit, source="cache")
-    except (OSError, KeyError, ValueError):
-        res = tune(pb)
-    _applied[(dkey, bkey)] = res
+    res = _applied.get((dkey, bkey))
+    if res is None:
+        try:
+            hit = json.loads(cache_path().read_text())[dkey][bkey]
+            res = dict(hit, source="cache", thresholds=[int(v) for v in hit["thresholds"]])
+        except (OSError, KeyError, TypeError, ValueError):
+            res = _measure(pb, CANDIDATES, 3)
+            _save(pb, res)
+        _applied[(dkey, bkey)] = res
+    thr = tuple(res["thresholds"])
+    pb.classes = None if thr == DEFAULT else thr
     return res

@@ -159,6 +159,7 @@ class PackedBatch:
         self.t = _upload(host, device)
         self.numbers = nums
         self.lanes = 1  # batches of about this size in flight at once (they share the SMs)
+        self.classes = None  # thresholds of the size classes 1..5 (None: dxtb_scf_team_sizes)
         self._nao32 = np.ascontiguousarray(nao, dtype=np.int32)
         self.set_positions(positions)
 
@@ -223,6 +224,14 @@ def _seg_sum(values: torch.Tensor, seg: torch.Tensor, nmol: int) -> torch.Tensor
 
 
 GB_KERNELS = {"p16": 0, "still": 1}
+
+
+def team_sizes(nao: np.ndarray, lanes: int = 1):
+    """Thresholds of the size classes 1..5 for molecules of nao (int32,
+    contiguous) orbitals, ``lanes`` such batches in flight at once."""
+    thr = (C.c_int32 * 5)()
+    _lib.check(_lib.lib().dxtb_scf_team_sizes(nao.ctypes.data, len(nao), lanes, thr), "size classes")
+    return thr
 
 
 def scf_launches(thr, nmax: int) -> int:
@@ -377,8 +386,7 @@ def run(pb: PackedBatch, *, etemp: float = 300.0, maxiter: int = 250, tol: float
                 _lib.ptr(W), Cm.data_ptr(), ev.data_ptr(), occ.data_ptr(), q.data_ptr(),
                 dp.data_ptr(), qp.data_ptr(), vorb.data_ptr(), vdp.data_ptr(), vqp.data_ptr(),
                 en.data_ptr(), status.data_ptr())
-    thr = (C.c_int32 * 5)()
-    _lib.check(L.dxtb_scf_team_sizes(pb._nao32.ctypes.data, pb.nmol, pb.lanes, thr), "size classes")
+    thr = team_sizes(pb._nao32, pb.lanes) if pb.classes is None else (C.c_int32 * 5)(*pb.classes)
     n_scf = scf_launches(thr, pb.struct.max_nao)
     grad = None
     if forces:
