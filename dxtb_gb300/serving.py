@@ -10,10 +10,11 @@ pack is one packed batch pushed through the device pipeline (geometry ->
 integrals -> persistent SCF -> adjoint gradient) on its slot's stream. Its
 basis, integral and density state stays device-resident until the host
 has its results. Packs on different streams run concurrently: a pack's
-SCF kernel holds one SM (or half of one) per molecule, so the other
-packs' molecules run on the SMs left free. Each molecule's SCF runs in
-its own CTA with a fixed reduction order, so a result does not depend on
-the pack it was admitted in.
+SCF kernel holds half an SM to 16 SMs per molecule, by its share of the pack
+(``dxtb_scf_team_sizes`` with the number of slots), so the other packs'
+molecules run on the SMs left free. Within a team the reduction order is
+fixed; teams of other sizes round differently, so a result depends on the
+pack it was admitted in by rounding alone.
 
 The reference has no serving loop: it evaluates one ``Calculator`` call
 at a time (``calculators/types/energy.py:78-414``). This module adds
@@ -103,8 +104,8 @@ class Server:
     requests would otherwise wait for the largest molecule admitted with
     them. Small requests may use an idle large slot while no large request
     is queued. ``large_sms`` caps the SMs that in-flight large packs hold
-    (``executor.team_sms(req)`` per molecule) while small requests are queued
-    or in flight: the SCF kernels are persistent and keep their SMs until the
+    (``executor.pack_sms(reqs)`` of each pack, or without it the sum of
+    ``executor.team_sms(req)``) while small requests are queued or in flight: the SCF kernels are persistent and keep their SMs until the
     molecule converges, so without a cap the large molecules' clusters can
     occupy every SM for seconds while small requests wait; once no small
     request is left, the large lane may use every SM. With ``order="size"`` each lane admits its smallest request
@@ -188,6 +189,12 @@ class Server:
             t = self.ex.team_sms(req) if hasattr(self.ex, "team_sms") else 1
             self._teams[id(req)] = t
         return t
+
+    def _pack_sms(self, reqs: list) -> int:
+        """SMs of a pack's SCF teams, counted against ``large_sms``."""
+        if len(reqs) > 1 and hasattr(self.ex, "pack_sms"):
+            return self.ex.pack_sms(reqs)  # a molecule's team shrinks with its share of the pack
+        return sum(self._team_sms(r) for r in reqs)
 
     def lane(self, req: Request) -> str:
         if self.large_slots > 0 and self._size(req) >= self.large_n:
@@ -292,11 +299,11 @@ class Server:
                             and (order != "size" or self._size(r) <= 2 * nhead)
                             and (order != "longest" or 2 * self._size(r) >= nhead)):
                         b = nb if r is head else self.ex.nbytes(r)
-                        t = self._team_sms(r) if capped else 0
-                        if tot + b <= free and (not capped or sms + t <= sms_free):
+                        t = self._pack_sms(take + [r]) if capped else 0
+                        if tot + b <= free and (not capped or t <= sms_free):
                             take.append(r)
                             tot += b
-                            sms += t
+                            sms = t
                             continue
                     rest.append(r)
                 self.queues[lane] = rest
@@ -449,19 +456,19 @@ class CudaExecutor:
         """Orbitals of the request's molecule."""
         return self._sizes(req)[0]
 
+    def pack_sms(self, reqs: list) -> int:
+        """SMs that the SCF of a pack of these requests holds while it runs, by
+        the thresholds that its launch will take: one for each molecule of the
+        one-CTA size classes, the cluster size (2-16) for the others."""
+        from .engine import team_sizes
+
+        n = np.array([self.norb(r) for r in reqs], dtype=np.int32)
+        c = np.searchsorted(np.array(team_sizes(n, len(self.streams))), n, side="right")  # class 0..5
+        return int(np.where(c <= 1, 1, 1 << np.maximum(c - 1, 0)).sum())
+
     def team_sms(self, req: Request) -> int:
-        """SMs the request's SCF holds while it runs: 1 for the one-CTA size
-        classes, the cluster size (2-16) for the others (the size-class
-        policy of the library)."""
-        import ctypes as C
-
-        from . import _lib
-
-        thr = (C.c_int32 * 5)()
-        _lib.check(_lib.lib().dxtb_scf_get_size_classes(thr), "size classes")
-        n = self.norb(req)
-        c = sum(1 for t in thr if n >= t)  # size class 0..5
-        return 1 if c <= 1 else 1 << (c - 1)
+        """``pack_sms`` of the request in a pack of its own."""
+        return self.pack_sms([req])
 
     def nbytes(self, req: Request) -> int:
         """Device bytes of one request's state (integrals, caches, SCF workspace, outputs)."""
