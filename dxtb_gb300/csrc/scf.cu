@@ -53,9 +53,9 @@ __host__ __device__ inline int64_t ws_size_base(int64_t n, int64_t nat) {
   return 3 * n * n + 10 * n + (2 * kRank + 7) * N + 64 + 16 * nat + lu_size(n) + n + 8 +
          4 * kRank + 64 + 64;
 }
-// with the digit planes of the tensor-core path (eigemm.cuh), where it is taken
-__host__ __device__ inline int64_t ws_size_mol(int64_t n, int64_t nat, bool multipole) {
-  return ws_size_base(n, nat) + (n > kTinyN ? fast_size(n, nat, multipole) : 0);
+// with the digit planes of the tensor-core path (eigemm.cuh)
+__host__ __device__ inline int64_t ws_size_mol(int64_t n, int64_t nat) {
+  return ws_size_base(n, nat) + fast_size(n, nat);
 }
 
 struct Ws {
@@ -108,7 +108,7 @@ __device__ inline Ws ws_carve(double *base, int n, int nat) {
 // and the SCF ends on 1e-4, its last bit shows in the forces by 1e-7); else
 // apart from them, which rounds less. Returns false on failure.
 template <bool IN_ORDER>
-__device__ __noinline__ bool fermi_warp(int n, const double *eps, const float *eh, const float *el, double nel, double kt,
+__device__ bool fermi_warp(int n, const double *eps, const float *eh, const float *el, double nel, double kt,
                            double *f) {
   const int lane = threadIdx.x & 31;
   if (nel <= 0.0) {
@@ -197,21 +197,6 @@ struct ScfArgs {
   int thr[kClasses];  // smallest n of each size class (thr[0] = 0)
   int fast;           // the workspace has room for the digit planes
 };
-
-// SCFs that keep the float64 path: up to kTinyN orbitals (less than a block), as
-// quick at 6 (1.87 ms against 1.92 for water), 5.9 ms against ~3.9 at
-// 12. Anderson mixing keeps it up to kLooseN, bit for bit as without the planes
-// (one CTA, potential and Fermi sum in their order): SCFs of few degrees of
-// freedom and a small gap take 30 to 57 steps to its 1e-4, their mixing systems
-// become singular to working precision, and the last bit of any product then
-// shows in the forces. Largest change of a molecule's forces (norm, Eh/Bohr)
-// between the two paths, 64 geometries of each of 618 molecules: n = 13-32
-// 3e-7, 33-49 8e-11, 50-63 1e-7 (one molecule; 2e-10 without it); float64
-// against itself with the last bit of the positions changed moves as far. 256
-// molecules of 3-9 atoms take 11.3 ms here, 7.4 ms on the planes.
-__device__ __forceinline__ bool small_scf(const ScfArgs &a, int n) {
-  return n <= (a.mixer == DXTB_MIXER_ANDERSON ? kLooseN : kTinyN);
-}
 
 // Potential x = (vorb [n], vdp [nat][3], vqp [nat][6]) from the shell and atom
 // charges and the atomic multipoles (interactions/base.py:135-181). The team's
@@ -732,7 +717,7 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
     mv.nsh = (int)(b.shell_off[m + 1] - mv.s0);
     mv.N = mv.n + (multipole ? 9 * mv.nat : 0);
     w = ws_carve(a.ws + a.ws_off[m], mv.n, mv.nat);
-    if (a.fast && mv.n > kTinyN) {
+    if (a.fast) {
       f = fast_carve(a.ws + a.ws_off[m] + ws_size_base(mv.n, mv.nat), mv.n, mv.nat, multipole);
       uint32_t dyn;
       asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
@@ -771,7 +756,19 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
   // The products and the eigenproblem run on digit planes; where a norm is not
   // finite or the vectors do not settle the float64 path takes an iteration,
   // after three such iterations, or without the workspace for the planes, all.
-  bool fast = a.fast != 0 && status == DXTB_OK && !small_scf(a, n);
+  // Up to kTinyN orbitals (less than a block) float64 stays: as quick at 6 (1.87
+  // ms against 1.92 for water), 5.9 ms against ~3.9 at 12. Anderson mixing keeps
+  // it up to kLooseN, bit for bit as without the planes (one CTA, potential and
+  // Fermi sum in their order): SCFs of few degrees of freedom and a small gap
+  // take 30 to 57 steps to its 1e-4, their mixing systems become singular to
+  // working precision, and the last bit of any product then shows in the
+  // forces. Largest change of a molecule's forces (norm, Eh/Bohr) between the
+  // two paths, 64 geometries of each of 618 molecules: n = 13-32 3e-7, 33-49
+  // 8e-11, 50-63 1e-7 (one molecule; 2e-10 without it); float64 against itself
+  // with the last bit of the positions changed moves as far. 256 molecules of
+  // 3-9 atoms take 11.3 ms here, 7.4 ms on the planes.
+  const bool small = n <= (a.mixer == DXTB_MIXER_ANDERSON ? kLooseN : kTinyN);
+  bool fast = a.fast != 0 && status == DXTB_OK && !small;
   if (fast) {
     fast = fast_setup(tm, n, w.Linv, f, sfour) &&
            fast_integrals(tm, n, f, S, H0, multipole ? a.D + mv.moff : nullptr,
@@ -1016,7 +1013,7 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
       tm.sync();
     }
     // ---- new potential G(x) and the root-solver step ----
-    if (!CL && (nat <= kFewAtoms || small_scf(a, n)))
+    if (!CL && (nat <= kFewAtoms || small))
       potential_few_atoms(a, mv, qsh, qat, dpa, qpa, vsh, vat, w.g, multipole, es3_shell);
     else
       potential_from_charges(a, mv, tm, qsh, qat, dpa, qpa, vsh, vat, w.lu, lu_size(n), w.g, multipole, es3_shell);
@@ -1138,11 +1135,7 @@ __global__ void __launch_bounds__(kScfBigThreads, 1) k_scf_cluster(const __grid_
 
 using namespace dxtb;
 
-extern "C" int64_t dxtb_scf_workspace_mol(int64_t n, int64_t nat) { return ws_size_mol(n, nat, true); }
-
-extern "C" int64_t dxtb_scf_workspace_size(int64_t n, int64_t nat, int32_t multipole, int32_t planes) {
-  return planes ? ws_size_mol(n, nat, multipole != 0) : ws_size_base(n, nat);
-}
+extern "C" int64_t dxtb_scf_workspace_mol(int64_t n, int64_t nat) { return ws_size_mol(n, nat); }
 
 #include <cmath>
 #include <mutex>
@@ -1598,31 +1591,11 @@ extern "C" int32_t dxtb_scf_teams(
     double *vorb, double *vdp, double *vqp, double *energies, int32_t *status, const double *cn,
     const double *mrad, double *dedcn, double *grad,
     const int32_t *min_n, void *stream) {
-  if (!min_n) return DXTB_ERR_ARGS;
-  dxtb_scf_plan plan = {};
-  for (int c = 0; c < kClasses - 1; ++c) plan.min_n[c] = min_n[c];
-  plan.planes = 1;
-  return dxtb_scf_planned(b, par_f, par_i, overlap, h0, dipole, quadrupole, gamma, hd, amat_sd, amat_dd,
-                          amat_sq, gb_mat, n0, nel, kt, cfg, ws_off, order, workspace, density, wdensity,
-                          coeff, evals, occ, q, dp, qp, vorb, vdp, vqp, energies, status, cn, mrad, dedcn,
-                          grad, &plan, stream);
-}
-
-extern "C" int32_t dxtb_scf_planned(
-    const dxtb_batch *b, const double *par_f, const int32_t *par_i, const double *overlap,
-    const double *h0, const double *dipole, const double *quadrupole, const double *gamma,
-    const double *hd, const double *amat_sd, const double *amat_dd, const double *amat_sq,
-    const double *gb_mat, const double *n0, const double *nel, double kt, const dxtb_scf_config *cfg,
-    const int64_t *ws_off, const int32_t *order, double *workspace, double *density,
-    double *wdensity, double *coeff, double *evals, double *occ, double *q, double *dp, double *qp,
-    double *vorb, double *vdp, double *vqp, double *energies, int32_t *status, const double *cn,
-    const double *mrad, double *dedcn, double *grad, const dxtb_scf_plan *plan, void *stream) {
-  if (!plan || !valid_classes(plan->min_n)) return DXTB_ERR_ARGS;
+  if (!min_n || !valid_classes(min_n)) return DXTB_ERR_ARGS;
   const GradArgs g{cn, mrad, dedcn, grad};
   return scf_call(b, par_f, par_i, overlap, h0, dipole, quadrupole, gamma, hd, amat_sd, amat_dd,
                   amat_sq, gb_mat, n0, nel, kt, cfg, ws_off, order, workspace, density, wdensity,
-                  coeff, evals, occ, q, dp, qp, vorb, vdp, vqp, energies, status, stream,
-                  plan->planes ? 1 : 0, plan->min_n, grad != nullptr ? &g : nullptr);
+                  coeff, evals, occ, q, dp, qp, vorb, vdp, vqp, energies, status, stream, 1, min_n, grad != nullptr ? &g : nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -1663,7 +1636,7 @@ __global__ void k_noalloc_layout(dxtb_batch b, int64_t *hdr, int64_t ws_start) {
       hdr[kNoallocHeader + m] = off;
       const int64_t n = b.ao_off[m + 1] - b.ao_off[m];
       const int64_t nat = b.atom_off[m + 1] - b.atom_off[m];
-      off += fast ? ws_size_mol(n, nat, true) : ws_size_base(n, nat);
+      off += fast ? ws_size_mol(n, nat) : ws_size_base(n, nat);
     }
     hdr[kNoallocHeader + b.nmol] = off;
     return ws_start + off;  // doubles needed from the start of the array
