@@ -108,7 +108,7 @@ __device__ inline Ws ws_carve(double *base, int n, int nat) {
 // and the SCF ends on 1e-4, its last bit shows in the forces by 1e-7); else
 // apart from them, which rounds less. Returns false on failure.
 template <bool IN_ORDER>
-__device__ bool fermi_warp(int n, const double *eps, const float *eh, const float *el, double nel, double kt,
+__device__ __noinline__ bool fermi_warp(int n, const double *eps, const float *eh, const float *el, double nel, double kt,
                            double *f) {
   const int lane = threadIdx.x & 31;
   if (nel <= 0.0) {
@@ -197,6 +197,21 @@ struct ScfArgs {
   int thr[kClasses];  // smallest n of each size class (thr[0] = 0)
   int fast;           // the workspace has room for the digit planes
 };
+
+// SCFs that keep the float64 path: up to kTinyN orbitals (less than a block), as
+// quick at 6 (1.87 ms against 1.92 for water), 5.9 ms against ~3.9 at
+// 12. Anderson mixing keeps it up to kLooseN, bit for bit as without the planes
+// (one CTA, potential and Fermi sum in their order): SCFs of few degrees of
+// freedom and a small gap take 30 to 57 steps to its 1e-4, their mixing systems
+// become singular to working precision, and the last bit of any product then
+// shows in the forces. Largest change of a molecule's forces (norm, Eh/Bohr)
+// between the two paths, 64 geometries of each of 618 molecules: n = 13-32
+// 3e-7, 33-49 8e-11, 50-63 1e-7 (one molecule; 2e-10 without it); float64
+// against itself with the last bit of the positions changed moves as far. 256
+// molecules of 3-9 atoms take 11.3 ms here, 7.4 ms on the planes.
+__device__ __forceinline__ bool small_scf(const ScfArgs &a, int n) {
+  return n <= (a.mixer == DXTB_MIXER_ANDERSON ? kLooseN : kTinyN);
+}
 
 // Potential x = (vorb [n], vdp [nat][3], vqp [nat][6]) from the shell and atom
 // charges and the atomic multipoles (interactions/base.py:135-181). The team's
@@ -756,19 +771,7 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
   // The products and the eigenproblem run on digit planes; where a norm is not
   // finite or the vectors do not settle the float64 path takes an iteration,
   // after three such iterations, or without the workspace for the planes, all.
-  // Up to kTinyN orbitals (less than a block) float64 stays: as quick at 6 (1.87
-  // ms against 1.92 for water), 5.9 ms against ~3.9 at 12. Anderson mixing keeps
-  // it up to kLooseN, bit for bit as without the planes (one CTA, potential and
-  // Fermi sum in their order): SCFs of few degrees of freedom and a small gap
-  // take 30 to 57 steps to its 1e-4, their mixing systems become singular to
-  // working precision, and the last bit of any product then shows in the
-  // forces. Largest change of a molecule's forces (norm, Eh/Bohr) between the
-  // two paths, 64 geometries of each of 618 molecules: n = 13-32 3e-7, 33-49
-  // 8e-11, 50-63 1e-7 (one molecule; 2e-10 without it); float64 against itself
-  // with the last bit of the positions changed moves as far. 256 molecules of
-  // 3-9 atoms take 11.3 ms here, 7.4 ms on the planes.
-  const bool small = n <= (a.mixer == DXTB_MIXER_ANDERSON ? kLooseN : kTinyN);
-  bool fast = a.fast != 0 && status == DXTB_OK && !small;
+  bool fast = a.fast != 0 && status == DXTB_OK && !small_scf(a, n);
   if (fast) {
     fast = fast_setup(tm, n, w.Linv, f, sfour) &&
            fast_integrals(tm, n, f, S, H0, multipole ? a.D + mv.moff : nullptr,
@@ -1013,7 +1016,7 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
       tm.sync();
     }
     // ---- new potential G(x) and the root-solver step ----
-    if (!CL && (nat <= kFewAtoms || small))
+    if (!CL && (nat <= kFewAtoms || small_scf(a, n)))
       potential_few_atoms(a, mv, qsh, qat, dpa, qpa, vsh, vat, w.g, multipole, es3_shell);
     else
       potential_from_charges(a, mv, tm, qsh, qat, dpa, qpa, vsh, vat, w.lu, lu_size(n), w.g, multipole, es3_shell);
