@@ -53,6 +53,12 @@ class ScfConfig(C.Structure):
     ]
 
 
+class ScfPlan(C.Structure):
+    """Mirror of ``dxtb_scf_plan``."""
+
+    _fields_ = [("min_n", i32 * 5), ("planes", i32)]
+
+
 MIXERS = {"broyden1": 0, "anderson": 1}
 
 
@@ -68,6 +74,7 @@ _SIGS = {
     "dxtb_graph_launch": (i32, [vp, vp]),
     "dxtb_graph_destroy": (i32, [vp]),
     "dxtb_scf_workspace_mol": (i64, [i64, i64]),
+    "dxtb_scf_workspace_size": (i64, [i64, i64, i32, i32]),
     "dxtb_scf": (i32, [vp] * 15 + [f64, vp] + [vp] * 17),
     "dxtb_gradient": (i32, [vp] * 22),
     "dxtb_scf_gradient": (i32, [vp] * 15 + [f64, vp] + [vp] * 21),
@@ -77,6 +84,7 @@ _SIGS = {
     "dxtb_scf_get_size_classes": (i32, [vp]),
     "dxtb_scf_team_sizes": (i32, [vp, i32, i32, vp]),
     "dxtb_scf_teams": (i32, [vp] * 15 + [f64, vp] + [vp] * 22),
+    "dxtb_scf_planned": (i32, [vp] * 15 + [f64, vp] + [vp] * 22),
     "dxtb_born_matrix": (i32, [vp, vp, vp, f64, i32, i32, f64, f64, vp, vp, vp, vp]),
     "dxtb_born_gradient": (i32, [vp, vp, vp, f64, i32, i32, f64, f64, vp, vp, vp, vp, vp]),
     "dxtb_fp64_fma_probe": (i32, [i64, i32, i32, vp, vp]),

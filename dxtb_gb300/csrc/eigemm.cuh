@@ -396,14 +396,16 @@ __device__ Four team_four(Team<CL> &tm, Four v, float4 *sm, float4 *g) {
 // 16-byte words of a lower tile's integrals: per lane 8 values (i, j) and
 // their mirrors (j, i), 10 numbers of 8 bytes each
 constexpr int kPairWords = 5 * 2 * 8 * 32;
+constexpr int kOneWords = 8 * 32;  // S alone (without multipoles), pairs only
+__host__ __device__ inline int pair_words(bool multipole) { return multipole ? kPairWords : kOneWords; }
 
 // Workspace of this path (doubles), np = n rounded up to 16.
-__host__ __device__ inline int64_t fast_size(int64_t n, int64_t nat) {
+__host__ __device__ inline int64_t fast_size(int64_t n, int64_t nat, bool multipole) {
   const int64_t nb = blocks16(n), np2 = 256 * nb * nb;
   // planes of six digits are 12 bytes a value (3/2 doubles), of three 3/4;
   // the integrals S, D, Q in fixed point; potential and population tables
   return (5 * 3 * np2) / 2 + (2 * 3 * np2) / 4 + 2 * np2 + 6 * 16 * nb + 64 + 64 +
-         nb * (nb + 1) / 2 * kPairWords * 2 + (n + 9 * nat) + 10 * n + 8;
+         nb * (nb + 1) / 2 * pair_words(multipole) * 2 + (n + 9 * nat) + 10 * n + 8;
 }
 
 // One copy per CTA in shared memory: as a local variable handed to functions
@@ -464,7 +466,7 @@ __device__ inline Fast fast_carve(double *base, int n, int nat, bool multipole) 
   f.inv = (int *)take(4 * 16 * nb);
   q += (16 - ((uintptr_t)q & 15)) & 15;
   f.Ft = f.Vm2;
-  f.M = (int4 *)take(nb * (nb + 1) / 2 * kPairWords * 16);
+  f.M = (int4 *)take(nb * (nb + 1) / 2 * pair_words(multipole) * 16);
   f.vo = (long long *)take(8 * (int64_t)n);
   f.vm = (int2 *)take(8 * 9 * (int64_t)nat);
   f.pop = (long long *)take(8 * 10 * (int64_t)n);
@@ -584,7 +586,7 @@ __device__ __noinline__ bool fast_integrals(Team<CL> &tm, int n, Fast &f, const 
         const int64_t o = y ? (int64_t)j * n + i : (int64_t)i * n + j;
         int2 m[10];
         m[0] = halves(in ? fix(S[o], kFix - f.eS) : 0);
-        int4 *out = f.M + (size_t)t * kPairWords + (y * 8 + e) * 32 + lane;
+        int4 *out = f.M + (size_t)t * pair_words(f.nm > 1) + (y * 8 + e) * 32 + lane;
         if (f.nm > 1) {
           for (int c = 0; c < 3; ++c) m[1 + c] = halves(in ? fix(D[c * mtot + o], kFix - f.eD) : 0);
           for (int c = 0; c < 6; ++c) m[4 + c] = halves(in ? fix(Q[c * mtot + o], kFix - f.eQ) : 0);
@@ -1222,7 +1224,7 @@ __device__ __noinline__ bool fast_fock(Team<CL> &tm, int n, Fast &f, const doubl
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const int i = r[(e >> 1) & 1], j = c[(e >> 2) * 2 + (e & 1)];
-        const int4 x = ld_stream(f.M + (size_t)t * kPairWords + e * 32 + (threadIdx.x & 31), pol);
+        const int4 x = ld_stream(f.M + (size_t)t * kOneWords + e * 32 + (threadIdx.x & 31), pol);
         long long b0 = 0, b1 = 0;
         mul_add(b0, b1, make_int2(x.x, x.y), halves(f.vo[i] + f.vo[j]));
         a0[e] = b0 + (b1 >> 29);
@@ -1280,7 +1282,7 @@ __device__ __noinline__ int fast_populations(Team<CL> &tm, int n, Fast &f, int e
       const int i = min(16 * ti + tile_row(e), n - 1), j = min(16 * tj + tile_col(e), n - 1);
       q[e] = halves(shift(p[e], f.xte[i] + f.xte[j] + 1 - kR + kFix - eP));
     }
-    const int4 *M = f.M + (size_t)t * kPairWords + lane;
+    const int4 *M = f.M + (size_t)t * pair_words(f.nm > 1) + lane;
     const int mirror = f.nm > 1 ? 256 : 0;
     int4 x[8];
 #pragma unroll

@@ -53,9 +53,9 @@ __host__ __device__ inline int64_t ws_size_base(int64_t n, int64_t nat) {
   return 3 * n * n + 10 * n + (2 * kRank + 7) * N + 64 + 16 * nat + lu_size(n) + n + 8 +
          4 * kRank + 64 + 64;
 }
-// with the digit planes of the tensor-core path (eigemm.cuh)
-__host__ __device__ inline int64_t ws_size_mol(int64_t n, int64_t nat) {
-  return ws_size_base(n, nat) + fast_size(n, nat);
+// with the digit planes of the tensor-core path (eigemm.cuh), where it is taken
+__host__ __device__ inline int64_t ws_size_mol(int64_t n, int64_t nat, bool multipole) {
+  return ws_size_base(n, nat) + (n > kTinyN ? fast_size(n, nat, multipole) : 0);
 }
 
 struct Ws {
@@ -732,7 +732,7 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
     mv.nsh = (int)(b.shell_off[m + 1] - mv.s0);
     mv.N = mv.n + (multipole ? 9 * mv.nat : 0);
     w = ws_carve(a.ws + a.ws_off[m], mv.n, mv.nat);
-    if (a.fast) {
+    if (a.fast && mv.n > kTinyN) {
       f = fast_carve(a.ws + a.ws_off[m] + ws_size_base(mv.n, mv.nat), mv.n, mv.nat, multipole);
       uint32_t dyn;
       asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
@@ -1138,7 +1138,11 @@ __global__ void __launch_bounds__(kScfBigThreads, 1) k_scf_cluster(const __grid_
 
 using namespace dxtb;
 
-extern "C" int64_t dxtb_scf_workspace_mol(int64_t n, int64_t nat) { return ws_size_mol(n, nat); }
+extern "C" int64_t dxtb_scf_workspace_mol(int64_t n, int64_t nat) { return ws_size_mol(n, nat, true); }
+
+extern "C" int64_t dxtb_scf_workspace_size(int64_t n, int64_t nat, int32_t multipole, int32_t planes) {
+  return planes ? ws_size_mol(n, nat, multipole != 0) : ws_size_base(n, nat);
+}
 
 #include <cmath>
 #include <mutex>
@@ -1594,11 +1598,31 @@ extern "C" int32_t dxtb_scf_teams(
     double *vorb, double *vdp, double *vqp, double *energies, int32_t *status, const double *cn,
     const double *mrad, double *dedcn, double *grad,
     const int32_t *min_n, void *stream) {
-  if (!min_n || !valid_classes(min_n)) return DXTB_ERR_ARGS;
+  if (!min_n) return DXTB_ERR_ARGS;
+  dxtb_scf_plan plan = {};
+  for (int c = 0; c < kClasses - 1; ++c) plan.min_n[c] = min_n[c];
+  plan.planes = 1;
+  return dxtb_scf_planned(b, par_f, par_i, overlap, h0, dipole, quadrupole, gamma, hd, amat_sd, amat_dd,
+                          amat_sq, gb_mat, n0, nel, kt, cfg, ws_off, order, workspace, density, wdensity,
+                          coeff, evals, occ, q, dp, qp, vorb, vdp, vqp, energies, status, cn, mrad, dedcn,
+                          grad, &plan, stream);
+}
+
+extern "C" int32_t dxtb_scf_planned(
+    const dxtb_batch *b, const double *par_f, const int32_t *par_i, const double *overlap,
+    const double *h0, const double *dipole, const double *quadrupole, const double *gamma,
+    const double *hd, const double *amat_sd, const double *amat_dd, const double *amat_sq,
+    const double *gb_mat, const double *n0, const double *nel, double kt, const dxtb_scf_config *cfg,
+    const int64_t *ws_off, const int32_t *order, double *workspace, double *density,
+    double *wdensity, double *coeff, double *evals, double *occ, double *q, double *dp, double *qp,
+    double *vorb, double *vdp, double *vqp, double *energies, int32_t *status, const double *cn,
+    const double *mrad, double *dedcn, double *grad, const dxtb_scf_plan *plan, void *stream) {
+  if (!plan || !valid_classes(plan->min_n)) return DXTB_ERR_ARGS;
   const GradArgs g{cn, mrad, dedcn, grad};
   return scf_call(b, par_f, par_i, overlap, h0, dipole, quadrupole, gamma, hd, amat_sd, amat_dd,
                   amat_sq, gb_mat, n0, nel, kt, cfg, ws_off, order, workspace, density, wdensity,
-                  coeff, evals, occ, q, dp, qp, vorb, vdp, vqp, energies, status, stream, 1, min_n, grad != nullptr ? &g : nullptr);
+                  coeff, evals, occ, q, dp, qp, vorb, vdp, vqp, energies, status, stream,
+                  plan->planes ? 1 : 0, plan->min_n, grad != nullptr ? &g : nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -1639,7 +1663,7 @@ __global__ void k_noalloc_layout(dxtb_batch b, int64_t *hdr, int64_t ws_start) {
       hdr[kNoallocHeader + m] = off;
       const int64_t n = b.ao_off[m + 1] - b.ao_off[m];
       const int64_t nat = b.atom_off[m + 1] - b.atom_off[m];
-      off += fast ? ws_size_mol(n, nat) : ws_size_base(n, nat);
+      off += fast ? ws_size_mol(n, nat, true) : ws_size_base(n, nat);
     }
     hdr[kNoallocHeader + b.nmol] = off;
     return ws_start + off;  // doubles needed from the start of the array

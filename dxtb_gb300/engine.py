@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import warnings
 from dataclasses import dataclass
 
 import numpy as np
@@ -129,8 +130,8 @@ class PackedBatch:
         self.nat2_off = _prefix(nat * nat)
         self.nsh2_off = _prefix(nsh * nsh)
         self.pair_off = _prefix(nsh * (nsh + 1) // 2)
-        ws = np.array([_lib.lib().dxtb_scf_workspace_mol(int(n), int(a)) for n, a in zip(nao, nat)])
-        self.ws_off = _prefix(ws)
+        self.planes = True  # the SCF workspace holds the digit planes
+        self.ws_off = self._workspaces()
 
         # one upload of all tables: 19 separate ones took 0.5 ms of host time
         # against 0.1 ms, more than all else in packing a small molecule
@@ -162,6 +163,17 @@ class PackedBatch:
         self.classes = None  # thresholds of the size classes 1..5 (None: dxtb_scf_team_sizes)
         self._nao32 = np.ascontiguousarray(nao, dtype=np.int32)
         self.set_positions(positions)
+
+    def _workspaces(self) -> np.ndarray:
+        size, mp = _lib.lib().dxtb_scf_workspace_size, int(self.tables.multipole)
+        return _prefix(np.array([size(int(n), int(a), mp, int(self.planes)) for n, a in zip(self.nao, self.nat)]))
+
+    def drop_planes(self) -> None:
+        """Workspaces without the digit planes, a fifth to a seventh of the size: the
+        SCF runs in float64, 2 to 10 times slower."""
+        self.planes = False
+        self.ws_off = self._workspaces()
+        self.t["ws_off"] = torch.from_numpy(self.ws_off).to(self.device)
 
     def set_positions(self, positions: list) -> None:
         pos = [torch.as_tensor(p, dtype=F64).reshape(-1, 3) for p in positions]
@@ -216,6 +228,16 @@ class Result:
     gradient: torch.Tensor | None  # [natoms, 3] packed
     state: dict
     launches: int = 0              # kernels of the library launched by this call
+
+
+def point_bytes(tables: Tables, n: int, nat: int, nsh: int, planes: bool = True) -> int:
+    """Device bytes of one molecule's state (integrals, caches, SCF workspace, outputs)."""
+    mp = tables.multipole
+    ws = int(_lib.lib().dxtb_scf_workspace_size(n, nat, int(mp), int(planes)))
+    mats = (5 + (9 if mp else 0)) * n * n          # S H P C W (+ D Q)
+    caches = nsh * nsh + (18 * nat * nat if mp else 0)
+    vecs = 16 * n + 40 * nat
+    return 8 * (mats + caches + vecs + ws) + 4096
 
 
 def _seg_sum(values: torch.Tensor, seg: torch.Tensor, nmol: int) -> torch.Tensor:
@@ -376,7 +398,17 @@ def run(pb: PackedBatch, *, etemp: float = 300.0, maxiter: int = 250, tol: float
     if status is None or status.numel() < pb.nmol:
         status = torch.empty(pb.nmol, dtype=torch.int32, device=dev)
         s["status"] = status
-    ws = buf("ws", tot["ws"])
+    grad, dedcn = (buf("grad", 3 * na), buf("dedcn", na)) if forces else (None, None)
+    try:
+        ws = buf("ws", tot["ws"])
+    except torch.OutOfMemoryError:
+        if not pb.planes:
+            raise
+        warnings.warn("no memory for the SCF's digit planes: this batch runs in float64, slower; "
+                      "smaller batches would fit", stacklevel=2)
+        s.pop("ws", None)
+        pb.drop_planes()
+        ws = buf("ws", pb.total["ws"])
     kt = etemp * radii.KELVIN2AU
     cfg = scf_config(maxiter, tol, scf)
     scf_args = (b, pf, pi, S.data_ptr(), H.data_ptr(), _lib.ptr(D), _lib.ptr(Q), gamma.data_ptr(),
@@ -388,22 +420,20 @@ def run(pb: PackedBatch, *, etemp: float = 300.0, maxiter: int = 250, tol: float
                 en.data_ptr(), status.data_ptr())
     thr = team_sizes(pb._nao32, pb.lanes) if pb.classes is None else (C.c_int32 * 5)(*pb.classes)
     n_scf = scf_launches(thr, pb.struct.max_nao)
-    grad = None
+    plan = C.byref(_lib.ScfPlan(thr, int(pb.planes)))
     if forces:
         # SCF and gradient fused per size class: each class's forces overlap
         # the SCF of the larger classes (grad and dE/dCN zeroed first)
-        grad = buf("grad", 3 * na)
         grad.zero_()
-        dedcn = buf("dedcn", na)
         dedcn.zero_()
         mark("scf", 0)
-        _lib.check(L.dxtb_scf_teams(*scf_args, cn.data_ptr(), _lib.ptr(mrad), dedcn.data_ptr(),
-                                    grad.data_ptr(), thr, st), "SCF and gradient")
+        _lib.check(L.dxtb_scf_planned(*scf_args, cn.data_ptr(), _lib.ptr(mrad), dedcn.data_ptr(),
+                                      grad.data_ptr(), plan, st), "SCF and gradient")
         launches += 4 * n_scf  # per class: SCF, pairs with d shells, other terms, CN chain rule
         mark("scf", 1)
     else:
         mark("scf", 0)
-        _lib.check(L.dxtb_scf_teams(*scf_args, None, None, None, None, thr, st), "SCF")
+        _lib.check(L.dxtb_scf_planned(*scf_args, None, None, None, None, plan, st), "SCF")
         launches += n_scf
         mark("scf", 1)
     if forces:

@@ -131,6 +131,8 @@ class Server:
             raise ValueError("a large lane needs large_n")
         self.ex = executor
         self.budget = int(hbm_budget)
+        if hasattr(executor, "budget"):
+            executor.budget = self.budget
         self.slots = slots
         self.max_pack = max_pack
         self.large_slots = large_slots
@@ -427,7 +429,8 @@ class CudaExecutor:
         prio = priorities or [0] * slots
         self.streams = [torch.cuda.Stream(self.device, priority=int(prio[i])) for i in range(slots)]
         self.opts = dict(etemp=etemp, maxiter=maxiter, tol=tol)
-        self._ws = {}
+        self.budget: int | None = None  # device bytes that one request may take (set by the server)
+        self._points: dict = {}
         # per-slot device state and pinned result buffers, reused by every
         # pack of the slot (a slot takes its next pack only after the host
         # has collected the last one): steady-state packs allocate almost
@@ -470,19 +473,22 @@ class CudaExecutor:
         """``pack_sms`` of the request in a pack of its own."""
         return self.pack_sms([req])
 
+    def _point(self, req: Request) -> tuple[int, bool]:
+        """Device bytes of one request's state, and whether it has the digit
+        planes: not where the server's budget would only hold it without."""
+        from .engine import point_bytes
+
+        key = (self.budget, req.method, *self._sizes(req))
+        if key not in self._points:
+            tb, sizes = self.tables[req.method], key[2:]
+            b = point_bytes(tb, *sizes)
+            planes = self.budget is None or b <= self.budget
+            self._points[key] = (b if planes else point_bytes(tb, *sizes, planes=False), planes)
+        return self._points[key]
+
     def nbytes(self, req: Request) -> int:
         """Device bytes of one request's state (integrals, caches, SCF workspace, outputs)."""
-        from . import _lib
-
-        n, nat, nsh = self._sizes(req)
-        key = (n, nat)
-        if key not in self._ws:
-            self._ws[key] = int(_lib.lib().dxtb_scf_workspace_mol(n, nat))
-        mp = req.method == "gfn2"
-        mats = (5 + (9 if mp else 0)) * n * n          # S H P C W (+ D Q)
-        caches = nsh * nsh + (18 * nat * nat if mp else 0)
-        vecs = 16 * n + 40 * nat
-        return 8 * (mats + caches + vecs + self._ws[key]) + 4096
+        return self._point(req)[0]
 
     def launch(self, reqs: list[Request], slot: int):
         torch = self.torch
@@ -495,6 +501,8 @@ class CudaExecutor:
                              device=self.device, charges=[r.chrg for r in reqs],
                              spins=[r.spin for r in reqs])
             pb.lanes = len(self.streams)
+            if not all(self._point(r)[1] for r in reqs):
+                pb.drop_planes()
             forces = any(r.forces for r in reqs)
             res = run(pb, forces=forces, state=self.state[slot], **self.opts)
             nm = pb.nmol

@@ -265,8 +265,15 @@ int32_t dxtb_graph_launch(void *exec, void *stream);
 int32_t dxtb_graph_destroy(void *exec);
 
 /* SCF workspace of one molecule in doubles (n AOs, nat atoms); the caller
- * lays the molecules' workspaces out at ws_off[m] (prefix of these sizes). */
+ * lays the molecules' workspaces out at ws_off[m] (prefix of these sizes).
+ * Large enough for either method; about 24 n^2. */
 int64_t dxtb_scf_workspace_mol(int64_t n, int64_t nat);
+
+/* The same by what the molecule uses: multipole as in the batch's parameter
+ * table (GFN1, 0: about 15 n^2), planes as in dxtb_scf_plan (0: about 3 n^2,
+ * for either method). */
+int64_t dxtb_scf_workspace_size(int64_t n, int64_t nat, int32_t multipole,
+                                int32_t planes);
 
 /* Self-consistent field for every molecule of the batch, one persistent
  * launch per size class and one team per molecule (a CTA, or a thread-block
@@ -363,6 +370,32 @@ int32_t dxtb_scf_teams(const dxtb_batch *b, const double *par_f,
                        double *vqp, double *energies, int32_t *status,
                        const double *cn, const double *mrad, double *dedcn,
                        double *grad, const int32_t *min_n, void *stream);
+
+/* What one SCF call may choose for itself. */
+typedef struct dxtb_scf_plan {
+  int32_t min_n[5];  /* smallest n of size classes 1-5                     */
+  int32_t planes;    /* 1: the workspaces hold the digit planes; 0: they
+                      * do not (dxtb_scf_workspace_size), and the SCF runs
+                      * in float64: 2 to 10 times slower, a seventh of the
+                      * workspace                                          */
+} dxtb_scf_plan;
+
+/* dxtb_scf_teams with a plan in place of the thresholds. */
+int32_t dxtb_scf_planned(const dxtb_batch *b, const double *par_f,
+                         const int32_t *par_i, const double *overlap,
+                         const double *h0, const double *dipole,
+                         const double *quadrupole, const double *gamma,
+                         const double *hd, const double *amat_sd,
+                         const double *amat_dd, const double *amat_sq,
+                         const double *gb_mat, const double *n0,
+                         const double *nel, double kt, const dxtb_scf_config *cfg,
+                         const int64_t *ws_off, const int32_t *order,
+                         double *workspace, double *density, double *wdensity,
+                         double *coeff, double *evals, double *occ, double *q,
+                         double *dp, double *qp, double *vorb, double *vdp,
+                         double *vqp, double *energies, int32_t *status,
+                         const double *cn, const double *mrad, double *dedcn,
+                         double *grad, const dxtb_scf_plan *plan, void *stream);
 
 /* Nuclear gradient dE/dR [natoms][3] at the converged SCF (analytic
  * adjoint; the reference differentiates with autograd through
