@@ -56,7 +56,7 @@ class ScfConfig(C.Structure):
 class ScfPlan(C.Structure):
     """Mirror of ``dxtb_scf_plan``."""
 
-    _fields_ = [("min_n", i32 * 5), ("planes", i32)]
+    _fields_ = [("min_n", i32 * 5), ("planes", i32), ("give_up", i64), ("rotation", f64)]
 
 
 MIXERS = {"broyden1": 0, "anderson": 1}

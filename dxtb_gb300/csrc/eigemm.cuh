@@ -987,9 +987,11 @@ __device__ __noinline__ void fast_sort(Team<CL> &tm, int n, Fast &f, double *lam
 
 // Eigenvectors (rows of V, ascending) and eigenvalues (lam, shared, every
 // CTA; in units of 2^s) of the matrix whose planes, scaled by 2^-s to a
-// Frobenius norm in (1/2, 1], are in f.Fr. False when the steps do not converge.
+// Frobenius norm in (1/2, 1], are in f.Fr. False when they do not settle within
+// max_steps. rotation: factor on the first bound of a step's rotations.
 template <bool CL>
-__device__ bool fast_eigen(Team<CL> &tm, int n, Fast &f, double *lam, double *sk, float *lh, float *ll, float4 *sm) {
+__device__ bool fast_eigen(Team<CL> &tm, int n, Fast &f, double *lam, double *sk, float *lh, float *ll, float4 *sm,
+                           int max_steps, float rotation) {
   const bool warm = f.warm;
   const float z0 = f.z0;
   __syncthreads();
@@ -997,9 +999,9 @@ __device__ bool fast_eigen(Team<CL> &tm, int n, Fast &f, double *lam, double *sk
   if (!warm) fast_identity(tm, n, f);
   // the first rotation shrinks from one problem to the next as the SCF converges
   bool low = !warm || 0.5f * z0 > kZLow;
-  float top = fmaxf(kZNorm, 0.2f * sqrtf((float)n)), zprev = 1.0f;
+  float top = rotation * fmaxf(kZNorm, 0.2f * sqrtf((float)n)), zprev = 1.0f;
   bool stalled = false;
-  for (int it = 0; it < kMaxSteps; ++it) {
+  for (int it = 0; it < max_steps; ++it) {
     if (low) {
       tiles<kDigLow>(tm, n, f, kStep, 0, 0, nullptr);
       tiles<kDigLow>(tm, n, f, kProject, 0, 0, nullptr);

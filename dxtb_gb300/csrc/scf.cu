@@ -196,6 +196,8 @@ struct ScfArgs {
   int32_t *status;
   int thr[kClasses];  // smallest n of each size class (thr[0] = 0)
   int fast;           // the workspace has room for the digit planes
+  int64_t give_up;    // dxtb_scf_plan
+  float rotation;
 };
 
 // SCFs that keep the float64 path: up to kTinyN orbitals (less than a block), as
@@ -791,7 +793,9 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
       for (int i = threadIdx.x; i < n; i += blockDim.x) aoat[i] = b.shell_atom[mv.s0 + b.ao_shell[mv.o0 + i]];
       __syncthreads();
       int s2;
-      fast = fast_fock(tm, n, f, H0, w.x, aoat, s2, sfour) && fast_eigen(tm, n, f, sd, se, df, e2f, sfour);
+      const int steps = it <= 64 && (a.give_up >> (it - 1) & 1) ? 0 : kMaxSteps;
+      fast = fast_fock(tm, n, f, H0, w.x, aoat, s2, sfour) &&
+             fast_eigen(tm, n, f, sd, se, df, e2f, sfour, steps, a.rotation);
       if (fast) {
         const double scale = ldexp(1.0, s2);
         for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -1503,7 +1507,7 @@ static int32_t apply_config(const dxtb_scf_config *c, ScfArgs &a) {
 }  // namespace dxtb
 
 // dxtb_scf (g: and the gradient); fast: the workspace holds ws_size_mol (else
-// ws_size_base) doubles a molecule; min_n as in launch_scf.
+// ws_size_base) doubles a molecule; plan: its thresholds, or null: the process's.
 static int32_t scf_call(const dxtb_batch *b, const double *par_f, const int32_t *par_i,
                         const double *overlap, const double *h0, const double *dipole,
                         const double *quadrupole, const double *gamma, const double *hd,
@@ -1513,7 +1517,7 @@ static int32_t scf_call(const dxtb_batch *b, const double *par_f, const int32_t 
                         double *workspace, double *density, double *wdensity, double *coeff,
                         double *evals, double *occ, double *q, double *dp, double *qp, double *vorb,
                         double *vdp, double *vqp, double *energies, int32_t *status, void *stream,
-                        int fast, const int32_t *min_n = nullptr, const GradArgs *g = nullptr) {
+                        int fast, const dxtb_scf_plan *plan = nullptr, const GradArgs *g = nullptr) {
   if (!b || b->nmol <= 0 || !overlap || !h0 || !gamma || !hd || !n0 || !nel || !ws_off ||
       !workspace || !density || !coeff || !evals || !occ || !q || !vorb || !energies || !status)
     return DXTB_ERR_ARGS;
@@ -1555,7 +1559,9 @@ static int32_t scf_call(const dxtb_batch *b, const double *par_f, const int32_t 
   a.energies = energies;
   a.status = status;
   a.fast = fast;
-  return launch_scf(a, b->nmol, (cudaStream_t)stream, min_n, g);
+  a.give_up = plan ? plan->give_up : 0;
+  a.rotation = plan && plan->rotation > 0.0 ? (float)plan->rotation : 1.0f;
+  return launch_scf(a, b->nmol, (cudaStream_t)stream, plan ? plan->min_n : nullptr, g);
 }
 
 extern "C" int32_t dxtb_scf(const dxtb_batch *b, const double *par_f, const int32_t *par_i,
@@ -1622,7 +1628,7 @@ extern "C" int32_t dxtb_scf_planned(
   return scf_call(b, par_f, par_i, overlap, h0, dipole, quadrupole, gamma, hd, amat_sd, amat_dd,
                   amat_sq, gb_mat, n0, nel, kt, cfg, ws_off, order, workspace, density, wdensity,
                   coeff, evals, occ, q, dp, qp, vorb, vdp, vqp, energies, status, stream,
-                  plan->planes ? 1 : 0, plan->min_n, grad != nullptr ? &g : nullptr);
+                  plan->planes ? 1 : 0, plan, grad != nullptr ? &g : nullptr);
 }
 
 // ---------------------------------------------------------------------------

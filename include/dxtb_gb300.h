@@ -378,6 +378,9 @@ typedef struct dxtb_scf_plan {
                       * do not (dxtb_scf_workspace_size), and the SCF runs
                       * in float64: 2 to 10 times slower, a seventh of the
                       * workspace                                          */
+  /* for tests of what an SCF does when its eigenvectors do not settle */
+  int64_t give_up;   /* bit k: SCF step k + 1 is taken in float64          */
+  double rotation;   /* first bound of the rotations over its default; 0: 1 */
 } dxtb_scf_plan;
 
 /* dxtb_scf_teams with a plan in place of the thresholds. */
