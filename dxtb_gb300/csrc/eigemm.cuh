@@ -4,12 +4,20 @@
 // The FP64 pipe of this part issues 1.7 FMA per clock and SM, the 16-bit
 // tensor instruction (mma.sync m16n8k16) 1020 (both measured): a product of
 // 60-bit fixed-point operands cut into six digits of ten bits takes 21 digit
-// products (orders p + q <= 5), still ~28 times the FP64 rate. The orders left
-// out are 2^-64 sqrt(5 n) of the operands' norms. The digit product sums are
-// integers in float32 accumulators, exact below 2^24: the orders 0 to 2 for any
-// operands of norm <= 1 (order 2 is carried upwards every 32 terms), the orders
-// from 3 on, of weight <= 2^-50, every 64 terms and for digits that are not all
-// at their limit (they would round, not overflow).
+// products (orders p + q <= 5), still ~28 times the FP64 rate (error-free
+// splitting as in Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59 (2012) 95,
+// with a fixed cut). The orders left out are 2^-64 sqrt(5 n) of the operands'
+// norms. The digit product sums are integers in float32 accumulators, exact below
+// 2^24 and rounded to an integer above. Six digits: the orders 0 to 2 are exact
+// for any operands of norm <= 1 (order 2 is carried upwards every 32 terms, all
+// orders every 64); from order 3 on, of weight <= 2^-50, for digits that are not
+// all at their limit. Three digits: orders 0 and 1 are exact for operands of norm
+// <= 1, order 2 can reach 4.5e7 in its 128 terms and is then rounded to a multiple
+// of 4, 2^-38 of operands that are cut at 2^-31. An update's left operand E^T
+// has rows of norm <= 8 and V columns of norm < 2, so that its values stay below
+// 16 as everywhere (2^24 in order 0, tile_fix); its order 1 may round the same
+// way, which the next step's R and T see, and which is below 2^-53 in the last
+// step, where E < 2^-28.
 // Nine-bit digits (54 bits) lost 2^-58 sqrt(5 n), with a sign on a diagonal: SCF
 // residuals then end at 6e-12 (n = 181) to 6e-10 (n = 1145), where float64 ends
 // at 6e-13 to 4e-12.
@@ -98,11 +106,11 @@ __device__ __forceinline__ void st_plane(uint4 *p, const uint4 &v) {
 }
 
 // The 16 x 16 tile sum_k A[i][k] B[j][k] over the k blocks [k0, k1) with NP
-// digits, as the sums of each order (acc[d], weight 2^(-10 (d + 2)), exact
-// integers): A, B are the first blocks of the two block rows, sa, sb the words
+// digits, as the sums of each order (acc[d], weight 2^(-10 (d + 2)), integers):
+// A, B are the first blocks of the two block rows, sa, sb the words
 // per block (planes stored x 32). Value e: row g + 8 ((e >> 1) & 1), column
 // 8 (e >> 2) + 2 q + (e & 1) for lane 4 g + q. Orders are carried into the one
-// above (multiples of 1024), which keeps them exact.
+// above (multiples of 1024); what stays exact is said at the top.
 template <int NP>
 __device__ __forceinline__ void tile_nt(const uint4 *A, int sa, const uint4 *B, int sb, bool left_b, int k0, int k1,
                                         float (&acc)[NP][8]) {
@@ -695,8 +703,12 @@ __device__ __noinline__ float tiles(Team<CL> &tm, int n, const Fast &f, Product 
   const int mb = what == kCoeff || dens ? (int)blocks16(arg) : nb;
   constexpr int S6 = kDig * 32, S3 = kDigLow * 32;
   const int row6 = nb * S6, row3 = nb * S3;
-  const uint4 *VT = f.VT[f.cur];
-  uint4 *VN = f.VT[f.cur ^ 1];
+  const uint4 *VT = nullptr;
+  uint4 *VN = nullptr;
+  if (what == kApply) {  // only there: thread 0 turns f.cur right after it
+    VT = f.VT[f.cur];
+    VN = f.VT[f.cur ^ 1];
+  }
   const int ntile = what == kStep                      ? nb * nb + nlow
                     : what == kApply || what == kHalf  ? nb * nb
                     : what == kCoeff                   ? nb * mb
@@ -1029,8 +1041,11 @@ __device__ bool fast_eigen(Team<CL> &tm, int n, Fast &f, double *lam, double *sk
     const float zm = s.m0 * sc;
     if (it == 0 && threadIdx.x == 0) f.z0 = zm;
     const bool last = !low && fmaxf(zf, rf) < kFinal;
-    const float em = zm + 0.5f * s.m1;
-    const int ke = em > 0x1p-50f ? -exp_above(em) : 50;
+    // scale of E for its digits: elements at most 1 and rows of norm at most 8,
+    // which bounds every sum E^T V (up to n = 64 the one gives the other; above, by
+    // the Frobenius norm)
+    const float em = zm + 0.5f * s.m1, ef = n > 64 ? 1.4143f * sc * zf + 0.5f * rf : 0.0f;
+    const int ke = min(em > 0x1p-50f ? -exp_above(em) : 50, 3 - exp_above(fmaxf(ef, 0x1p-60f)));
     step_update_planes(tm, n, f, sc, ke);
     // a coarse step that no longer shrinks the rotations has met its own rounding
     // (pairs closer than ~2^-20 of the norm): full steps from here on
