@@ -1282,13 +1282,6 @@ static int32_t class_gradient(const ScfArgs &a, const GradArgs *g, int c, cudaSt
                          a.vqp, a.S, a.D, g->dedcn, g->grad, f, s);
 }
 
-static bool default_policy() {
-  std::lock_guard<std::mutex> lock(g_policy_mutex);
-  for (int c = 1; c < kClasses; ++c)
-    if (g_thr[c] != kDefaultThr[c]) return false;
-  return true;
-}
-
 // min_n: thresholds of classes 1..5 for this call, or null: the process-wide ones.
 static int32_t launch_scf(ScfArgs a, int nmol, cudaStream_t st, const int32_t *min_n, const GradArgs *g) {
   if (min_n != nullptr) {
@@ -1301,12 +1294,11 @@ static int32_t launch_scf(ScfArgs a, int nmol, cudaStream_t st, const int32_t *m
       a.thr[c] = g_thr[c];
       preset = preset && g_thr[c] == kDefaultThr[c];
     }
+    // (the float64 path of a loose SCF, small_scf, on the team whose bits it keeps)
+    const int first = a.mixer == DXTB_MIXER_ANDERSON ? kLooseN + 1 : 0;
     if (preset)
-      for (int c = 0; c < kClasses; ++c) a.thr[c] = min(a.thr[c], kFewThr[c]);
+      for (int c = 1; c < kClasses; ++c) a.thr[c] = max(first, min(a.thr[c], kFewThr[c]));
   }
-  // the float64 path of a loose SCF (scf_body) on the team whose bits it keeps
-  if (a.mixer == DXTB_MIXER_ANDERSON && default_policy())
-    for (int c = 1; c < kClasses; ++c) a.thr[c] = max(a.thr[c], kLooseN + 1);
   int sms = 0;
   if (device_sms(&sms) != DXTB_OK) return DXTB_ERR_LAUNCH;
   const int nmax = a.b.max_nao;

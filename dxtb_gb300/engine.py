@@ -256,6 +256,22 @@ def team_sizes(nao: np.ndarray, lanes: int = 1):
     return thr
 
 
+LOOSE_N = 32  # largest order of the float64 path under Anderson mixing (kLooseN, csrc/scf.cu)
+
+
+def call_classes(pb: PackedBatch, mixer: int):
+    """Thresholds of the size classes 1..5 for one SCF call on ``pb``: the
+    batch's own, or the rule. Loose Anderson SCFs keep one CTA of 256 threads,
+    whose bits they follow, unless the process has a set of its own."""
+    thr = team_sizes(pb._nao32, pb.lanes) if pb.classes is None else (C.c_int32 * 5)(*pb.classes)
+    if mixer == _lib.MIXERS["anderson"]:
+        from . import autotune
+
+        if autotune.get_classes() == autotune.DEFAULT:
+            thr[:] = [max(t, LOOSE_N + 1) for t in thr]
+    return thr
+
+
 def scf_launches(thr, nmax: int) -> int:
     """SCF kernels launched for a batch whose largest molecule has nmax
     orbitals under the size classes thr: one per cluster class up to the
@@ -418,7 +434,7 @@ def run(pb: PackedBatch, *, etemp: float = 300.0, maxiter: int = 250, tol: float
                 _lib.ptr(W), Cm.data_ptr(), ev.data_ptr(), occ.data_ptr(), q.data_ptr(),
                 dp.data_ptr(), qp.data_ptr(), vorb.data_ptr(), vdp.data_ptr(), vqp.data_ptr(),
                 en.data_ptr(), status.data_ptr())
-    thr = team_sizes(pb._nao32, pb.lanes) if pb.classes is None else (C.c_int32 * 5)(*pb.classes)
+    thr = call_classes(pb, cfg.mixer)
     n_scf = scf_launches(thr, pb.struct.max_nao)
     plan = C.byref(_lib.ScfPlan(thr, int(pb.planes)))
     if forces:

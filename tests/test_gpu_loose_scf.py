@@ -45,3 +45,21 @@ def test_forces_of_the_float64_path(method, copies):
     got = np.concatenate(got).reshape(max(copies, 1), len(grad), 3)
     assert (np.concatenate(its).reshape(-1, len(mols)) == d[f"{method}_iterations"]).all()
     assert np.abs(got - grad).max() <= 1e-12
+
+
+@pytest.mark.parametrize("n", [31, 32, 33, 34])
+def test_the_launches_that_are_counted(n):
+    """Alone, molecules of 30 orbitals and more take a CTA of 512 threads, loose
+    Anderson SCFs from 33 on: one class fewer, of which a call launches one SCF
+    and, with forces, three gradient kernels."""
+    from dxtb_gb300.calculators import tables
+    from dxtb_gb300.engine import PackedBatch, run
+    from dxtb_gb300.workloads import build_geometry
+
+    heavy, nh = (n - 2) // 6, n - 4 * ((n - 2) // 6)
+    z, pos = build_geometry(np.random.default_rng(n), [7 if nh % 2 else 6] + [6] * (heavy - 1), nh)
+    pb = PackedBatch(tables("gfn2"), [z], [torch.tensor(pos)])
+    assert int(pb.nao[0]) == n
+    assert run(pb, forces=True).launches == 3 + 2 * 4
+    r = run(pb, forces=True, **OPTS)
+    assert int(r.status[0]) == 0 and r.launches == 3 + (1 if n <= 32 else 2) * 4
