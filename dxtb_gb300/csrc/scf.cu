@@ -445,9 +445,12 @@ enum ScfAction : int { kNext = 0, kStop = 1 };
 // (six multiply-adds a history element) and by the reductions' barriers: the
 // norms are summed together. (Gm F = Gm dy - dx_prev would need four, but its
 // rounding errors add up: a molecule of 89 steps no longer reached 1e-10.)
+// in_order (one CTA): d . F of the new vector as a sum of its own over the scaled
+// vector, as for the others, which is the order of the float64 path; its last bit
+// moved Hessians of up to 12 orbitals by 2e-8 of their norm.
 template <bool CL>
 __device__ __noinline__ int broyden_step(const ScfArgs &a, Team<CL> &tm, Ws &w, int N, int it, Broyden &br,
-                                         int &status, double *red) {
+                                         int &status, double *red, bool in_order) {
   __shared__ double s3[99];
   double *sdot = w.sdot;           // [kRank] c_k . dx
   double *sdot2 = sdot + kRank;    // [kRank] d_k . dy
@@ -534,6 +537,19 @@ __device__ __noinline__ int broyden_step(const ScfArgs &a, Team<CL> &tm, Ws &w, 
     const double idyv = 1.0 / dyv;
     fd = sum[2] * idyv;
     for (int t = tm.tid; t < N; t += tm.nthr) dn[t] *= idyv;
+    if constexpr (!CL) {
+      if (in_order) {
+        __syncthreads();
+        if (threadIdx.x < 32) {
+          double r = 0.0;
+          for (int t = lane; t < N; t += 32) r = fma(dn[t], w.x[t] - w.g[t], r);
+          r = warp_sum(r);
+          if (lane == 0) s3[0] = r;
+        }
+        __syncthreads();
+        fd = s3[0];
+      }
+    }
     ++br.nrank;
     if (br.dx_norm < a.xtol && ynorm < a.ftol) return kStop;  // converged at x
   }
@@ -1030,7 +1046,7 @@ __device__ void scf_body(const ScfArgs &a, int m_, Team<CL> &tm, double *dsm, bo
     } else if (a.mixer == DXTB_MIXER_ANDERSON) {
       act = anderson_step(a, tm, w, N, it, br, status, red);
     } else {
-      act = broyden_step(a, tm, w, N, it, br, status, red);
+      act = broyden_step(a, tm, w, N, it, br, status, red, !CL && small_scf(a, n));
     }
     tm.sync();
     if (act == kStop) {

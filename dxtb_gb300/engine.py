@@ -166,7 +166,9 @@ class PackedBatch:
 
     def _workspaces(self) -> np.ndarray:
         size, mp = _lib.lib().dxtb_scf_workspace_size, int(self.tables.multipole)
-        return _prefix(np.array([size(int(n), int(a), mp, int(self.planes)) for n, a in zip(self.nao, self.nat)]))
+        pairs = list(zip(self.nao.tolist(), self.nat.tolist()))
+        ws = {p: size(*p, mp, int(self.planes)) for p in set(pairs)}
+        return _prefix(np.array([ws[p] for p in pairs]))
 
     def drop_planes(self) -> None:
         """Workspaces without the digit planes, a fifth to a seventh of the size: the
