@@ -48,7 +48,7 @@
 //
 // Measured against the Householder / float64 path (GB300, energy + forces):
 // one molecule of 72 orbitals 36.9 -> 8.0 ms, of 233 orbitals 292 -> 28.4 ms
-// (there 4 CTAs, here 16), 256 molecules of 22-172 orbitals 223 -> 74.1 ms, with
+// (there 4 CTAs, here 16), 256 molecules of 22-172 orbitals 223 -> 71.7 ms, with
 // no larger distance from the CPU oracle over the benchmark sets (|dE| <= 7.0e-12
 // Eh, |dF| <= 5.2e-12 Eh/Bohr; 7.0e-12 and 1.2e-10 there).
 #pragma once

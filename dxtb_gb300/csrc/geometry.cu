@@ -1,7 +1,8 @@
 // Geometry-only terms of the GFN-xTB single point: coordination numbers and
 // the interaction caches that stay fixed during the SCF (ES2 gamma, ES3
 // Hubbard derivatives, AES2 damping radii and kernels, repulsion energy).
-// One CTA per molecule; threads stride over atom or shell pairs.
+// Coordination numbers: a warp per atom; caches: several CTAs a molecule, a thread
+// per atom or shell pair.
 #include "common.cuh"
 
 namespace dxtb {

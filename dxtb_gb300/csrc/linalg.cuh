@@ -23,11 +23,12 @@
 // The SCF needs only the orbitals with non-vanishing occupation, so the
 // O(n^3) accumulation of QL rotations is never done.
 //
-// In a cluster team, data written by another CTA is read with ld.global.cg
-// (L2, never a stale L1 line) after a barrier.cluster arrive.release /
-// wait.acquire pair, or from that CTA's shared memory (mapa +
-// ld/st.shared::cluster, team_tridiag); a one-CTA team uses plain loads and
-// __syncthreads.
+// In a cluster team, data written by another CTA is read after a barrier.cluster
+// arrive.release / wait.acquire pair, whose acquire makes plain loads right (the
+// digit planes and their tables, eigemm.cuh, are read so); the float64 phases
+// here take ld.global.cg, which leaves the L1 to their own rows. Or it is read
+// from that CTA's shared memory (mapa + ld/st.shared::cluster, team_tridiag). A
+// one-CTA team uses plain loads and __syncthreads.
 //
 // A float64 instruction costs a warp ~64 cycles on this part whatever its
 // active lanes (the SM issues about one warp-instruction per 19 cycles over

@@ -312,8 +312,10 @@ int32_t dxtb_scf(const dxtb_batch *b, const double *par_f, const int32_t *par_i,
  * 8 or 16 CTAs on as many SMs (classes 2-5) that share every O(n^3) phase.
  * min_n[c-1] is the smallest n of class c (non-decreasing); the default is
  * {112, 136, 160, 320, 640}, under which a batch of one or two molecules
- * takes larger teams ({30, 60, 60, 90, 130}) and dxtb_scf_team_sizes fits the
- * teams to the batch; any other setting holds for every batch. Clusters need the launch order of dxtb_scf;
+ * takes larger teams ({30, 60, 60, 90, 130}; with the Anderson mixer none of
+ * them below 33) and dxtb_scf_team_sizes fits the teams to the batch; any
+ * other setting holds for every call without thresholds of its own. Clusters
+ * need the launch order of dxtb_scf;
  * cluster sizes the GPU cannot place fold into the largest one it can.
  * Each class runs on a stream of its own, forked from the caller's stream:
  * larger classes get higher stream priorities, unless the caller's stream
