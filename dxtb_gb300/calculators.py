@@ -323,10 +323,11 @@ class Calculator:
             if g is None and forces not in self._graphs:
                 self._pb.copy_positions_(packed)
                 try:
-                    g = engine.GraphStep(self._pb, **kw)
+                    g = engine.GraphStep(self._pb, fallback=False, **kw)
                     res = g.first
                 except RuntimeError as err:
-                    # a capture the driver refuses: keep the eager launches
+                    # a capture the driver refuses, or no memory for a second
+                    # state: keep the eager launches
                     warnings.warn(f"CUDA graph capture failed ({err}); launching eagerly",
                                   stacklevel=3)
                     g = None

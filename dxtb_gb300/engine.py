@@ -173,8 +173,11 @@ class PackedBatch:
     def drop_planes(self) -> None:
         """Workspaces without the digit planes, a fifth to a seventh of the size: the
         SCF runs in float64, 2 to 10 times slower."""
+        if not self.planes:
+            return
         self.planes = False
         self.ws_off = self._workspaces()
+        self.t["ws_off_planes"] = self.t["ws_off"]  # a captured step may still read it
         self.t["ws_off"] = torch.from_numpy(self.ws_off).to(self.device)
 
     def set_positions(self, positions: list) -> None:
@@ -326,7 +329,8 @@ def scf_config(maxiter: int, tol: float, scf: dict | None = None) -> _lib.ScfCon
 
 def run(pb: PackedBatch, *, etemp: float = 300.0, maxiter: int = 250, tol: float = 1e-10,
         forces: bool = False, gb: dict | None = None, state: dict | None = None,
-        events: dict | None = None, scf: dict | None = None, collect: bool = True) -> Result:
+        events: dict | None = None, scf: dict | None = None, collect: bool = True,
+        fallback: bool = True) -> Result:
     """
     One single point for every molecule of the packed batch. With ``events``
     (a dict), CUDA events are recorded on the current stream around each
@@ -334,6 +338,8 @@ def run(pb: PackedBatch, *, etemp: float = 300.0, maxiter: int = 250, tol: float
     and its tolerances (``scf_config``). With ``collect=False`` only the
     library's kernels are launched (no PyTorch operation allocates) and the
     number of launches is returned; ``collect_result`` then reads the state.
+    Without memory for the SCF's digit planes the batch drops them and runs in
+    float64 (``fallback``; else torch's OutOfMemoryError).
     """
     L = _lib.lib()
 
@@ -420,7 +426,7 @@ def run(pb: PackedBatch, *, etemp: float = 300.0, maxiter: int = 250, tol: float
     try:
         ws = buf("ws", tot["ws"])
     except torch.OutOfMemoryError:
-        if not pb.planes:
+        if not (pb.planes and fallback):
             raise
         warnings.warn("no memory for the SCF's digit planes: this batch runs in float64, slower; "
                       "smaller batches would fit", stacklevel=2)

@@ -53,6 +53,50 @@ def test_batch_without_room_for_the_planes():
     assert not pb.planes and (r.energy - e).abs().max() <= 1e-9
 
 
+def test_a_captured_step_outlives_the_planes_of_its_batch():
+    """A graph captured with planes keeps its layout when the batch drops them."""
+    from dxtb_gb300.calculators import tables
+    from dxtb_gb300.engine import GraphStep, PackedBatch, run
+    from dxtb_gb300.workloads import config_molecules
+
+    mols = config_molecules(2)[:12]
+    pb = PackedBatch(tables("gfn2"), [m[0] for m in mols], [torch.tensor(m[1]) for m in mols])
+    step = GraphStep(pb, forces=True)
+    e = step.first.energy.clone()
+    pb.drop_planes()
+    assert (run(pb, forces=True).energy - e).abs().max() <= 1e-9
+    junk = [torch.full((256,), -1, dtype=torch.int64, device="cuda") for _ in range(64)]
+    assert (step.replay().energy - e).abs().max() <= 1e-10
+    del junk
+
+
+def test_no_memory_for_a_captured_step():
+    """A calculator whose graph does not fit beside its state launches eagerly,
+    with the planes it has."""
+    from dxtb_gb300 import GFN2Calculator
+    from dxtb_gb300.workloads import config_molecules
+
+    mols = config_molecules(2)[:31]
+    nat = max(len(z) for z, _ in mols)
+    num, pos = torch.zeros(len(mols), nat, dtype=torch.int64), torch.zeros(len(mols), nat, 3, dtype=torch.float64)
+    for i, (z, p) in enumerate(mols):
+        num[i, : len(z)], pos[i, : len(z)] = torch.as_tensor(z), torch.as_tensor(p)
+    opts = {"exclude": ["disp", "d4sc"], "guess": "sad", "scf_mode": "implicit", "x_atol": 1e-10,
+            "f_atol": 1e-10, "maxiter": 250}
+    calc = GFN2Calculator(num, opts=opts, device="cuda")
+    e = calc.get_energy(pos.cuda()).clone()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (40 << 20)) / total)
+        calc.reset()
+        with pytest.warns(UserWarning, match="capture failed"):
+            again = calc.get_energy(pos.cuda())
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert calc._pb.planes and (again - e).abs().max() <= 1e-10
+
+
 @pytest.mark.parametrize("method", ["gfn1", "gfn2"])
 def test_hessian_in_packs(method):
     from dxtb_gb300.calculators import tables
